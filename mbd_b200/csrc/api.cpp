@@ -420,17 +420,24 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
     int st = relay_learned(ctx, gd, sl, mstride, ev[3], &Xv);
     if (st != MBD_OK) return st;
   } else {
-    // 3. blocked Cholesky, batched over the 21 frequencies
+    // 3. Cholesky of the 21 frequency matrices in one launch
     BatchMat bm{sl.relay64.as<double>(), mstride, p.ld, n, kNFreq};
     const int nblk = (n + kCholNB - 1) / kCholNB;
     const size_t lstride = (size_t)nblk * kCholNB * kCholNB;
     double* Linv = sl.linv.as<double>();
-    for (int k0 = 0; k0 < n; k0 += kCholNB) {
-      launch_potrf_diag_f64(bm, k0, Linv, lstride, gd->info, s);
-      launch_trsm_panel_f64(bm, k0, Linv, lstride, s);
-      launch_syrk_lower_f64(bm, k0, s);
-      ctx->launches += (k0 + kCholNB < n) ? 3 : 1;
-    }
+    CholFlowArgs cf{};
+    cf.src = cf.L = bm.A;
+    cf.src_stride = cf.l_stride = mstride;
+    cf.src_ld = cf.ld = p.ld;
+    cf.n = n;
+    cf.batch = kNFreq;
+    cf.linv = Linv;
+    cf.linv_stride = lstride;
+    cf.info = gd->info;
+    cf.sync = sl.chol_sync.as<int>();
+    cf.err = ctx->err_flag;
+    MBD_CUDA(launch_chol_flow(cf, ctx->num_sms, s));
+    ctx->launches += 1;
     mark(3);
     // 4. solve X = A^-1 [I;..;I]
     double* Wv = sl.rhs.as<double>();
@@ -499,12 +506,13 @@ int run_tail_single(mbd_ctx* ctx, GeomDev* gd, cudaStream_t s) {
 
 // ---- workspaces and the batch plan ----------------------------------------
 
-size_t plain_bytes(const GeomPlan& p, size_t* relay, size_t* linv, size_t* rhs) {
+size_t plain_bytes(const GeomPlan& p, size_t* relay, size_t* linv, size_t* rhs, size_t* sync) {
   const int nblk = (p.n + kCholNB - 1) / kCholNB;
   *relay = sizeof(double) * (size_t)kNFreq * p.n * p.ld;
   *linv = sizeof(double) * (size_t)kNFreq * nblk * kCholNB * kCholNB;
   *rhs = sizeof(double) * 3 * (size_t)kNFreq * p.n * 3;
-  return *relay + *linv + *rhs;
+  *sync = sizeof(int) * chol_flow_sync_ints(p.n, kNFreq);
+  return *relay + *linv + *rhs + *sync;
 }
 
 size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, size_t* res, size_t* sync) {
@@ -536,7 +544,7 @@ int plan_slots(mbd_ctx* ctx) {
       slot_of[g] = s;
       load[s] += std::pow((double)p.n, 3.0);
       size_t a, b, c, d, e, f, h;
-      need[s] = std::max(need[s], plain_bytes(p, &a, &b, &c) + mixed_bytes(p, &d, &e, &f, &h, &a));
+      need[s] = std::max(need[s], plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a));
     }
     double total = 0.0;
     for (size_t x : need) total += (double)x;
@@ -597,19 +605,21 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   int st = plan_slots(ctx);
   if (st != MBD_OK) return st;
   for (int s = 0; s < ctx->n_slots; ++s) {
-    size_t relay = 0, linv = 0, rhs = 0;
+    size_t relay = 0, linv = 0, rhs = 0, sync = 0;
     for (int g : ctx->order) {
       if (ctx->geoms[g]->slot != s) continue;
-      size_t a, b, c;
-      plain_bytes(ctx->geoms[g]->plan, &a, &b, &c);
+      size_t a, b, c, d;
+      plain_bytes(ctx->geoms[g]->plan, &a, &b, &c, &d);
       relay = std::max(relay, a);
       linv = std::max(linv, b);
       rhs = std::max(rhs, c);
+      sync = std::max(sync, d);
     }
     RelaySlot& sl = *ctx->slots[s];
     MBD_CUDA(sl.relay64.reserve(relay));
     MBD_CUDA(sl.linv.reserve(linv));
     MBD_CUDA(sl.rhs.reserve(rhs));
+    MBD_CUDA(sl.chol_sync.reserve(sync));
     if (eigen) {
       size_t tw = 0;
       for (int g : ctx->order)
@@ -973,7 +983,7 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
     ctx->priorities = !(pr && pr[0] == '0');
   }
   MBD_CUDA(init_device_constants());
-  MBD_CUDA(init_chol_attributes());
+  MBD_CUDA(init_cholflow_attributes());
   MBD_CUDA(init_eigval_attributes());
   MBD_CUDA(init_tc3_attributes());
   MBD_CUDA(init_mixed_attributes());
@@ -1528,6 +1538,7 @@ int mbd_rsscs_set_option(mbd_ctx* ctx, int option, double value) {
       MBD_CUDA(set_wait_limit_tridiag(cycles));
       MBD_CUDA(set_wait_limit_mixed(cycles));
       MBD_CUDA(set_wait_limit_tc3(cycles));
+      MBD_CUDA(set_wait_limit_cholflow(cycles));
       ctx->wait_limit_s = value;
       return MBD_OK;
     }

@@ -112,7 +112,7 @@ struct RelaySlot {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   Sy2sbLookAhead la{};   // the dense -> band look-ahead's stream and events
-  DevBuf relay64, linv, rhs;                                  // plain FP64 path
+  DevBuf relay64, linv, rhs, chol_sync;                       // plain FP64 path
   DevBuf relay32, p_hi, p_lo, l_hi, l_lo, mixv, res_ws, solve_sync;   // mixed path
   DevBuf cg, gnn;                                             // learned path: CG vectors, network work
   DevBuf trd_ws;                                              // dense -> band workspace
@@ -125,7 +125,7 @@ struct RelaySlot {
     if (stream) cudaStreamDestroy(stream);
   }
   size_t held() const {
-    return relay64.bytes + linv.bytes + rhs.bytes + relay32.bytes + p_hi.bytes + p_lo.bytes + l_hi.bytes +
+    return relay64.bytes + linv.bytes + rhs.bytes + chol_sync.bytes + relay32.bytes + p_hi.bytes + p_lo.bytes + l_hi.bytes +
            l_lo.bytes + mixv.bytes + res_ws.bytes + solve_sync.bytes + cg.bytes + gnn.bytes + trd_ws.bytes;
   }
 };

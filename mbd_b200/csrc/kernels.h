@@ -68,12 +68,33 @@ struct BatchMat {
   size_t stride;           // elements between matrices
   int ld, n, batch;
 };
-// Linv: per matrix, ceil(n/64) blocks of 64x64 inverses of the diagonal factor blocks.
-void launch_potrf_diag_f64(const BatchMat& m, int k0, double* Linv, size_t linv_stride, int* info,
-                           cudaStream_t s);
-void launch_trsm_panel_f64(const BatchMat& m, int k0, const double* Linv, size_t linv_stride,
-                           cudaStream_t s);
-void launch_syrk_lower_f64(const BatchMat& m, int k0, cudaStream_t s);
+// Batched Cholesky src + shift I = L L^T in one persistent launch
+// (k_cholflow.cu).  src may be L itself (same leading dimension); only lower
+// triangles are read and written.  The diagonal blocks of L are not stored,
+// their inverses are: linv holds, per matrix, ceil(n/64) blocks of 64 x 64
+// (row-major, zeros above the diagonal).
+struct CholFlowArgs {
+  const double* src;       // source matrices; stride 0: one source for all
+  size_t src_stride;
+  int src_ld;
+  double* L;               // factors, row-major lower
+  size_t l_stride;
+  int ld, n;
+  int batch;               // matrices (at most, where batch_dev is given)
+  const int* batch_dev;    // matrices, read on the device; null: batch
+  const double* shift;     // [batch] added to the diagonal; null: none
+  double* linv;
+  size_t linv_stride;
+  double* logdet;          // [batch][ceil(n/64)]: sum of log(pivot * ref) of a diagonal block; null: not wanted
+  const double* ref;       // [batch]
+  int* info;               // [batch]: first failing column + 1 where a pivot is not positive; zeroed by the caller
+  int* sync;               // chol_flow_sync_ints(n, batch) ints
+  int* err;                // the context's error flag (a wait that ran out)
+};
+constexpr int kCholFlowHead = 32;
+size_t chol_flow_sync_ints(int n, int batch);
+cudaError_t init_cholflow_attributes();
+cudaError_t launch_chol_flow(const CholFlowArgs& a, int num_sms, cudaStream_t s);
 // Y (n x 3 per matrix, row-major, stride ystride) := stacked identities [I;I;..;I].
 void launch_init_rhs(double* Y, size_t ystride, int n, int batch, cudaStream_t s);
 // Forward step: reads W at block k0, writes Z at block k0, updates W below it.
@@ -82,7 +103,6 @@ void launch_trsv_fwd_step(const BatchMat& m, int k0, const double* Linv, size_t 
 // Backward step: reads Zw at block k0, writes X at block k0, updates Zw above it.
 void launch_trsv_bwd_step(const BatchMat& m, int k0, const double* Linv, size_t linv_stride, double* Zw,
                           double* X, size_t ystride, cudaStream_t s);
-cudaError_t init_chol_attributes();
 
 // ---- epilogues (UTILS.f90:479-495, 272-315, 731-741) ----
 struct EpilogueArgs {
@@ -299,5 +319,6 @@ cudaError_t set_wait_limit_sb2st(long long cycles);
 cudaError_t set_wait_limit_tridiag(long long cycles);
 cudaError_t set_wait_limit_mixed(long long cycles);
 cudaError_t set_wait_limit_tc3(long long cycles);
+cudaError_t set_wait_limit_cholflow(long long cycles);
 
 }  // namespace mbd

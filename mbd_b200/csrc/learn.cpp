@@ -386,6 +386,7 @@ int mbd_rsscs_learned_train(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms, int
     work = std::max(work, gnn_work_floats(p.N, kNFreq, gd->n_edges, true));
   }
   MBD_CUDA(ctx->gnn_train_work.reserve(sizeof(float) * work));
+  MBD_CUDA(cudaMemsetAsync(ctx->err_flag, 0, sizeof(int), ctx->stream));
   MBD_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->launches = 0;
   for (int g : ctx->order) {
