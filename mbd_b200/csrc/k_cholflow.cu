@@ -17,9 +17,9 @@
 // Bound: FP64 tensor-core rate (36.9 TFLOP/s measured for m8n8k4 with all
 // operands in registers) while a block column has tiles for the whole chip;
 // below that the chain diagonal block -> tile below it -> next diagonal
-// block, n / 64 links of ~32 us.  Measured, 21 relay matrices of n rows (right-looking
+// block, n / 64 links of 20 us.  Measured, 21 relay matrices of n rows (right-looking
 // kernels before -> now): n = 3000 17.5 -> 7.6 ms (10.8 -> 24.9 TFLOP/s),
-// n = 384 0.85 -> 0.20 ms; n = 6000 53 ms (28.4 TFLOP/s).
+// n = 384 0.85 -> 0.15 ms; n = 6000 50.7 ms (29.8 TFLOP/s).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,164 +89,154 @@ __device__ int wait_count(const int* p, int want, int* err) {
 }
 
 // ---- the 64 x 64 diagonal block -------------------------------------------
-// S (row stride FS) holds the updated block's lower triangle; X receives
-// L^-1 (zeros above the diagonal).  Two 32-column halves: one warp factors a
-// 32 x 32 block with a row per lane, each new column broadcast through
-// shared memory (its transpose Lt serves the inverse as well), the products
-// between the halves run on the tensor cores of all 8 warps.
-constexpr int LTS = 34;
+// S (row stride FS) holds the updated block's lower triangle, overwritten
+// with L; X receives L^-1 (zeros above the diagonal).  Eight 8-column panels:
+// warp 0 factors a panel (two rows per lane, the pivot row's entries by
+// shuffles), all warps then update the next panel's columns, and while warp 0
+// factors on, the other seven update the rest and build the inverse behind
+// it.  Bound by the chain of 64 pivots (reciprocal square root, product,
+// shuffle).  The code is kept small on purpose: straight-line 32-column
+// panels ran at the instruction fetch's pace (58 000 cycles a block; 29 000 now, 2 300 a panel).
 
-__device__ void warp_potrf32(double* S, double* Lt, double* dinv, int lane, int col0, int n_valid, int* bad,
-                             double ref, double* logsum) {
-  double a[32];
+// The shift stays apart from the diagonal (whose updates then round at the
+// source matrix's size, not at the shift's) and is added to form the pivot;
+// the logarithm of (x + shift) / (c2 + shift) is log1p((x - c2) * ref).
+struct DiagShift {
+  double shift, c2, ref;
+};
+
+__device__ __forceinline__ void panel8(double* S, int s, int lane, double shift, int col0, int n, int* bad,
+                                       double* dinv, double* diagx) {
+  const int r0 = 8 * s + lane, r1 = r0 + 32;
+  double a0[8], a1[8];
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {
-    const double2 v = *reinterpret_cast<const double2*>(S + lane * FS + j);
-    a[j] = v.x;
-    a[j + 1] = v.y;
+  for (int j = 0; j < 8; j += 2) {
+    double2 v = make_double2(0.0, 0.0), w = v;
+    if (r0 < NB) v = *reinterpret_cast<const double2*>(S + r0 * FS + 8 * s + j);
+    if (r1 < NB) w = *reinterpret_cast<const double2*>(S + r1 * FS + 8 * s + j);
+    a0[j] = v.x;
+    a0[j + 1] = v.y;
+    a1[j] = w.x;
+    a1[j + 1] = w.y;
   }
-  double mypiv = 1.0;
+  // the chain pivot -> rsqrt -> entry below it -> next pivot: a lane forms its
+  // own next pivot (its diagonal entry before the shift is kept for the
+  // logarithm), the sign test is on the pivot's high word
+  double x = a0[0];
+  double piv = x + shift;
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    double piv = __shfl_sync(0xffffffffu, a[c], c);
-    if (!(piv > 0.0)) {          // not SPD (or NaN): the first failing column, factor on with a unit pivot
-      if (*bad == 0 && col0 + c < n_valid) *bad = col0 + c + 1;
+  for (int c = 0; c < 8; ++c) {
+    if (lane == c) diagx[8 * s + c] = x;
+    piv = __shfl_sync(0xffffffffu, piv, c);
+    if ((unsigned)(__double2hiint(piv) - 0x00100000) >= 0x7fe00000u) {
+      // not SPD (or NaN): the first failing column; factor on with a unit pivot
+      if (*bad == 0 && col0 + 8 * s + c < n) *bad = col0 + 8 * s + c + 1;
       piv = 1.0;
     }
     const double inv = rsqrt(piv);
-    if (lane == c) {
-      mypiv = piv;
-      dinv[c] = inv;
+    const double u = a0[c] * inv;
+    if (c < 7) {
+      x = fma(-u, u, a0[c + 1]);
+      piv = fma(-u, u, a0[c + 1] + shift);
     }
-    const double l = lane > c ? a[c] * inv : (lane == c ? piv * inv : 0.0);
-    a[c] = l;
-    Lt[c * LTS + lane] = l;
-    __syncwarp();
-    if (c + 1 < 32) {
-      if ((c + 1) & 1) a[c + 1] -= l * Lt[c * LTS + c + 1];
+    const double l0 = lane > c ? u : 0.0;   // L's own diagonal is not needed, only its reciprocal
+    const double l1 = a1[c] * inv;
+    if (lane == c) dinv[8 * s + c] = inv;
 #pragma unroll
-      for (int j = (c + 2) & ~1; j < 32; j += 2) {
-        const double2 q = *reinterpret_cast<const double2*>(Lt + c * LTS + j);
-        a[j] -= l * q.x;
-        a[j + 1] -= l * q.y;
-      }
+    for (int j = c + 1; j < 8; ++j) {
+      const double lj = __shfl_sync(0xffffffffu, l0, j);
+      a0[j] = fma(-l0, lj, a0[j]);
+      a1[j] = fma(-l1, lj, a1[j]);
     }
+    a0[c] = l0;
+    a1[c] = l1;
   }
 #pragma unroll
-  for (int j = 0; j < 32; j += 2)
-    *reinterpret_cast<double2*>(S + lane * FS + j) = make_double2(a[j], a[j + 1]);
-  if (logsum) {
-    double lg = (col0 + lane < n_valid) ? log(mypiv * ref) : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
-    *logsum = lg;
+  for (int j = 0; j < 8; j += 2) {
+    if (r0 < NB) *reinterpret_cast<double2*>(S + r0 * FS + 8 * s + j) = make_double2(a0[j], a0[j + 1]);
+    if (r1 < NB) *reinterpret_cast<double2*>(S + r1 * FS + 8 * s + j) = make_double2(a1[j], a1[j + 1]);
   }
+}
+
+// C(i, j) -= L(i, s) L(j, s)^T, 8 x 8 blocks; one warp.
+__device__ __forceinline__ void update8(double* S, int i, int j, int s, int g, int q) {
+  double2* c = reinterpret_cast<double2*>(S + (8 * i + g) * FS + 8 * j + 2 * q);
+  double2 v = *c;
+#pragma unroll
+  for (int kk = 0; kk < 8; kk += 4)
+    dmma(v.x, v.y, -S[(8 * i + g) * FS + 8 * s + kk + q], S[(8 * j + g) * FS + 8 * s + kk + q]);
+  *c = v;
+}
+
+// X(s, s) = L(s, s)^-1, a column per lane; one warp.
+__device__ __forceinline__ void inverse8(const double* S, const double* dinv, double* X, int s, int lane) {
+  double x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    x[i] *= dinv[8 * s + i];
+#pragma unroll
+    for (int k = i + 1; k < 8; ++k) x[k] = fma(-S[(8 * s + k) * FS + 8 * s + i], x[i], x[k]);
+  }
+  if (lane < 8)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) X[(8 * s + i) * FS + 8 * s + lane] = x[i];
+}
+
+// X(s, j) = -X(s, s) sum_{k=j}^{s-1} L(s, k) X(k, j); one warp.
+__device__ __forceinline__ void inverse_row8(const double* S, double* X, int s, int j, int g, int q) {
+  double2 w = make_double2(0.0, 0.0);
+  for (int kk = 8 * j; kk < 8 * s; kk += 4) dmma(w.x, w.y, S[(8 * s + g) * FS + kk + q], X[(kk + q) * FS + 8 * j + g]);
+  double2* out = reinterpret_cast<double2*>(X + (8 * s + g) * FS + 8 * j + 2 * q);
+  *out = w;
   __syncwarp();
-}
-
-// X (32 x 32, row stride FS) = L^-1, a column per lane; Lt, dinv from warp_potrf32.
-__device__ void warp_inv32(const double* Lt, const double* dinv, double* X, int lane) {
-  double x[32];
+  double2 v = make_double2(0.0, 0.0);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = (i == lane) ? 1.0 : 0.0;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const double xi = x[i] * dinv[i];
-    x[i] = xi;
-    if (i + 1 < 32) {
-      if ((i + 1) & 1) x[i + 1] -= xi * Lt[i * LTS + i + 1];
-#pragma unroll
-      for (int j = (i + 2) & ~1; j < 32; j += 2) {
-        const double2 q = *reinterpret_cast<const double2*>(Lt + i * LTS + j);
-        x[j] -= xi * q.x;
-        x[j + 1] -= xi * q.y;
-      }
-    }
-    X[i * FS + lane] = xi;
-  }
+  for (int kk = 0; kk < 8; kk += 4)
+    dmma(v.x, v.y, -X[(8 * s + g) * FS + 8 * s + kk + q], X[(8 * s + kk + q) * FS + 8 * j + g]);
   __syncwarp();
+  *out = v;
 }
 
-// acc (16 x 8 of a 32 x 32 product, this warp's part) += A B^T (bt) or A B
-// over K = 32; A, B in shared memory with row stride FS.
-template <bool BT>
-__device__ __forceinline__ void mma32(const double* A, const double* B, int warp, int lane, double acc[2][2]) {
-  const int g = lane >> 2, q = lane & 3;
-  const int r0 = (warp >> 2) * 16, c0 = (warp & 3) * 8;
-#pragma unroll
-  for (int kk = 0; kk < 32; kk += 4) {
-    const double b = BT ? B[(c0 + g) * FS + kk + q] : B[(kk + q) * FS + c0 + g];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) dmma(acc[i][0], acc[i][1], A[(r0 + 8 * i + g) * FS + kk + q], b);
-  }
-}
-
-// Factors S (64 x 64) and inverts the factor into X.  All 256 threads.
-__device__ void diag_factor(double* S, double* X, double* Lt, double* dinv, int tid, int col0, int n, int* bad,
-                            double ref, double* logsum) {
+// Factors S and inverts the factor into X; dinv, diagx: 64 doubles each.
+// All 256 threads.
+__device__ __forceinline__ void diag_factor(double* S, double* X, double* dinv, double* diagx, int tid, int col0,
+                                            int n, int* bad, double shift) {
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  const int r0 = (warp >> 2) * 16, c0 = (warp & 3) * 8;
-  double* A21 = S + 32 * FS;
-  double* A22 = S + 32 * FS + 32;
-  double* X21 = X + 32 * FS;
-  double* X22 = X + 32 * FS + 32;
-  double lg0 = 0.0, lg1 = 0.0;
-  if (warp == 0) {
-    warp_potrf32(S, Lt, dinv, lane, col0, n, bad, ref, logsum ? &lg0 : nullptr);
-    warp_inv32(Lt, dinv, X, lane);
-  } else if (warp == 1) {
-    for (int r = 0; r < 32; ++r) X[r * FS + 32 + lane] = 0.0;
-  }
+  for (int e = tid; e < NB * FS / 2; e += kFlowThreads) reinterpret_cast<double2*>(X)[e] = make_double2(0.0, 0.0);
   __syncthreads();
-  {   // L21 = A21 L11^-T
-    double acc[2][2] = {};
-    mma32<true>(A21, X, warp, lane, acc);
+#pragma unroll 1
+  for (int s = 0; s < 10; ++s) {
+    // warp 0: panel s.  The others: what panel s - 1 does to the columns
+    // past s, the inverse of diagonal block s - 1, row s - 2 of the inverse
+    if (warp == 0) {
+      if (s < 8) panel8(S, s, lane, shift, col0, n, bad, dinv, diagx);
+    } else {
+      if (warp == 1 && s >= 1 && s <= 8) inverse8(S, dinv, X, s - 1, lane);
+      if (s >= 2 && warp <= s - 2) inverse_row8(S, X, s - 2, warp - 1, g, q);
+      if (s >= 1 && s < 8) {
+        int t = 7 - warp;   // tiles (i, j), s < j <= i < 8, dealt from warp 7 down
+        for (int j = s + 1; j < 8; ++j)
+          for (int i = j; i < 8; ++i)
+            if (--t < 0) {
+              update8(S, i, j, s - 1, g, q);
+              t = 6;
+            }
+      }
+    }
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      *reinterpret_cast<double2*>(A21 + (r0 + 8 * i + g) * FS + c0 + 2 * q) = make_double2(acc[i][0], acc[i][1]);
-  }
-  __syncthreads();
-  {   // A22 -= L21 L21^T
-    double acc[2][2] = {};
-    mma32<true>(A21, A21, warp, lane, acc);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      double2* p = reinterpret_cast<double2*>(A22 + (r0 + 8 * i + g) * FS + c0 + 2 * q);
-      double2 v = *p;
-      v.x -= acc[i][0];
-      v.y -= acc[i][1];
-      *p = v;
+    if (s < 7) {   // panel s on the columns of panel s + 1
+      if (s + 1 + warp < 8) update8(S, s + 1 + warp, s + 1, s, g, q);
+      __syncthreads();
     }
   }
-  // W = L21 L11^-1, kept in registers while warp 0 factors A22
-  double w[2][2] = {};
-  mma32<false>(A21, X, warp, lane, w);
-  __syncthreads();
-  if (warp == 0) {
-    warp_potrf32(A22, Lt, dinv, lane, col0 + 32, n, bad, ref, logsum ? &lg1 : nullptr);
-    warp_inv32(Lt, dinv, X22, lane);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i)   // L21 is no longer needed: W takes its place
-    *reinterpret_cast<double2*>(A21 + (r0 + 8 * i + g) * FS + c0 + 2 * q) = make_double2(w[i][0], w[i][1]);
-  __syncthreads();
-  {   // X21 = -L22^-1 W
-    double acc[2][2] = {};
-    mma32<false>(X22, A21, warp, lane, acc);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      *reinterpret_cast<double2*>(X21 + (r0 + 8 * i + g) * FS + c0 + 2 * q) = make_double2(-acc[i][0], -acc[i][1]);
-  }
-  if (logsum && tid == 0) *logsum = lg0 + lg1;
-  __syncthreads();
 }
 
 // ---- the launch -------------------------------------------------------------
 __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs a) {
   extern __shared__ __align__(16) double dsm[];
-  __shared__ double s_dinv[32];
-  __shared__ double s_log;
+  __shared__ double s_dinv[NB], s_diagx[NB];
   __shared__ int s_ticket, s_avail, s_bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, q4 = lane & 3;
@@ -373,7 +363,6 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
       if (tid == 0) s_bad = 0;
       __syncthreads();
       if (half == 0 && !idle) {
-        const double sh = a.shift ? a.shift[b] : 0.0;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -382,26 +371,33 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
             for (int h = 0; h < 2; ++h) {
               const int rr = wr + 8 * i + g, cc = wc + 8 * j + 2 * q4 + h;
               double v = -(acc[i][j][h] + S[rr * FS + cc]);
-              if (rr == cc) v += sh;
               if (col0 + rr >= a.n || col0 + cc >= a.n) v = rr == cc ? 1.0 : 0.0;   // identity padding
               S[rr * FS + cc] = v;
             }
       }
       __syncthreads();
-      diag_factor(S, X, X + (size_t)NB * FS, s_dinv, tid, col0, a.n, &s_bad, a.ref ? a.ref[b] : 1.0, a.logdet ? &s_log : nullptr);
+      DiagShift ds{0.0, 0.0, 0.0};
+      if (a.shift) ds = DiagShift{a.shift[b], *a.c2, a.ref[b]};
+      diag_factor(S, X, s_dinv, s_diagx, tid, col0, a.n, &s_bad, ds.shift);
       double* Li = a.linv + (size_t)b * a.linv_stride + (size_t)k * NB * NB;
       for (int e = tid; e < NB * NB / 2; e += kFlowThreads) {
         const int rr = e / (NB / 2), cc = 2 * (e % (NB / 2));
         *reinterpret_cast<double2*>(Li + rr * NB + cc) = *reinterpret_cast<const double2*>(X + rr * FS + cc);
       }
-      if (tid == 0) {
-        if (s_bad) atomicCAS(&a.info[b], 0, s_bad);
-        if (a.logdet) a.logdet[(size_t)b * T + k] = s_log;
-      }
       __syncthreads();
       if (tid == 0) {
+        if (s_bad) atomicCAS(&a.info[b], 0, s_bad);
         __threadfence();
         st_release(diag + b, k + 1);
+      }
+      if (a.logdet && warp == 1) {   // off the chain
+        double lg = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (col0 + lane + 32 * h < a.n) lg += log1p((s_diagx[lane + 32 * h] - ds.c2) * ds.ref);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
+        if (lane == 0) a.logdet[(size_t)b * T + k] = lg;
       }
       continue;
     }
@@ -422,37 +418,31 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
     cp_commit();
     cp_wait<0>();
     __syncthreads();
+    // 64 rows at a time, so that the block row the next diagonal block waits
+    // for is out first; a warp takes 8 rows and, of the inverse's lower
+    // triangle, the blocks that are not zero
+    for (int h = 0; h <= (two ? 1 : 0); ++h) {
+      const double* Sr = S + (64 * h + 8 * warp + g) * FS;
+      double o[8][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 8; ++j) o[j][0] = o[j][1] = 0.0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    const int kmax = wc + 32;                        // the inverse is lower triangular
-#pragma unroll 4
-    for (int kk = 0; kk < kmax; kk += 4) {
-      double af[4], bf[4];
+      for (int kk = 0; kk < NB; kk += 4) {
+        const double af = Sr[kk + q4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) af[i] = S[(wr + 8 * i + g) * FS + kk + q4];
+        for (int j = kk / 8; j < 8; ++j) dmma(o[j][0], o[j][1], af, X[(8 * j + g) * FS + kk + q4]);
+      }
+      const int rr = row0 + 64 * h + 8 * warp + g;
+      if (rr < a.n) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = X[(wc + 8 * j + g) * FS + kk + q4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rr = row0 + wr + 8 * i + g;
-      if (rr < a.n)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          *reinterpret_cast<double2*>(L + (size_t)rr * a.ld + col0 + wc + 8 * j + 2 * q4) =
-              make_double2(acc[i][j][0], acc[i][j][1]);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      st_release(done_b + rb0, k + 1);
-      if (two) st_release(done_b + rb0 + 1, k + 1);
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<double2*>(L + (size_t)rr * a.ld + col0 + 8 * j + 2 * q4) = make_double2(o[j][0], o[j][1]);
+      }
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        st_release(done_b + rb0 + h, k + 1);
+      }
     }
   }
 }

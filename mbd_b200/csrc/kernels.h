@@ -85,8 +85,11 @@ struct CholFlowArgs {
   const double* shift;     // [batch] added to the diagonal; null: none
   double* linv;
   size_t linv_stride;
-  double* logdet;          // [batch][ceil(n/64)]: sum of log(pivot * ref) of a diagonal block; null: not wanted
+  // with shifts: [batch][ceil(n/64)] sum over a diagonal block of
+  // log(pivot / (c2 + shift)), ref = 1 / (c2 + shift)
+  double* logdet;
   const double* ref;       // [batch]
+  const double* c2;        // [1]
   int* info;               // [batch]: first failing column + 1 where a pivot is not positive; zeroed by the caller
   int* sync;               // chol_flow_sync_ints(n, batch) ints
   int* err;                // the context's error flag (a wait that ran out)
