@@ -186,7 +186,10 @@ int mbd_rsscs_vdw_params(int z, double* alpha0, double* c6, double* r0);
  * With n >= 10 also [8] the dense -> band part of [6] and [9] the rest;
  * with n >= 12 also [10] the one-stage (dense -> tridiagonal) launch of the
  * matrices that skip the band and [11] the band -> tridiagonal launch, the
- * two batch-wide launches [9] is made of.  n must be >= 8. */
+ * two batch-wide launches [9] is made of.  Geometries whose energy is taken
+ * from shifted Cholesky factors of their Hamiltonian skip [6]; that stage is
+ * part of [7] and, with n >= 13, [12] (summed over the geometries).  n must
+ * be >= 8. */
 int mbd_rsscs_last_timings(mbd_ctx* ctx, double* ms, int n);
 
 /* Counters of the last upload/compute/download: [0] kernel launches issued

@@ -468,8 +468,14 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   launch_cfdm_build(cb, s);
   ctx->launches += 1;
   mark(5);
-  // 6. dense -> band (stage 1 of the two-stage tridiagonalisation)
-  if (two_stage(ctx, p.nH)) {
+  // 6. the energy from shifted Cholesky factors, or dense -> band (stage 1 of
+  // the two-stage tridiagonalisation)
+  if (gd->trace) {
+    TraceArgs ta{gd->hmat.as<double>(), p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
+                 sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag};
+    MBD_CUDA(launch_trace_energy(ta, ctx->num_sms, s));
+    ctx->launches += kTraceLaunches;
+  } else if (two_stage(ctx, p.nH)) {
     MBD_CUDA(launch_sy2sb(gd->hmat.as<double>(), p.ldH, p.nH, sl.trd_ws.as<double>(), gd->band.as<double>(),
                           ctx->num_sms, s, tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),
                           lookahead_for(ctx, sl.la)));
@@ -481,13 +487,23 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
 
 namespace {
 
-// Eigen stages of one geometry on stream s with its own launches (the
-// residual-gate fallback of download; run_front has reduced a two-stage
-// geometry's Hamiltonian to its band already).
+// Eigen stages of one geometry on stream s with its own launches: the
+// residual-gate fallback of download (run_front has reduced a two-stage
+// geometry's Hamiltonian to its band already), and a refused trace form.
 int run_tail_single(mbd_ctx* ctx, GeomDev* gd, cudaStream_t s) {
   const GeomPlan& p = gd->plan;
   if (two_stage(ctx, p.nH)) {
-    int st = band_to_tridiag_single(ctx, gd->band.as<double>(), p.nH, gd->d, gd->e, ctx->fb_ws, s);
+    double* band = gd->band.as<double>();
+    if (gd->trace) {   // refused: the Hamiltonian is still whole
+      MBD_CUDA(ctx->fb_band.reserve(sizeof(double) * (size_t)p.nH * kBandLd));
+      MBD_CUDA(ctx->fb_trd.reserve(sizeof(double) * sy2sb_workspace_doubles(p.nH)));
+      band = ctx->fb_band.as<double>();
+      MBD_CUDA(launch_sy2sb(gd->hmat.as<double>(), p.ldH, p.nH, ctx->fb_trd.as<double>(), band, ctx->num_sms, s,
+                            tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),
+                            lookahead_for(ctx, ctx->slots[gd->slot]->la)));
+      ctx->launches += sy2sb_launches(p.nH);
+    }
+    int st = band_to_tridiag_single(ctx, band, p.nH, gd->d, gd->e, ctx->fb_ws, s);
     if (st != MBD_OK) return st;
   } else {
     TridiagJob job{gd->hmat.as<double>(), p.nH, p.ldH, gd->d, gd->e};
@@ -515,6 +531,16 @@ size_t plain_bytes(const GeomPlan& p, size_t* relay, size_t* linv, size_t* rhs, 
   return *relay + *linv + *rhs + *sync;
 }
 
+// The trace form's factors and inverses (they take the relay's buffers, used
+// up by then) and its own workspace.
+size_t trace_bytes(const GeomPlan& p, size_t* factors, size_t* linv, size_t* ws) {
+  const int nblk = (p.nH + kCholNB - 1) / kCholNB;
+  *factors = sizeof(double) * (size_t)kTraceBatch * p.nH * p.ldH;
+  *linv = sizeof(double) * (size_t)kTraceBatch * nblk * kCholNB * kCholNB;
+  *ws = trace_ws_bytes(p.nH);
+  return *factors + *linv + *ws;
+}
+
 size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, size_t* res, size_t* sync) {
   *r32 = sizeof(float) * (size_t)kNFreq * p.n * p.ld;
   *pan = sizeof(float) * (size_t)kNFreq * round_up(p.n, kMixNB) * kMixNB;
@@ -526,13 +552,23 @@ size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, siz
 
 // Assigns the geometries to relay slots (longest first onto the least loaded
 // slot, load = (3N)^3), with as many slots as fit in the device memory share.
-int plan_slots(mbd_ctx* ctx) {
+int plan_slots(mbd_ctx* ctx, bool eigen) {
   const int ng = (int)ctx->order.size();
   size_t free_b = 0, total_b = 0;
   MBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
   size_t held = 0;
   for (auto& s : ctx->slots) held += s->held();
   const double budget = kSlotMemoryShare * (double)(free_b + held);
+  // Energies as traces: not while an eigenvalue kernel is asked for (its
+  // environment switches, the stalled chase of the failure tests), nor for
+  // Hamiltonians so large that the factors would not fit a share of the memory
+  for (auto& gd : ctx->geoms) gd->trace = false;
+  if (eigen && ctx->trace_form && !ctx->test_stall_wait)
+    for (int g : ctx->order) {
+      size_t a, b, c;
+      GeomDev& gd = *ctx->geoms[g];
+      gd.trace = gd.plan.nH <= kTraceMaxN && (double)trace_bytes(gd.plan, &a, &b, &c) <= 0.5 * budget;
+    }
   int S = std::max(1, std::min(kMaxSlots, ng));
   std::vector<int> slot_of(ctx->geoms.size(), 0);
   for (; S >= 1; --S) {
@@ -544,7 +580,14 @@ int plan_slots(mbd_ctx* ctx) {
       slot_of[g] = s;
       load[s] += std::pow((double)p.n, 3.0);
       size_t a, b, c, d, e, f, h;
-      need[s] = std::max(need[s], plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a));
+      size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a);
+      // the trace form's factors past what the relay's matrices leave
+      if (ctx->geoms[g]->trace) {
+        plain_bytes(p, &a, &b, &c, &h);
+        bytes += trace_bytes(p, &d, &e, &f);
+        bytes -= std::min(a, d) + std::min(b, e);
+      }
+      need[s] = std::max(need[s], bytes);
     }
     double total = 0.0;
     for (size_t x : need) total += (double)x;
@@ -587,9 +630,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
                    [&](int a, int b) { return ctx->geoms[a]->plan.n > ctx->geoms[b]->plan.n; });
   for (int g : ctx->order) {
     const GeomPlan& p = ctx->geoms[g]->plan;
-    if (!eigen) continue;
-    MBD_CUDA(ctx->geoms[g]->hmat.reserve(sizeof(double) * (size_t)p.nH * p.ldH));
-    if (two_stage(ctx, p.nH)) MBD_CUDA(ctx->geoms[g]->band.reserve(sizeof(double) * (size_t)p.nH * kBandLd));
+    if (eigen) MBD_CUDA(ctx->geoms[g]->hmat.reserve(sizeof(double) * (size_t)p.nH * p.ldH));
   }
   const size_t nev = ctx->geoms.size() * kGeomEvents;
   while (ctx->events.size() < nev) {
@@ -602,28 +643,44 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
     ctx->n_trd_groups = ctx->trd_total_ctas = ctx->n_eig_jobs = ctx->n_eig_batch = 0;
     return MBD_OK;
   }
-  int st = plan_slots(ctx);
+  int st = plan_slots(ctx, eigen);
   if (st != MBD_OK) return st;
+  // geometries whose energy comes from eigenvalues, by the two-stage reduction
+  auto banded = [&](int g) {
+    const GeomDev& gd = *ctx->geoms[g];
+    return !gd.trace && two_stage(ctx, gd.plan.nH);
+  };
+  if (eigen)
+    for (int g : ctx->order)
+      if (banded(g))
+        MBD_CUDA(ctx->geoms[g]->band.reserve(sizeof(double) * (size_t)ctx->geoms[g]->plan.nH * kBandLd));
   for (int s = 0; s < ctx->n_slots; ++s) {
-    size_t relay = 0, linv = 0, rhs = 0, sync = 0;
+    size_t relay = 0, linv = 0, rhs = 0, sync = 0, trace = 0;
     for (int g : ctx->order) {
-      if (ctx->geoms[g]->slot != s) continue;
+      const GeomDev& gd = *ctx->geoms[g];
+      if (gd.slot != s) continue;
       size_t a, b, c, d;
-      plain_bytes(ctx->geoms[g]->plan, &a, &b, &c, &d);
+      plain_bytes(gd.plan, &a, &b, &c, &d);
       relay = std::max(relay, a);
       linv = std::max(linv, b);
       rhs = std::max(rhs, c);
       sync = std::max(sync, d);
+      if (!gd.trace) continue;
+      trace_bytes(gd.plan, &a, &b, &c);
+      relay = std::max(relay, a);
+      linv = std::max(linv, b);
+      trace = std::max(trace, c);
     }
     RelaySlot& sl = *ctx->slots[s];
     MBD_CUDA(sl.relay64.reserve(relay));
     MBD_CUDA(sl.linv.reserve(linv));
     MBD_CUDA(sl.rhs.reserve(rhs));
     MBD_CUDA(sl.chol_sync.reserve(sync));
+    MBD_CUDA(sl.trace_ws.reserve(trace));
     if (eigen) {
       size_t tw = 0;
       for (int g : ctx->order)
-        if (ctx->geoms[g]->slot == s && two_stage(ctx, ctx->geoms[g]->plan.nH))
+        if (ctx->geoms[g]->slot == s && banded(g))
           tw = std::max(tw, sizeof(double) * sy2sb_workspace_doubles(ctx->geoms[g]->plan.nH));
       MBD_CUDA(sl.trd_ws.reserve(tw));
     }
@@ -635,7 +692,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   // one-stage tridiagonal plan for the matrices too large for the two-stage path
   std::vector<int> sizes, one_stage;
   for (int g : ctx->order)
-    if (!two_stage(ctx, ctx->geoms[g]->plan.nH)) {
+    if (!ctx->geoms[g]->trace && !two_stage(ctx, ctx->geoms[g]->plan.nH)) {
       sizes.push_back(ctx->geoms[g]->plan.nH);
       one_stage.push_back(g);
     }
@@ -675,7 +732,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
       GeomDev* gd = ctx->geoms[g].get();
       const GeomPlan& p = gd->plan;
       const bool fits = p.nH <= kEigBatchMaxN;
-      if (fits != (pass == 0)) continue;
+      if (gd->trace || fits != (pass == 0)) continue;
       eig.push_back(EigJob{gd->d, gd->e, gd->ev, gd->scalars, gd->energy, p.nH, p.nsl});
       if (fits) ctx->eig_batch_max_n = std::max(ctx->eig_batch_max_n, p.nH);
       else ctx->eig_single.push_back(g);
@@ -693,14 +750,14 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   // launch's length
   int big = 0;
   for (int g : ctx->order)
-    if (two_stage(ctx, ctx->geoms[g]->plan.nH)) big = std::max(big, ctx->geoms[g]->plan.nH);
+    if (banded(g)) big = std::max(big, ctx->geoms[g]->plan.nH);
   const bool cluster_ok = ctx->cluster_chase && !ctx->test_stall_wait && big > 0 &&
                           big <= sb2st_cluster_max_n() && tuned_chase_c(ctx, big) != kChaseFlag;
   const int cap = cluster_ok ? sb2st_cluster_max_n() : 0;
   ctx->band_max_n = ctx->band_cluster_max_n = 0;
   for (int g : ctx->order) {
     GeomDev* gd = ctx->geoms[g].get();
-    if (!two_stage(ctx, gd->plan.nH)) continue;
+    if (!banded(g)) continue;
     const BandJob bj{gd->band.as<double>(), gd->plan.nH, gd->d, gd->e};
     if (bj.n <= cap) {
       bjobs.push_back(bj);
@@ -854,7 +911,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
     ctx->launches += 2;
   }
   launch_energy_batch(ctx->eig_jobs, ctx->n_eig_jobs, s);
-  ctx->launches += 1;
+  ctx->launches += ctx->n_eig_jobs > 0 ? 1 : 0;
   record_timing(ctx, ctx->bev[3], s);
   return cuda_status(cudaGetLastError());
 }
@@ -921,7 +978,7 @@ std::vector<long long> batch_signature(const mbd_ctx* ctx, int mode) {
     const GeomPlan& p = gd.plan;
     sig.insert(sig.end(), {p.N, p.nsl, p.nH, gd.slot, (long long)p.scs_shifts.size(),
                            (long long)p.cfdm_shifts.size(), (long long)p.diff_shift.size(),
-                           two_stage(ctx, p.nH) ? 1 : 0});
+                           gd.trace ? 2 : (two_stage(ctx, p.nH) ? 1 : 0)});
   }
   return sig;
 }
@@ -994,6 +1051,11 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
     const char* ts = std::getenv("MBD_B200_TWO_STAGE");
     ctx->two_stage_max_n = sy2sb_max_n();
     ctx->two_stage_force = (ts && ts[0] == '1') ? 1 : ((ts && ts[0] == '0') ? 0 : -1);
+    // MBD_B200_TRACE=0: every energy from eigenvalues; a switch that picks
+    // one of their kernels asks for them too
+    const char* tf = std::getenv("MBD_B200_TRACE");
+    ctx->trace_form = tf ? tf[0] != '0'
+                         : !(ts || std::getenv("MBD_B200_CLUSTER_CHASE") || std::getenv("MBD_B200_PANEL_QR"));
   }
   MBD_CUDA(init_sb2st_attributes());
   ctx->trd_ctas_per_sm = std::max(1, tridiag_max_ctas_per_sm());
@@ -1180,15 +1242,17 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
   };
   ctx->last_ms[Stage::kTotal] = elapsed(ctx->bev[0], ctx->bev[3]);
   ctx->last_ms[Stage::kTridiag] = elapsed(ctx->bev[1], ctx->bev[2]);
-  ctx->last_band_ms = 0.0;
+  ctx->last_band_ms = ctx->last_trace_ms = 0.0;
   ctx->last_chase_ms = ctx->last_ms[Stage::kTridiag];
   ctx->last_onestage_ms = elapsed(ctx->bev[1], ctx->bev[4]);
   ctx->last_sb2st_ms = elapsed(ctx->bev[4], ctx->bev[2]);
   ctx->last_ms[Stage::kEig] = elapsed(ctx->bev[2], ctx->bev[3]);
   for (int g : ctx->order) {
     cudaEvent_t* evs = ctx->events.data() + (size_t)g * kGeomEvents;
-    for (int k = 1; k < kGeomEvents; ++k) ctx->last_ms[k] += elapsed(evs[k - 1], evs[k]);   // [6]: dense -> band
-    ctx->last_band_ms += elapsed(evs[5], evs[6]);
+    for (int k = 1; k + 1 < kGeomEvents; ++k) ctx->last_ms[k] += elapsed(evs[k - 1], evs[k]);
+    const double last = elapsed(evs[kGeomEvents - 2], evs[kGeomEvents - 1]);
+    ctx->last_ms[ctx->geoms[g]->trace ? Stage::kEig : Stage::kTridiag] += last;
+    (ctx->geoms[g]->trace ? ctx->last_trace_ms : ctx->last_band_ms) += last;
   }
   int first = MBD_OK;
   for (size_t g = 0; g < ctx->geoms.size(); ++g) {
@@ -1235,12 +1299,28 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
       }
       if (!(worst <= ctx->residual_gate)) {
         int st = run_front(ctx, gd, (int)g, MBD_MODE_PLAIN_FP64);
-        if (st == MBD_OK) st = run_tail_single(ctx, gd, ctx->slots[gd->slot]->stream);
+        if (st == MBD_OK && !gd->trace) st = run_tail_single(ctx, gd, ctx->slots[gd->slot]->stream);
         if (st != MBD_OK) return st;
         const cudaStream_t ss = ctx->slots[gd->slot]->stream;
         MBD_CUDA(fetch(g, ss));   // the re-run's results replace the staged ones
         MBD_CUDA(cudaStreamSynchronize(ss));
         r.refine_iters = -1;
+      }
+    }
+    if (gd->trace && err == 0) {
+      // a refused trace form (an imaginary mode, or a Hamiltonian too near
+      // one): the eigenvalues, if the relay gave a Hamiltonian at all
+      const double* sc = reinterpret_cast<const double*>(host(g, gd->scalars));
+      const int* fi = reinterpret_cast<const int*>(host(g, gd->info));
+      bool relay_ok = sc[2] == 0.0;
+      for (int f = 0; f < 21; ++f) relay_ok = relay_ok && fi[f] == 0;
+      if (relay_ok && reinterpret_cast<const double*>(host(g, gd->energy))[3] != kTraceOk) {
+        const cudaStream_t ss = ctx->slots[gd->slot]->stream;
+        int st = run_tail_single(ctx, gd, ss);
+        if (st != MBD_OK) return st;
+        MBD_CUDA(cudaMemcpyAsync(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ss));
+        MBD_CUDA(fetch(g, ss));
+        MBD_CUDA(cudaStreamSynchronize(ss));
       }
     }
     const double* aiw = reinterpret_cast<const double*>(host(g, gd->alpha_iw));
@@ -1616,6 +1696,7 @@ int mbd_rsscs_last_timings(mbd_ctx* ctx, double* ms, int n) {
     ms[Stage::kCount + 2] = ctx->last_onestage_ms;   // the grouped one-stage launch alone
     ms[Stage::kCount + 3] = ctx->last_sb2st_ms;      // the bulge-chasing launch alone
   }
+  if (n >= Stage::kCount + 5) ms[Stage::kCount + 4] = ctx->last_trace_ms;   // the trace forms, summed over geometries
   return MBD_OK;
 }
 

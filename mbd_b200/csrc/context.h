@@ -91,6 +91,7 @@ struct GeomDev {
   double* cgstate;   // [21][kCgState] block-CG recurrence state (MIXED_LEARNED)
   int* info;
   int status_host = MBD_OK;
+  bool trace = false;   // energy from shifted Cholesky factors (k_trace.cu); eigenvalues only where that is refused
   int slot = 0;      // relay slot running this geometry's relay and CFDM stages
   // learned warm start: neighbour graph (built on first use), training data
   DevBuf graph;      // off, nbr, src, species (int); dvec, efeat, eproj (float)
@@ -116,6 +117,7 @@ struct RelaySlot {
   DevBuf relay32, p_hi, p_lo, l_hi, l_lo, mixv, res_ws, solve_sync;   // mixed path
   DevBuf cg, gnn;                                             // learned path: CG vectors, network work
   DevBuf trd_ws;                                              // dense -> band workspace
+  DevBuf trace_ws;                                            // trace form: bounds, nodes, counters
   int solve_epoch = 0;
   ~RelaySlot() {
     if (done) cudaEventDestroy(done);
@@ -126,7 +128,7 @@ struct RelaySlot {
   }
   size_t held() const {
     return relay64.bytes + linv.bytes + rhs.bytes + chol_sync.bytes + relay32.bytes + p_hi.bytes + p_lo.bytes + l_hi.bytes +
-           l_lo.bytes + mixv.bytes + res_ws.bytes + solve_sync.bytes + cg.bytes + gnn.bytes + trd_ws.bytes;
+           l_lo.bytes + mixv.bytes + res_ws.bytes + solve_sync.bytes + cg.bytes + gnn.bytes + trd_ws.bytes + trace_ws.bytes;
   }
 };
 
@@ -148,7 +150,7 @@ struct Stage {
   enum { kTotal = 0, kSetup, kBuild, kFactor, kSolve, kCfdm, kTridiag, kEig, kCount };
 };
 // Events per geometry: start, then the ends of setup, build, factor, solve,
-// CFDM build and dense -> band reduction.
+// CFDM build and dense -> band reduction (or trace form).
 constexpr int kGeomEvents = 7;
 
 
@@ -164,6 +166,7 @@ struct mbd_ctx {
   std::vector<std::unique_ptr<mbd::RelaySlot>> slots;
   int n_slots = 0;                           // slots in use for the current batch
   mbd::DevBuf tridiag_ws, tables, misc, fb_ws;
+  mbd::DevBuf fb_band, fb_trd;   // a refused trace form's reduction (never part of a graph)
   mbd::HostBuf staging;   // download: every geometry's results in one pass
   mbd::Sy2sbLookAhead la_ctx{};   // look-ahead stream and events of the context-stream reductions
   bool lookahead = true;     // dense -> band look-ahead (MBD_B200_LOOKAHEAD=0: off)
@@ -229,10 +232,11 @@ struct mbd_ctx {
   int two_stage_max_n = 0;                   // largest matrix the two-stage reduction takes on this device
   bool two_stage_batch = false;              // two-stage reduction for the matrices it can take
   int two_stage_force = -1;                  // 1 / 0: forced on / off; -1: policy
+  bool trace_form = true;                    // energies as traces where they apply (prepare_batch)
   bool capturing = false;
   int mode_runs[3] = {0, 0, 0};              // computes of the uploaded batch, per mode
   double last_ms[mbd::Stage::kCount] = {0};
-  double last_band_ms = 0.0, last_chase_ms = 0.0;
+  double last_band_ms = 0.0, last_chase_ms = 0.0, last_trace_ms = 0.0;
   double last_onestage_ms = 0.0, last_sb2st_ms = 0.0;   // the two batch-wide launches of last_chase_ms
   double launches = 0, h2d_bytes = 0, d2h_bytes = 0;
   int last_mode = 0;
@@ -323,6 +327,10 @@ int reserve_learned(mbd_ctx* ctx);
 // (grown as needed), on stream s.
 int band_to_tridiag_single(mbd_ctx* ctx, double* Br, int n, double* d, double* e, DevBuf& scratch, cudaStream_t s);
 int relay_learned(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cudaEvent_t ev_net, double** X_out);
+
+// Largest Hamiltonian the trace form takes: past it the reduction to a band,
+// (4/3) n^3 operations against ~4 n^3, is the faster one.
+constexpr int kTraceMaxN = 9216;
 
 // Matrices reduced by the two-stage path (the rest by the one-stage kernel).
 inline bool two_stage(const mbd_ctx* ctx, int n) {

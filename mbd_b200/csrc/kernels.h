@@ -267,6 +267,26 @@ int sb2st_cluster_min(int n);
 int sb2st_cluster_cmax();
 cudaError_t launch_sb2st_cluster(const BandJob* jobs, int n_jobs, int max_n, int C, cudaStream_t s);
 
+// ---- the energy as a trace (k_trace.cu) ----
+// sum_i sqrt(lambda_i) of the Hamiltonian from shifted Cholesky factors,
+// without its eigenvalues.  Node 0 certifies H - m I positive definite.
+constexpr int kTraceNodes = 20;                    // quadrature nodes at most
+constexpr int kTraceBatch = kTraceNodes + 1;
+struct TraceArgs {
+  const double* H;         // n x n, row-major lower, ld
+  int n, ld, nsl;
+  double* L;               // kTraceBatch factors of stride n * ld
+  double* linv;            // kTraceBatch * ceil(n/64) blocks of 64 x 64
+  void* ws;                // trace_ws_bytes(n)
+  const double* scalars;   // relay scalars ([1] = sum of 3 omega)
+  double* out;             // energy outputs: [0] E, [1] sum sqrt, [2] 0 negative, [3] kTraceOk or kTraceRefused
+  int* err;
+};
+constexpr double kTraceOk = 1.0, kTraceRefused = 2.0;
+size_t trace_ws_bytes(int n);
+constexpr int kTraceLaunches = 5;
+cudaError_t launch_trace_energy(const TraceArgs& a, int num_sms, cudaStream_t s);
+
 // ---- block-CG relay solve of the MIXED_LEARNED mode (UTILS.f90:469-473) ----
 constexpr int kCgState = 24;   // per-frequency recurrence state (doubles)
 constexpr int kCgIndefinite = 21;   // state slot: 1 when a search direction found p^T A p < 0
