@@ -17,9 +17,9 @@
 // Bound: FP64 tensor-core rate (36.9 TFLOP/s measured for m8n8k4 with all
 // operands in registers) while a block column has tiles for the whole chip;
 // below that the chain diagonal block -> tile below it -> next diagonal
-// block, n / 64 links of 20 us.  Measured, 21 relay matrices of n rows (right-looking
-// kernels before -> now): n = 3000 17.5 -> 7.6 ms (10.8 -> 24.9 TFLOP/s),
-// n = 384 0.85 -> 0.15 ms; n = 6000 50.7 ms (29.8 TFLOP/s).
+// block, n / 64 links of 19 us.  Measured, 21 relay matrices of n rows (right-looking
+// kernels before -> now): n = 3000 17.5 -> 7.0 ms (10.8 -> 27 TFLOP/s),
+// n = 384 0.85 -> 0.15 ms; n = 6000 49.5 ms (30.5 TFLOP/s).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -267,30 +267,6 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
     const double* src = a.src + (size_t)b * a.src_stride;
     double* L = a.L + (size_t)b * a.l_stride;
     int* done_b = done + (size_t)b * T;
-    // this warp's 32 x 32 part; the diagonal block's three lower quadrants go
-    // to warps 0-3 and 4-7, which take half of the columns of a stage each
-    const int wr = is_diag ? ((warp & 3) >> 1) * 32 : (warp >> 1) * 32;
-    const int wc = (warp & 1) * 32;
-    const int half = is_diag ? (warp >> 2) : 0;
-    const bool idle = is_diag && wc > wr;
-    double acc[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j][0] = acc[i][j][1] = 0.0;
-        const int rr = row0 + wr + 8 * i + g, cc = col0 + wc + 8 * j + 2 * q4;
-        if (half == 0 && !idle && rr < a.n) {
-          if (!is_diag || cc + 1 < a.n) {
-            const double2 v = *reinterpret_cast<const double2*>(src + (size_t)rr * a.src_ld + cc);
-            acc[i][j][0] = -v.x;
-            acc[i][j][1] = -v.y;
-          } else if (cc < a.n) {
-            acc[i][j][0] = -src[(size_t)rr * a.src_ld + cc];
-          }
-        }
-      }
-    const int n_chunks = k * (NB / KC);
     int avail = 0;                                   // block columns known to be finished for all operands
     auto await = [&](int want) {                     // block-uniform
       if (tid == 0) {
@@ -302,79 +278,88 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
       __syncthreads();
       avail = s_avail;
     };
-    auto issue = [&](int c) {
-      if (c < n_chunks) {
-        double* st = dsm + (c % kStages) * kStageElems;
-        const double* Lc = L + c * KC;
-        const int rows = is_diag ? NB : RT + NB;
-        for (int e = tid; e < rows * (KC / 2); e += kFlowThreads) {
-          const int rr = e / (KC / 2), cc = 2 * (e % (KC / 2));
-          // operand rows: the tile's 128, then the block column's own 64
-          const int gr = rr < RT && !is_diag ? row0 + rr : col0 + (is_diag ? rr : rr - RT);
-          const int ok = gr < a.n ? 16 : 0;
-          cp_async16(st + rr * KS + cc, Lc + (size_t)(ok ? gr : 0) * a.ld + cc, ok);
-        }
-      }
-      cp_commit();
-    };
-    if (n_chunks > 0) await(1);
-    for (int c = 0; c < kStages - 1; ++c) issue(c);    // n_chunks is 0 or >= 4: both in block column 0
-    for (int c = 0; c < n_chunks; ++c) {
-      cp_wait<kStages - 2>();
-      __syncthreads();
-      const int nx = c + kStages - 1, need = nx / (NB / KC) + 1;
-      const bool now = nx >= n_chunks || need <= avail;
-      if (now) issue(nx);
-      if (!idle) {
-        const double* As = dsm + (c % kStages) * kStageElems;
-        const double* Bs = is_diag ? As : As + RT * KS;
-#pragma unroll
-        for (int kk = 0; kk < KC; kk += 4) {
-          if (is_diag && (kk >= KC / 2) != (half == 1)) continue;
-          double af[4], bf[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) af[i] = As[(wr + 8 * i + g) * KS + kk + q4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) bf[j] = Bs[(wc + 8 * j + g) * KS + kk + q4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
-        }
-      }
-      if (!now) {
-        await(need);
-        issue(nx);
-      }
-    }
-    cp_wait<0>();
-    __syncthreads();
-    double* S = dsm;                                 // tile (128 or 64 rows, stride FS)
-    double* X = dsm + (size_t)(is_diag ? NB : RT) * FS;
     if (is_diag) {
-      if (half == 1 && !idle) {
+      // Lower triangle of the 8 x 8 blocks, a block row per warp: rows 7, 6,
+      // 5, 4 on warps 0-3 and 0-3 on warps 4-7, nine blocks for every
+      // sub-partition.  Whole block columns of L in two buffers: behind the
+      // last one, which the chain waits for, all of its loads are out at once.
+      const int bi = warp < 4 ? 7 - warp : warp - 4;
+      double acc[8][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<double2*>(S + (wr + 8 * i + g) * FS + wc + 8 * j + 2 * q4) =
-                make_double2(acc[i][j][0], acc[i][j][1]);
+      for (int j = 0; j < 8; ++j) {
+        acc[j][0] = acc[j][1] = 0.0;
+        const int rr = col0 + 8 * bi + g, cc = col0 + 8 * j + 2 * q4;
+        if (j <= bi && rr < a.n) {
+          if (cc + 1 < a.n) {
+            const double2 v = *reinterpret_cast<const double2*>(src + (size_t)rr * a.src_ld + cc);
+            acc[j][0] = -v.x;
+            acc[j][1] = -v.y;
+          } else if (cc < a.n) {
+            acc[j][0] = -src[(size_t)rr * a.src_ld + cc];
+          }
+        }
       }
+      auto issue = [&](int p) {
+        double* buf = dsm + (p & 1) * (NB * FS);
+        const double* Lp = L + p * NB;
+#pragma unroll
+        for (int c = 0; c < NB / KC; ++c) {
+          for (int e = tid; e < NB * (KC / 2); e += kFlowThreads) {
+            const int rr = e / (KC / 2), cc = KC * c + 2 * (e % (KC / 2));
+            const int ok = col0 + rr < a.n ? 16 : 0;
+            cp_async16(buf + rr * FS + cc, Lp + (size_t)(ok ? col0 + rr : 0) * a.ld + cc, ok);
+          }
+          cp_commit();
+        }
+      };
+      if (k > 0) {
+        await(1);
+        issue(0);
+      }
+      for (int p = 0; p < k; ++p) {
+        const bool next = p + 2 <= avail && p + 1 < k;
+        if (next) issue(p + 1);   // its buffer was last read before the barrier that closed block column p - 1
+        const double* buf = dsm + (p & 1) * (NB * FS);
+#pragma unroll
+        for (int c = 0; c < NB / KC; ++c) {
+          if (next) {
+            if (c == 0) cp_wait<7>();
+            if (c == 1) cp_wait<6>();
+            if (c == 2) cp_wait<5>();
+            if (c == 3) cp_wait<4>();
+          } else {
+            if (c == 0) cp_wait<3>();
+            if (c == 1) cp_wait<2>();
+            if (c == 2) cp_wait<1>();
+            if (c == 3) cp_wait<0>();
+          }
+          __syncthreads();
+#pragma unroll
+          for (int kk = KC * c; kk < KC * (c + 1); kk += 4) {
+            const double af = buf[(8 * bi + g) * FS + kk + q4];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (j <= bi) dmma(acc[j][0], acc[j][1], af, buf[(8 * j + g) * FS + kk + q4]);
+          }
+        }
+        __syncthreads();
+        if (!next && p + 1 < k) {
+          await(p + 2);
+          issue(p + 1);
+        }
+      }
+      double* S = dsm;
+      double* X = dsm + (size_t)NB * FS;
       if (tid == 0) s_bad = 0;
-      __syncthreads();
-      if (half == 0 && !idle) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int rr = wr + 8 * i + g, cc = wc + 8 * j + 2 * q4 + h;
-              double v = -(acc[i][j][h] + S[rr * FS + cc]);
-              if (col0 + rr >= a.n || col0 + cc >= a.n) v = rr == cc ? 1.0 : 0.0;   // identity padding
-              S[rr * FS + cc] = v;
-            }
-      }
+      for (int j = 0; j < 8; ++j)
+        if (j <= bi) {
+          const int rr = 8 * bi + g, cc = 8 * j + 2 * q4;
+          double2 v = make_double2(-acc[j][0], -acc[j][1]);
+          if (col0 + rr >= a.n || col0 + cc >= a.n) v.x = rr == cc ? 1.0 : 0.0;   // identity padding
+          if (col0 + rr >= a.n || col0 + cc + 1 >= a.n) v.y = rr == cc + 1 ? 1.0 : 0.0;
+          *reinterpret_cast<double2*>(S + rr * FS + cc) = v;
+        }
       __syncthreads();
       DiagShift ds{0.0, 0.0, 0.0};
       if (a.shift) ds = DiagShift{a.shift[b], *a.c2, a.ref[b]};
@@ -401,7 +386,70 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
       }
       continue;
     }
-    // tile: T = A - sum, then L = T Linv^T with the diagonal block's inverse
+    // tile: T = A - sum, then L = T Linv^T with the diagonal block's inverse;
+    // a 32 x 32 part per warp
+    const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int rr = row0 + wr + 8 * i + g, cc = col0 + wc + 8 * j + 2 * q4;
+        double2 v = make_double2(0.0, 0.0);
+        if (rr < a.n) v = *reinterpret_cast<const double2*>(src + (size_t)rr * a.src_ld + cc);
+        acc[i][j][0] = -v.x;
+        acc[i][j][1] = -v.y;
+      }
+    const int n_chunks = k * (NB / KC);
+    auto issue = [&](int c) {
+      if (c < n_chunks) {
+        double* st = dsm + (c % kStages) * kStageElems;
+        const double* Lc = L + c * KC;
+#pragma unroll 1
+        for (int u = 0; u < (RT + NB) * (KC / 2) / kFlowThreads; ++u) {
+          const int e = tid + u * kFlowThreads;
+          const int rr = e / (KC / 2), cc = 2 * (e % (KC / 2));
+          // operand rows: the tile's 128, then the block column's own 64
+          const int gr = rr < RT ? row0 + rr : col0 + rr - RT;
+          const int ok = gr < a.n ? 16 : 0;
+          cp_async16(st + rr * KS + cc, Lc + (size_t)(ok ? gr : 0) * a.ld + cc, ok);
+        }
+      }
+      cp_commit();
+    };
+    if (n_chunks > 0) await(1);
+    for (int c = 0; c < kStages - 1; ++c) issue(c);    // n_chunks is 0 or >= 4: both in block column 0
+    for (int c = 0; c < n_chunks; ++c) {
+      cp_wait<kStages - 2>();
+      __syncthreads();
+      const int nx = c + kStages - 1, need = nx / (NB / KC) + 1;
+      const bool now = nx >= n_chunks || need <= avail;
+      if (now) issue(nx);
+      const double* As = dsm + (c % kStages) * kStageElems + (wr + g) * KS + q4;
+      const double* Bs = dsm + (c % kStages) * kStageElems + (RT + wc + g) * KS + q4;
+      // unrolled by two: 30.5 TFLOP/s at n = 6000 against 28.5 by four (and 27 with
+      // the copy loop unrolled too): the copies and loads in a burst stall the MMAs
+#pragma unroll 2
+      for (int kk = 0; kk < KC; kk += 4) {
+        double af[4], bf[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) af[i] = As[8 * i * KS + kk];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bf[j] = Bs[8 * j * KS + kk];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+      }
+      if (!now) {
+        await(need);
+        issue(nx);
+      }
+    }
+    cp_wait<0>();
+    __syncthreads();
+    double* S = dsm;                                 // the tile, row stride FS
+    double* X = dsm + (size_t)RT * FS;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -464,7 +512,12 @@ cudaError_t launch_chol_flow(const CholFlowArgs& a, int num_sms, cudaStream_t s)
   const long long T = (a.n + NB - 1) / NB;
   long long tasks = 0;
   for (long long k = 0; k < T; ++k) tasks += a.batch * (1 + (T - k) / 2);
-  const int grid = (int)std::min<long long>(tasks, 2LL * num_sms);
+  // Every slot of the device where the products set the time; where the chain
+  // of diagonal blocks does (20 us a link), twice the CTAs it can keep at
+  // work, so that the waiting ones leave room for other streams' kernels.
+  const double work_us = a.batch * (double)a.n * a.n * a.n / 3.0 / 29e6, chain_us = 20.0 * T;
+  const double share = std::min(1.0, std::max(2.0 * work_us / chain_us, 6.0 * a.batch / (2.0 * num_sms)));
+  const int grid = (int)std::min<long long>(tasks, (long long)(2.0 * num_sms * share));
   chol_flow_kernel<<<grid, kFlowThreads, kFlowSmem, s>>>(a);
   return cudaGetLastError();
 }
