@@ -1041,6 +1041,7 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
   }
   MBD_CUDA(init_device_constants());
   MBD_CUDA(init_cholflow_attributes());
+  MBD_CUDA(init_cg_attributes());
   MBD_CUDA(init_eigval_attributes());
   MBD_CUDA(init_tc3_attributes());
   MBD_CUDA(init_mixed_attributes());

@@ -18,6 +18,7 @@
 //              later launch returns at once for that frequency
 // The 3x3 sums are added in one fixed order by every CTA, so all CTAs of a
 // launch take the same decisions.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -215,6 +216,16 @@ template <typename T>
 __device__ __forceinline__ typename Pair<T>::V load_pair(const T* A, size_t o) {
   return *reinterpret_cast<const typename Pair<T>::V*>(A + o);
 }
+// A float as a double by integer operations: the conversion instruction has a
+// sixteenth of the ALU's rate, and its queue set the FP32 pass's time.  Zeros
+// and denormals come out as some 1e-38, infinities and NaN as some 1e38 (the
+// residual gate turns such a solve away).
+__device__ __forceinline__ double widen(float x) {
+  const int b = __float_as_int(x);
+  return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
 // TA = double: the FP64 pass (FP64 products and sums).  TA = float: the pass
 // of the mixed-precision block-CG, products and the per-tile sums of 64
 // terms in FP32 (at 2x the FP64 rate: the FP32 pass would otherwise stay
@@ -300,7 +311,7 @@ __global__ void __launch_bounds__(TT, sizeof(TA) == 4 ? 4 : 3) cg_tile_kernel(Cg
     double y = 0.0;
     if (tid < CT * 3) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) y += (double)buf[k * RP + tid];
+      for (int k = 0; k < 16; ++k) y += widen(buf[k * RP + tid]);
     }
     __syncthreads();
     // column sums: the 16 row groups of each column
@@ -314,7 +325,7 @@ __global__ void __launch_bounds__(TT, sizeof(TA) == 4 ? 4 : 3) cg_tile_kernel(Cg
     if (tid < CT * 3) {
       double z = 0.0;
 #pragma unroll
-      for (int k = 0; k < 16; ++k) z += (double)buf[k * RP + tid];
+      for (int k = 0; k < 16; ++k) z += widen(buf[k * RP + tid]);
       if (!diag) {
         pr[((size_t)ti * a.nt + tj) * CT * 3 + tid] = y;
         pr[((size_t)tj * a.nt + ti) * CT * 3 + tid] = z;
@@ -546,11 +557,453 @@ __global__ void __launch_bounds__(AT) cg_dir_kernel(CgArgs a, int it) {
   }
 }
 
+// ---- all iterations of a phase in one launch -------------------------------
+// One thread-block cluster per frequency runs the FP32-pass iterations of
+// launch_cg_iteration to the end, with a cluster barrier where that has a
+// launch boundary: a converged frequency leaves at once, and a geometry costs
+// the host one launch a phase instead of four an iteration (a batch of 256
+// clusters issued 91 000 launches, 430 ms of host time).  Every CTA takes the
+// 3 x 3 decisions from the same records in the same order, so the cluster
+// stays uniform.
+//
+// Matrix pass: a CTA owns 64-row blocks in pairs from both ends (equal work)
+// and forms their products whole -- its rows up to the diagonal, then the
+// columns below it, 16 rows or columns to a warp -- so no partial sums leave
+// the CTA and nothing is reduced across lanes until a warp has swept its row.
+// An entry off the diagonal blocks is read twice (by its row's and its
+// column's owner): matrices of this size stay in L2, and the symmetric sweep
+// tried first spent more on the exchange than on the products.  Sums as in
+// cg_tile_kernel<float>: four products in FP32, everything beyond in FP64.
+// P is kept in shared memory of every CTA in FP32, written by its owners
+// through the cluster.
+constexpr int CLT = 256;
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// A warp's matrix chunks (32 lanes x 4 loads of 16 bytes) on their way, each
+// lane's own: a sweep is bound by the bytes it has in flight.
+constexpr int kRing = 4;
+__device__ __forceinline__ void ring_copy(float4* dst, const float* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// P in shared memory: per row (x, y, z, 0), and the three columns apart.
+struct PShared {
+  float4* row;     // [nt * 64 + 32]
+  float* col[3];   // [nt * 64 + 32] each
+};
+__host__ __device__ constexpr size_t p_shared_rows(int nt) { return (size_t)nt * CT + 32; }
+size_t p_shared_bytes(int nt) {
+  return p_shared_rows(nt) * (sizeof(float4) + 3 * sizeof(float)) + sizeof(float4) * kRing * 4 * CLT;
+}
+
+// d[4][3] over lanes that differ in the bits OFF, OFF/2, OFF/4: afterwards
+// out holds the sums of element ((lane / (OFF/2)) & 3).
+template <int OFF>
+__device__ __forceinline__ void scatter4(double (&d)[4][3], int lane, double (&out)[3]) {
+  const bool u1 = lane & OFF, u2 = lane & (OFF / 2);
+  double e[2][3];
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double send = u1 ? d[t][q] : d[t + 2][q], keep = u1 ? d[t + 2][q] : d[t][q];
+      e[t][q] = keep + __shfl_xor_sync(0xffffffffu, send, OFF);
+    }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double send = u2 ? e[0][q] : e[1][q], keep = u2 ? e[1][q] : e[0][q];
+    const double v = keep + __shfl_xor_sync(0xffffffffu, send, OFF / 2);
+    out[q] = v + __shfl_xor_sync(0xffffffffu, v, OFF / 4);
+  }
+}
+
+// out[16][3] = A[r0 .. r0 + 16)[0 .. diagonal] P, the diagonal included.
+// Lane: four columns of 32 (cg) and four rows (rg).  Rows past n repeat row
+// n - 1; their sums are not used.
+__device__ __forceinline__ void rows_task(const float* A, int ld, int n, const PShared& ps, int r0, int lane,
+                                          float4* ring, double* out) {
+  const int cg = lane & 7, rg = lane >> 3;
+  const float* Ar[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) Ar[t] = A + (size_t)min(r0 + 4 * rg + t, n - 1) * ld + 4 * cg;
+  double rs[4][3];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) rs[t][q] = 0.0;
+  const int chunks = r0 / 32 + 1;              // the last holds the diagonal
+  auto issue = [&](int c) {
+    if (c < chunks)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) ring_copy(ring + ((c & (kRing - 1)) * 4 + t) * 32 + lane, Ar[t] + 32 * c);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c = 0; c < kRing - 1; ++c) issue(c);
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+    float4 v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = ring[((c & (kRing - 1)) * 4 + t) * 32 + lane];
+    issue(c + kRing - 1);
+    const int gc = 32 * c + 4 * cg;
+    if (c + 1 == chunks) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int r = r0 + 4 * rg + t;
+        if (gc > r) v[t].x = 0.f;
+        if (gc + 1 > r) v[t].y = 0.f;
+        if (gc + 2 > r) v[t].z = 0.f;
+        if (gc + 3 > r) v[t].w = 0.f;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float4 x = *reinterpret_cast<const float4*>(ps.col[q] + gc);
+      const unsigned long long x01 = pack2(x.x, x.y), x23 = pack2(x.z, x.w);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        float lo, hi;
+        unpack2(fma2(pack2(v[t].z, v[t].w), x23, mul2(pack2(v[t].x, v[t].y), x01)), lo, hi);
+        rs[t][q] += widen(lo + hi);
+      }
+    }
+  }
+  double y[3];
+  scatter4<4>(rs, lane, y);
+  if ((lane & 1) == 0) {
+    double* o = out + (4 * rg + ((lane >> 1) & 3)) * 3;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o[q] = y[q];
+  }
+}
+
+// out[16][3] = (A[below the diagonal .. n)[c0 .. c0 + 16))^T P.  Lane: four
+// columns (cg) and every eighth row.  P is zero past n.
+__device__ __forceinline__ void cols_task(const float* A, int ld, int n, const PShared& ps, int c0, int lane,
+                                          float4* ring, double* out) {
+  const int cg = lane & 3, rp = lane >> 2;
+  const float* Ac = A + c0 + 4 * cg;
+  double cs[4][3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) cs[k][q] = 0.0;
+  const int chunks = (n - c0 + 31) / 32;
+  auto issue = [&](int c) {
+    if (c < chunks)
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        ring_copy(ring + ((c & (kRing - 1)) * 4 + t) * 32 + lane, Ac + (size_t)min(c0 + 32 * c + rp + 8 * t, n - 1) * ld);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c = 0; c < kRing - 1; ++c) issue(c);
+  for (int c = 0; c < chunks; ++c) {
+    const int R = c0 + 32 * c;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+    float4 v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = ring[((c & (kRing - 1)) * 4 + t) * 32 + lane];
+    issue(c + kRing - 1);
+    if (R == c0) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int r = R + rp + 8 * t, gc = c0 + 4 * cg;
+        if (gc >= r) v[t].x = 0.f;
+        if (gc + 1 >= r) v[t].y = 0.f;
+        if (gc + 2 >= r) v[t].z = 0.f;
+        if (gc + 3 >= r) v[t].w = 0.f;
+      }
+    }
+    unsigned long long c01[3], c23[3];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float4 x = ps.row[R + rp + 8 * t];
+      const unsigned long long e01 = pack2(v[t].x, v[t].y), e23 = pack2(v[t].z, v[t].w);
+      const float xq[3] = {x.x, x.y, x.z};
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const unsigned long long xx = pack2(xq[q], xq[q]);
+        c01[q] = t == 0 ? mul2(e01, xx) : fma2(e01, xx, c01[q]);
+        c23[q] = t == 0 ? mul2(e23, xx) : fma2(e23, xx, c23[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      float lo, hi;
+      unpack2(c01[q], lo, hi);
+      cs[0][q] += widen(lo);
+      cs[1][q] += widen(hi);
+      unpack2(c23[q], lo, hi);
+      cs[2][q] += widen(lo);
+      cs[3][q] += widen(hi);
+    }
+  }
+  double y[3];
+  scatter4<16>(cs, lane, y);
+  if ((lane & 4) == 0) {
+    double* o = out + (4 * cg + ((lane >> 3) & 3)) * 3;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o[q] = y[q];
+  }
+}
+
+// Records of the cluster's CTAs summed in order; totals for the whole CTA.
+__device__ __forceinline__ void sum_cluster_records(const double* rec, int C, double* out) {
+  if (threadIdx.x < kRed) {
+    double v = 0.0;
+    for (int k = 0; k < C; ++k) v += __ldcg(rec + k * kRed + threadIdx.x);
+    out[threadIdx.x] = v;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(CLT, 2) cg_cluster_kernel(CgArgs a, int it0, int it1) {
+  namespace cgr = cooperative_groups;
+  cgr::cluster_group cl = cgr::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int f = blockIdx.x / C;
+  extern __shared__ __align__(16) float4 xs[];
+  __shared__ double Rs[CT][3], Zp[4][CT][3], ys[2][2][CT * 3], sm[kRed * 32];
+  __shared__ double tot[kRed], s_zr[9], s_m[9];
+  __shared__ int s_flag;
+  if (stopped(a, f)) return;                     // uniform: the flag is raised behind cluster barriers only
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = a.n, nt = a.nt, pairs = (nt + 1) / 2;
+  const size_t prow = p_shared_rows(nt);
+  float* pc = reinterpret_cast<float*>(xs + prow);
+  const PShared ps{xs, {pc, pc + prow, pc + 2 * prow}};
+  float4* ring = reinterpret_cast<float4*>(pc + 3 * prow) + (tid >> 5) * (kRing * 4 * 32);
+  const float* A = a.A32 + (size_t)f * a.a_stride;
+  const size_t vo = (size_t)f * a.ystride;
+  double* rec1 = a.red + (size_t)f * nt * kRed;
+  double* rec2 = a.red2 + (size_t)f * nt * kRed;
+  double* st = a.state + f * kCgState;
+  if (tid < 9) s_zr[tid] = st[kZR0 + tid];
+  const int r = tid / 3, q = tid % 3;            // thread's row and column of a 64-row block (tid < 192)
+  for (int i = tid; i < (int)prow; i += CLT) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n) {
+      const double* p = a.P + vo + (size_t)3 * i;
+      x = make_float4((float)p[0], (float)p[1], (float)p[2], 0.f);
+    }
+    xs[i] = x;
+    pc[i] = x.x;
+    pc[prow + i] = x.y;
+    pc[2 * prow + i] = x.z;
+  }
+  cl.sync();
+  for (int it = it0; it < it1; ++it) {
+    // Q = A P on this CTA's blocks; its part of P^T Q
+    double vals[kRed];
+#pragma unroll
+    for (int k = 0; k < kRed; ++k) vals[k] = 0.0;
+    for (int p = rank; p < pairs; p += C) {
+      for (int e = 0; e < 2; ++e) {
+        const int I = e == 0 ? p : nt - 1 - p;
+        if (e == 1 && I == p) break;
+        const int r0 = I * CT + 16 * (warp & 3);
+        if (r0 < n) {
+          double* o = ys[e][warp >> 2] + 48 * (warp & 3);
+          if (warp < 4) rows_task(A, a.ld, n, ps, r0, lane, ring, o);
+          else cols_task(A, a.ld, n, ps, r0, lane, ring, o);
+        }
+      }
+      __syncthreads();
+      for (int e = 0; e < 2; ++e) {
+        const int I = e == 0 ? p : nt - 1 - p, gr = I * CT + r;
+        if (e == 1 && I == p) break;
+        if (tid < CT * 3 && gr < n) {
+          const size_t o = vo + (size_t)gr * 3;
+          const double y = ys[e][0][tid] + ys[e][1][tid];
+          a.Q[o + q] = y;
+          for (int c = 0; c < 3; ++c) {
+            const double t = a.P[o + c] * y;
+            if (q == 0) vals[3 * c] += t;
+            if (q == 1) vals[3 * c + 1] += t;
+            if (q == 2) vals[3 * c + 2] += t;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    cta_record(vals, sm, rec1 + rank * kRed);
+    cl.sync();
+    // alpha = (P^T Q)^-1 (Z^T R)
+    sum_cluster_records(rec1, C, tot);
+    if (tid == 0) {
+      double pq[9], ipq[9], al[9], zr[9];
+      for (int k = 0; k < 9; ++k) {
+        pq[k] = tot[k];
+        zr[k] = s_zr[k];
+        al[k] = 0.0;
+      }
+      if (inv3(pq, ipq)) mul3(ipq, zr, al);
+      for (int k = 0; k < 9; ++k) s_m[k] = al[k];
+    } else if (tid == 32) {
+      double pq[9];
+      for (int k = 0; k < 9; ++k) pq[k] = tot[k];
+      s_flag = negative_curvature(pq) ? 1 : 0;
+    }
+    __syncthreads();
+    if (s_flag) {                                // A is not positive definite: ends this frequency's solve
+      if (rank == 0 && tid == 0) {
+        st[kCgIndefinite] = 1.0;
+        st[0] = 3.0;
+      }
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < kRed; ++k) vals[k] = 0.0;
+    for (int p = rank; p < pairs; p += C)
+      for (int e = 0; e < 2; ++e) {
+        const int I = e == 0 ? p : nt - 1 - p, gr = I * CT + r;
+        if (e == 1 && I == p) break;
+        const size_t o = vo + (size_t)gr * 3;
+        // M^-1 (symmetric: a thread's row is read down its column) is on its way while R is formed
+        const double* M = a.Minv + ((size_t)f * nt + I) * CT * CT;
+        const int row = tid & 63, kg = tid >> 6;
+        double m[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) m[k] = M[(16 * kg + k) * CT + row];
+        double rv = 0.0;
+        if (tid < CT * 3) {
+          if (gr < n) {
+            double x = a.X[o + q];
+            rv = a.R[o + q];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              x += a.P[o + c] * s_m[3 * c + q];
+              rv -= a.Q[o + c] * s_m[3 * c + q];
+            }
+            a.X[o + q] = x;
+            a.R[o + q] = rv;
+          }
+          Rs[r][q] = rv;
+        }
+        __syncthreads();
+        {   // Z = M^-1 R: four chains of 16 for each row
+          double z0 = 0.0, z1 = 0.0, z2 = 0.0;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            z0 += m[k] * Rs[16 * kg + k][0];
+            z1 += m[k] * Rs[16 * kg + k][1];
+            z2 += m[k] * Rs[16 * kg + k][2];
+          }
+          Zp[kg][row][0] = z0;
+          Zp[kg][row][1] = z1;
+          Zp[kg][row][2] = z2;
+        }
+        __syncthreads();
+        if (tid < CT * 3) {
+          double z[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) z[c] = (Zp[0][r][c] + Zp[1][r][c]) + (Zp[2][r][c] + Zp[3][r][c]);
+          if (gr < n) a.Z[o + q] = q == 0 ? z[0] : (q == 1 ? z[1] : z[2]);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double t = z[c] * rv;
+            if (q == 0) vals[3 * c] += t;
+            if (q == 1) vals[3 * c + 1] += t;
+            if (q == 2) vals[3 * c + 2] += t;
+          }
+          vals[9] += rv * rv;
+        }
+      }
+    __syncthreads();
+    cta_record(vals, sm, rec2 + rank * kRed);
+    cl.sync();
+    // beta = (Z^T R)_old^-1 (Z^T R)_new; convergence test
+    sum_cluster_records(rec2, C, tot);
+    if (tid == 0) {
+      double zo[9], izo[9], zn[9], be[9];
+      for (int k = 0; k < 9; ++k) {
+        zo[k] = s_zr[k];
+        zn[k] = tot[k];
+      }
+      int done = 0;
+      if (tot[9] <= a.tol2) {
+        done = 1;
+      } else if (!inv3(zo, izo)) {
+        done = 2;
+      } else {
+        mul3(izo, zn, be);
+        for (int k = 0; k < 9; ++k) s_m[k] = be[k];
+      }
+      for (int k = 0; k < 9; ++k) s_zr[k] = zn[k];
+      s_flag = done;
+      if (rank == 0) {
+        st[kRR] = tot[9];
+        st[1] = (double)(it + 1);
+        if (done) st[0] = (double)done;
+      }
+    }
+    __syncthreads();
+    if (s_flag) return;
+    for (int p = rank; p < pairs; p += C)
+      for (int e = 0; e < 2; ++e) {
+        const int I = e == 0 ? p : nt - 1 - p, gr = I * CT + r;
+        if (e == 1 && I == p) break;
+        const size_t o = vo + (size_t)gr * 3;
+        const bool live = tid < CT * 3 && gr < n;
+        double v = 0.0;
+        if (live) {
+          v = a.Z[o + q];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) v += a.P[o + c] * s_m[3 * c + q];
+        }
+        __syncthreads();                         // a row's three entries are read by three threads
+        if (live) {
+          a.P[o + q] = v;
+          const float vf = (float)v;             // the entry in every CTA's copies
+          for (int k = 0; k < C; ++k) {
+            float4* other = cl.map_shared_rank(xs, k);
+            reinterpret_cast<float*>(other + gr)[q] = vf;
+            reinterpret_cast<float*>(other + prow)[q * prow + gr] = vf;
+          }
+        }
+      }
+    cl.sync();
+  }
+  if (rank == 0 && tid < 9) st[kZR0 + tid] = s_zr[tid];   // for a launch that carries on
+}
+
 }  // namespace
 
 size_t cg_minv_doubles(int n, int batch) {
   const int nt = (n + CT - 1) / CT;
   return (size_t)batch * nt * CT * CT;
+}
+
+int num_sms() {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 148;
+  }
+  return sms;
 }
 
 // CTAs of the grid-stride tile launch: every resident slot of the device.
@@ -576,6 +1029,33 @@ size_t cg_red_doubles(int n, int batch) {
   const int nt = (n + CT - 1) / CT;
   const int nb = (n / 3 + AT - 1) / AT;
   return (size_t)batch * (nt > nb ? nt : nb) * kRed;
+}
+
+cudaError_t init_cg_attributes() {
+  return cudaFuncSetAttribute(cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)p_shared_bytes((kCgClusterMaxN + CT - 1) / CT));
+}
+
+cudaError_t launch_cg_cluster(const CgArgs& a, int it0, int it1, int share, cudaStream_t s) {
+  // A pair of blocks for every CTA, up to the portable cluster size; where
+  // `share` geometries run side by side, no more CTAs than the device holds of
+  // all of them (a CTA's share of an iteration is then larger than what the
+  // iteration's barriers and 3 x 3 steps cost).
+  const int room = std::max(2, 2 * num_sms() / (a.batch * std::max(1, share)));
+  const int C = std::max(1, std::min({8, room, (a.nt + 1) / 2}));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(a.batch * C);
+  cfg.blockDim = dim3(CLT);
+  cfg.dynamicSmemBytes = p_shared_bytes(a.nt);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, cg_cluster_kernel, a, it0, it1);
 }
 
 void launch_cg_setup(const CgArgs& a, cudaStream_t s) {

@@ -315,6 +315,16 @@ void launch_cg_setup(const CgArgs& a, cudaStream_t s);
 // skips it.  fp32: the matrix pass reads A32 instead of A (FP64 vectors and
 // sums either way).
 void launch_cg_iteration(const CgArgs& a, int it, cudaStream_t s, bool fp32 = false);
+// Iterations [it0, it1) of an FP32-pass phase in one launch, for n <= kCgClusterMaxN
+// (state as launch_cg_iteration leaves it, but for the Z^T R slots).  Relay
+// solve of one cluster, four launches an iteration against this (ms): N = 61
+// 0.54 / 0.41, 200 0.84 / 0.68, 500 2.02 / 1.83, 680 2.76 / 2.26; beyond, a
+// cluster per frequency leaves too much of the device idle once most
+// frequencies have converged.
+constexpr int kCgClusterMaxN = 2048;
+cudaError_t init_cg_attributes();
+// share: geometries whose solves run side by side.
+cudaError_t launch_cg_cluster(const CgArgs& a, int it0, int it1, int share, cudaStream_t s);
 // Restart between the two phases of the mixed-precision solve: the true
 // residual R = B - A X from the FP64 matrix, Z = M^-1 R, P = Z, Z^T R; the
 // frequencies the first phase stopped (converged or broke down) run again,

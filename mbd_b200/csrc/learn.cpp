@@ -32,6 +32,7 @@ constexpr double kCgTol = 3e-11;   // relative residual the iteration stops at (
 // from a residual ~1e-5 of B, and the FP32 rounding of the matrix (~6e-8
 // relative) then leaves ~1e-12 in the final residual, far below the gate.
 constexpr int kCgPhaseMaxIters = 40;
+constexpr int kCgNarrowIters = 16;
 constexpr double kCgTol1 = 1e-5;
 
 // Image range and bounding box of the network's neighbour lists (within the
@@ -310,13 +311,28 @@ int relay_learned(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cuda
     const double tol2 = a.tol2;
     a.tol2 = kCgTol1 * kCgTol1 * 3.0 * N;
     launch_cg_setup(a, s);
-    const int it1 = sched(gd->cg_iters_seen1, kCgPhaseMaxIters);
-    for (int it = 0; it < it1; ++it) launch_cg_iteration(a, it, s, true);
+    // a phase's iterations: a cluster per frequency for small systems (in a
+    // batch narrow clusters first; the few frequencies that need more than
+    // kCgNarrowIters then get clusters of the full width), four launches each
+    // for large ones, whose matrix passes take the whole device
+    auto phase = [&](int seen) {
+      const int its = sched(seen, kCgPhaseMaxIters);
+      if (n <= kCgClusterMaxN) {
+        const int first = std::min(its, kCgNarrowIters);
+        cudaError_t e = launch_cg_cluster(a, 0, first, ctx->n_slots, s);
+        if (e == cudaSuccess && its > first) e = launch_cg_cluster(a, first, its, 1, s);
+        ctx->launches += its > first ? 2 : 1;
+        return e;
+      }
+      for (int it = 0; it < its; ++it) launch_cg_iteration(a, it, s, true);
+      ctx->launches += 4 * its;
+      return cudaSuccess;
+    };
+    MBD_CUDA(phase(gd->cg_iters_seen1));
     a.tol2 = tol2;
     launch_cg_restart(a, s);
-    const int it2 = sched(gd->cg_iters_seen, kCgPhaseMaxIters);
-    for (int it = 0; it < it2; ++it) launch_cg_iteration(a, it, s, true);
-    ctx->launches += 5 + 5 + 4 * (it1 + it2);
+    MBD_CUDA(phase(gd->cg_iters_seen));
+    ctx->launches += 5 + 5;
   } else {
     launch_cg_setup(a, s);
     const int iters = sched(gd->cg_iters_seen, kCgMaxIters);
