@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "chol64.cuh"
 #include "kernels.h"
 
 namespace mbd {
@@ -133,67 +134,48 @@ __device__ void cta_record(const double* vals, double* sm /* [kRed][32] */, doub
 __device__ __forceinline__ bool stopped(const CgArgs& a, int f) { return a.state[f * kCgState] != 0.0; }
 
 // Minv[f][I] = inverse of the diagonal tile A_II (rows beyond n: the
-// identity): Cholesky L L^T = A_II in place, W = L^-1 column by column (W's
-// column c kept as row c of the upper triangle, its diagonal in wd), then
-// Minv = W^T W.  A tile that is not positive definite gets the identity (the
-// iteration then cannot converge and the residual gate sends the geometry to
-// the direct solve).
-__global__ void __launch_bounds__(256) cg_tile_inv_kernel(CgArgs a) {
-  __shared__ double T[CT][CT + 1];
-  __shared__ double wd[CT];
+// identity) = W^T W with W = L^-1 of its Cholesky factor (chol64.cuh), the
+// product on the FP64 tensor cores.  A tile that is not positive definite
+// gets the identity (the iteration then cannot converge and the residual gate
+// sends the geometry to the direct solve).  Bound by the factor's chain of 64
+// pivots; a column-at-a-time factor with dot products by single threads took
+// 153 us a launch (300-atom clusters) against 28.
+constexpr size_t kTileInvSmem = sizeof(double) * 2 * NB * FS;
+__global__ void __launch_bounds__(kDiagThreads) cg_tile_inv_kernel(CgArgs a) {
+  extern __shared__ __align__(16) double dsm[];
+  __shared__ double s_dinv[NB], s_diagx[NB];
   __shared__ int s_bad;
+  double* S = dsm;
+  double* X = dsm + NB * FS;
   const int I = blockIdx.x, f = blockIdx.y, tid = threadIdx.x;
   const double* A = a.A + (size_t)f * a.a_stride;
-  for (int e = tid; e < CT * CT; e += blockDim.x) {
-    const int r = e / CT, c = e % CT;
-    const int gr = I * CT + r, gc = I * CT + c;
-    double v = (r == c) ? 1.0 : 0.0;
-    if (gr < a.n && gc < a.n) v = (c <= r) ? A[(size_t)gr * a.ld + gc] : A[(size_t)gc * a.ld + gr];
-    T[r][c] = v;
+  for (int e = tid; e < NB * NB; e += kDiagThreads) {
+    const int r = e / NB, c = e % NB, gr = I * NB + r, gc = I * NB + c;
+    S[r * FS + c] = (c <= r && gr < a.n) ? A[(size_t)gr * a.ld + gc] : (r == c ? 1.0 : 0.0);
   }
   if (tid == 0) s_bad = 0;
   __syncthreads();
-  for (int k = 0; k < CT; ++k) {
-    if (tid == 0) {
-      const double d = T[k][k];
-      if (!(d > 0.0) || !isfinite(d)) s_bad = 1;
-      T[k][k] = sqrt(fmax(d, 1e-300));
-    }
-    __syncthreads();
-    const double lkk = T[k][k];
-    for (int i = k + 1 + tid; i < CT; i += blockDim.x) T[i][k] /= lkk;
-    __syncthreads();
-    const int w = CT - k - 1;
-    for (int e = tid; e < w * w; e += blockDim.x) {
-      const int i = k + 1 + e / w, j = k + 1 + e % w;
-      if (j <= i) T[i][j] -= T[i][k] * T[j][k];
-    }
-    __syncthreads();
+  diag_factor(S, X, s_dinv, s_diagx, tid, 0, NB, &s_bad, 0.0);
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  double o[8][2];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) o[j][0] = o[j][1] = 0.0;
+  for (int kk = 8 * warp; kk < NB; kk += 4) {   // W is lower triangular: k >= max(row, column)
+    const double af = X[(kk + q) * FS + 8 * warp + g];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (8 * j <= kk + 3) dmma(o[j][0], o[j][1], af, X[(kk + q) * FS + 8 * j + g]);
   }
-  if (tid < CT) {
-    // W(i, c) = (delta_ic - sum_{c <= k < i} L(i, k) W(k, c)) / L(i, i); W(k, c) at T[c][k] (k > c)
-    const int c = tid;
-    const double wcc = 1.0 / T[c][c];
-    wd[c] = wcc;
-    for (int i = c + 1; i < CT; ++i) {
-      double sum = T[i][c] * wcc;
-      for (int k = c + 1; k < i; ++k) sum += T[i][k] * T[c][k];
-      T[c][i] = -sum / T[i][i];
-    }
-  }
-  __syncthreads();
-  double* M = a.Minv + ((size_t)f * a.nt + I) * CT * CT;
-  for (int e = tid; e < CT * CT; e += blockDim.x) {
-    const int i = e / CT, j = e % CT;
-    double sum = 0.0;
+  double* M = a.Minv + ((size_t)f * a.nt + I) * NB * NB;
+  const int row = 8 * warp + g;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int c = 8 * j + 2 * q;
     if (s_bad) {
-      sum = (i == j) ? 1.0 : 0.0;
-    } else {
-      // (W^T W)(i, j) = sum_{k >= max(i, j)} W(k, i) W(k, j)
-      const int k0 = i > j ? i : j;
-      for (int k = k0; k < CT; ++k) sum += (k == i ? wd[i] : T[i][k]) * (k == j ? wd[j] : T[j][k]);
+      o[j][0] = row == c ? 1.0 : 0.0;
+      o[j][1] = row == c + 1 ? 1.0 : 0.0;
     }
-    M[e] = sum;
+    *reinterpret_cast<double2*>(M + row * NB + c) = make_double2(o[j][0], o[j][1]);
   }
 }
 
@@ -1032,6 +1014,9 @@ size_t cg_red_doubles(int n, int batch) {
 }
 
 cudaError_t init_cg_attributes() {
+  cudaError_t e = cudaFuncSetAttribute(cg_tile_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kTileInvSmem);
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)p_shared_bytes((kCgClusterMaxN + CT - 1) / CT));
 }
@@ -1062,7 +1047,7 @@ void launch_cg_setup(const CgArgs& a, cudaStream_t s) {
   const long long items = (long long)a.nt * (a.nt + 1) / 2 * a.batch;
   const int tgrid = (int)std::min<long long>(cg_tile_grid<double>(), items);
   cudaMemsetAsync(a.state, 0, sizeof(double) * kCgState * a.batch, s);
-  cg_tile_inv_kernel<<<dim3(a.nt, a.batch), 256, 0, s>>>(a);
+  cg_tile_inv_kernel<<<dim3(a.nt, a.batch), kDiagThreads, kTileInvSmem, s>>>(a);
   cg_tile_kernel<double><<<tgrid, TT, 0, s>>>(a, a.A, a.X);
   cg_rows_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1);
   cg_init_tiles_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a);
