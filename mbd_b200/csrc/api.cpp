@@ -233,6 +233,57 @@ TrdPlan plan_tridiag(const std::vector<int>& sizes, int ctas) {
 
 // ---- relay stages of one geometry (on its slot's stream) ------------------
 
+// Direct FP64 relay solve: the factors of the matrices in sl.relay64 into L
+// (which may be the matrices themselves), the solution into sl.rhs.
+int relay_direct(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, double* L, cudaEvent_t ev_factor, double** X_out) {
+  const GeomPlan& p = gd->plan;
+  cudaStream_t s = sl.stream;
+  const int n = p.n;
+  const size_t mstride = (size_t)n * p.ld, ystride = (size_t)n * 3;
+  const int nblk = (n + kCholNB - 1) / kCholNB;
+  const size_t lstride = (size_t)nblk * kCholNB * kCholNB;
+  BatchMat bm{L, mstride, p.ld, n, kNFreq};
+  double* Linv = sl.linv.as<double>();
+  CholFlowArgs cf{};
+  cf.src = sl.relay64.as<double>();
+  cf.L = L;
+  cf.src_stride = cf.l_stride = mstride;
+  cf.src_ld = cf.ld = p.ld;
+  cf.n = n;
+  cf.batch = kNFreq;
+  cf.linv = Linv;
+  cf.linv_stride = lstride;
+  cf.info = gd->info;
+  cf.sync = sl.chol_sync.as<int>();
+  cf.err = ctx->err_flag;
+  MBD_CUDA(launch_chol_flow(cf, ctx->num_sms, s));
+  ctx->launches += 1;
+  record_timing(ctx, ev_factor, s);
+  double* Wv = sl.rhs.as<double>();
+  double* Zv = Wv + kNFreq * ystride;
+  double* Xv = Zv + kNFreq * ystride;
+  launch_init_rhs(Wv, ystride, n, kNFreq, s);
+  for (int k0 = 0; k0 < n; k0 += kCholNB) launch_trsv_fwd_step(bm, k0, Linv, lstride, Wv, Zv, ystride, s);
+  for (int k0 = (nblk - 1) * kCholNB; k0 >= 0; k0 -= kCholNB)
+    launch_trsv_bwd_step(bm, k0, Linv, lstride, Zv, Xv, ystride, s);
+  ctx->launches += 1 + 2 * nblk;
+  *X_out = Xv;
+  return MBD_OK;
+}
+
+// Mixed relay solve of a matrix small enough for the direct FP64 solve to be
+// the faster one (kMixedDirectMaxN): its factors beside the matrices, and the
+// residual the gate reads.
+int relay_mixed_direct(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, cudaEvent_t ev_factor, double** X_out) {
+  const GeomPlan& p = gd->plan;
+  int st = relay_direct(ctx, gd, sl, sl.relay32.as<double>(), ev_factor, X_out);
+  if (st != MBD_OK) return st;
+  launch_relay_residual(sl.relay64.as<double>(), (size_t)p.n * p.ld, p.ld, p.n, kNFreq, *X_out, nullptr,
+                        sl.rhs.as<double>(), (size_t)p.n * 3, sl.res_ws.as<double>(), gd->rnorm2, sl.stream);
+  ctx->launches += 3;
+  return MBD_OK;
+}
+
 // Mixed relay solve: FP32 copy factorised with 3xTF32 tcgen05 GEMMs (128-wide
 // panels), FP64 iterative refinement against the FP64 matrices.  Leaves the
 // refined solution X (n x 3 per frequency) at the start of slot.mixv.
@@ -392,6 +443,7 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   cudaEvent_t* ev = ctx->events.data() + (size_t)gi * kGeomEvents;
   auto mark = [&](int k) { record_timing(ctx, ev[k], s); };
   const bool mixed = mode == MBD_MODE_MIXED;
+  const bool direct = mixed && mixed_direct(*gd, sl);
   const bool learned = mode == MBD_MODE_MIXED_LEARNED;
   mark(0);
   // 1. per-atom frequency table
@@ -404,14 +456,17 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   const size_t mstride = (size_t)n * p.ld;
   RelayBuildArgs rb{N, p.ld, mstride, gd->coords, gd->alpha_w, gd->sgm, gd->rvdw_iso, gd->scs_shifts,
                     (int)p.scs_shifts.size() / 3, p.beta, p.scs_eval_cut, sl.relay64.as<double>(),
-                    (mixed || (learned && ctx->cg_fp32)) ? sl.relay32.as<float>() : nullptr};
+                    ((mixed && !direct) || (learned && ctx->cg_fp32)) ? sl.relay32.as<float>() : nullptr};
   rb.f32_math = (mixed || learned) && ctx->f32_tensor_build;
   launch_relay_build(rb, s);
   ctx->launches += 1;
   mark(2);
   const size_t ystride = (size_t)n * 3;
   double* Xv = nullptr;
-  if (mixed) {
+  if (direct) {
+    int st = relay_mixed_direct(ctx, gd, sl, ev[3], &Xv);
+    if (st != MBD_OK) return st;
+  } else if (mixed) {
     int st = relay_mixed(ctx, gd, sl, mstride, ev[3]);
     if (st != MBD_OK) return st;
     Xv = sl.mixv.as<double>();
@@ -420,34 +475,9 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
     int st = relay_learned(ctx, gd, sl, mstride, ev[3], &Xv);
     if (st != MBD_OK) return st;
   } else {
-    // 3. Cholesky of the 21 frequency matrices in one launch
-    BatchMat bm{sl.relay64.as<double>(), mstride, p.ld, n, kNFreq};
-    const int nblk = (n + kCholNB - 1) / kCholNB;
-    const size_t lstride = (size_t)nblk * kCholNB * kCholNB;
-    double* Linv = sl.linv.as<double>();
-    CholFlowArgs cf{};
-    cf.src = cf.L = bm.A;
-    cf.src_stride = cf.l_stride = mstride;
-    cf.src_ld = cf.ld = p.ld;
-    cf.n = n;
-    cf.batch = kNFreq;
-    cf.linv = Linv;
-    cf.linv_stride = lstride;
-    cf.info = gd->info;
-    cf.sync = sl.chol_sync.as<int>();
-    cf.err = ctx->err_flag;
-    MBD_CUDA(launch_chol_flow(cf, ctx->num_sms, s));
-    ctx->launches += 1;
-    mark(3);
-    // 4. solve X = A^-1 [I;..;I]
-    double* Wv = sl.rhs.as<double>();
-    double* Zv = Wv + kNFreq * ystride;
-    Xv = Zv + kNFreq * ystride;
-    launch_init_rhs(Wv, ystride, n, kNFreq, s);
-    for (int k0 = 0; k0 < n; k0 += kCholNB) launch_trsv_fwd_step(bm, k0, Linv, lstride, Wv, Zv, ystride, s);
-    for (int k0 = (nblk - 1) * kCholNB; k0 >= 0; k0 -= kCholNB)
-      launch_trsv_bwd_step(bm, k0, Linv, lstride, Zv, Xv, ystride, s);
-    ctx->launches += 1 + 2 * nblk;
+    // 3. Cholesky of the 21 frequency matrices in place, 4. X = A^-1 [I;..;I]
+    int st = relay_direct(ctx, gd, sl, sl.relay64.as<double>(), ev[3], &Xv);
+    if (st != MBD_OK) return st;
   }
   EpilogueArgs ea{N, Xv, ystride, gd->alpha_iw, gd->molpol, gd->alpha0, gd->c6free, gd->r0,
                   gd->c6_eff, gd->alpha_eff, gd->omega, gd->rvdw_eff, gd->scalars};
@@ -541,7 +571,14 @@ size_t trace_bytes(const GeomPlan& p, size_t* factors, size_t* linv, size_t* ws)
   return *factors + *linv + *ws;
 }
 
-size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, size_t* res, size_t* sync) {
+// direct: the FP64 factors in the place of the FP32 copy and its panels.
+size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, size_t* res, size_t* sync, bool direct) {
+  if (direct) {
+    *r32 = sizeof(double) * (size_t)kNFreq * p.n * p.ld;
+    *pan = *vec = *sync = 0;
+    *res = sizeof(double) * relay_residual_ws_doubles(p.n, kNFreq);
+    return *r32 + *res;
+  }
   *r32 = sizeof(float) * (size_t)kNFreq * p.n * p.ld;
   *pan = sizeof(float) * (size_t)kNFreq * round_up(p.n, kMixNB) * kMixNB;
   *vec = sizeof(double) * 4 * (size_t)kNFreq * p.n * 3;
@@ -580,7 +617,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
       slot_of[g] = s;
       load[s] += std::pow((double)p.n, 3.0);
       size_t a, b, c, d, e, f, h;
-      size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a);
+      size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a, p.n <= kMixedDirectMaxN);
       // the trace form's factors past what the relay's matrices leave
       if (ctx->geoms[g]->trace) {
         plain_bytes(p, &a, &b, &c, &h);
@@ -816,20 +853,11 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   return MBD_OK;
 }
 
-// Buffers only the mixed modes use (allocated on first use).
+// Buffers only the mixed mode uses (allocated on first use).  Where the FP64
+// factors of a slot's small geometries do not fit, they go the way of the
+// large ones.
 int reserve_mixed(mbd_ctx* ctx) {
   for (int s = 0; s < ctx->n_slots; ++s) {
-    size_t r32 = 0, pan = 0, vec = 0, res = 0, sync = 0;
-    for (int g : ctx->order) {
-      if (ctx->geoms[g]->slot != s) continue;
-      size_t a, b, c, d, e;
-      mixed_bytes(ctx->geoms[g]->plan, &a, &b, &c, &d, &e);
-      r32 = std::max(r32, a);
-      pan = std::max(pan, b);
-      vec = std::max(vec, c);
-      res = std::max(res, d);
-      sync = std::max(sync, e);
-    }
     RelaySlot& sl = *ctx->slots[s];
     bool moved = false;
     auto grow = [&](DevBuf& b, size_t bytes) {
@@ -837,15 +865,36 @@ int reserve_mixed(mbd_ctx* ctx) {
       moved = moved || re;
       return b.reserve(bytes);
     };
-    MBD_CUDA(grow(sl.relay32, r32));
-    MBD_CUDA(grow(sl.p_hi, pan));
-    MBD_CUDA(grow(sl.p_lo, pan));
-    MBD_CUDA(grow(sl.l_hi, pan));
-    MBD_CUDA(grow(sl.l_lo, pan));
-    MBD_CUDA(grow(sl.mixv, vec));
-    MBD_CUDA(grow(sl.res_ws, res));
-    MBD_CUDA(grow(sl.solve_sync, sync));
+    auto reserve = [&]() -> cudaError_t {
+      size_t r32 = 0, pan = 0, vec = 0, res = 0, sync = 0;
+      for (int g : ctx->order) {
+        const GeomDev& gd = *ctx->geoms[g];
+        if (gd.slot != s) continue;
+        size_t a, b, c, d, e;
+        mixed_bytes(gd.plan, &a, &b, &c, &d, &e, mixed_direct(gd, sl));
+        r32 = std::max(r32, a);
+        pan = std::max(pan, b);
+        vec = std::max(vec, c);
+        res = std::max(res, d);
+        sync = std::max(sync, e);
+      }
+      cudaError_t e = grow(sl.relay32, r32);
+      for (DevBuf* b : {&sl.p_hi, &sl.p_lo, &sl.l_hi, &sl.l_lo})
+        if (e == cudaSuccess) e = grow(*b, pan);
+      if (e == cudaSuccess) e = grow(sl.mixv, vec);
+      if (e == cudaSuccess) e = grow(sl.res_ws, res);
+      if (e == cudaSuccess) e = grow(sl.solve_sync, sync);
+      return e;
+    };
+    sl.mixed_direct = true;
+    cudaError_t e = reserve();
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      sl.mixed_direct = false;
+      e = reserve();
+    }
     if (moved) drop_graphs(ctx, true);
+    MBD_CUDA(e);
   }
   return MBD_OK;
 }
@@ -868,7 +917,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
   for (int k = 0; k < ctx->n_slots; ++k) {
     RelaySlot& sl = *ctx->slots[k];
     MBD_CUDA(cudaStreamWaitEvent(sl.stream, ctx->fork_ev, 0));
-    if (mode == MBD_MODE_MIXED) {
+    if (mode == MBD_MODE_MIXED && sl.solve_sync.p) {
       MBD_CUDA(cudaMemsetAsync(sl.solve_sync.p, 0, sl.solve_sync.bytes, sl.stream));
       sl.solve_epoch = 0;
     }
@@ -1279,7 +1328,7 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
       double worst = 0.0;
       for (int f = 0; f < 21; ++f) worst = std::max(worst, std::sqrt(rn[f] / (3.0 * N)));
       r.err_est[0] = r.err_est[1] = r.err_est[2] = worst;
-      r.refine_iters = kRefineIters;
+      r.refine_iters = mixed_direct(*gd, *ctx->slots[gd->slot]) ? 1 : kRefineIters;
       if (ctx->last_mode == MBD_MODE_MIXED_LEARNED) {
         const double* cs = reinterpret_cast<const double*>(host(g, gd->cgstate));
         double most = 0.0, most1 = 0.0;

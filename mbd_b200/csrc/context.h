@@ -119,6 +119,7 @@ struct RelaySlot {
   DevBuf trd_ws;                                              // dense -> band workspace
   DevBuf trace_ws;                                            // trace form: bounds, nodes, counters
   int solve_epoch = 0;
+  bool mixed_direct = true;   // room for the FP64 factors of the mixed mode's small geometries
   ~RelaySlot() {
     if (done) cudaEventDestroy(done);
     if (la.ready) cudaEventDestroy(la.ready);
@@ -331,6 +332,16 @@ int relay_learned(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cuda
 // Largest Hamiltonian the trace form takes: past it the reduction to a band,
 // (4/3) n^3 operations against ~4 n^3, is the faster one.
 constexpr int kTraceMaxN = 9216;
+
+// Relay matrices the mixed mode solves by the FP64 factors instead of 3xTF32
+// factors and refinement.  Factor + solve (ms, direct / 3xTF32): N = 61 0.14 /
+// 0.76, 533 2.3 / 6.9, 1000 8.8 / 15.4, 2000 54 / 49: the refinement's
+// triangular sweeps and the FP32 panels' chain cost more than the tensor cores
+// save below ~1700 atoms.
+constexpr int kMixedDirectMaxN = 5000;
+inline bool mixed_direct(const GeomDev& gd, const RelaySlot& sl) {
+  return sl.mixed_direct && gd.plan.n <= kMixedDirectMaxN;
+}
 
 // Matrices reduced by the two-stage path (the rest by the one-stage kernel).
 inline bool two_stage(const mbd_ctx* ctx, int n) {
