@@ -262,12 +262,17 @@ int relay_direct(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, double* L, cudaEvent_
   double* Wv = sl.rhs.as<double>();
   double* Zv = Wv + kNFreq * ystride;
   double* Xv = Zv + kNFreq * ystride;
+  *X_out = Xv;
+  if (n <= kTrsvMaxN) {
+    MBD_CUDA(launch_trsv_cluster(bm, Linv, lstride, Xv, ystride, s));
+    ctx->launches += 1;
+    return MBD_OK;
+  }
   launch_init_rhs(Wv, ystride, n, kNFreq, s);
   for (int k0 = 0; k0 < n; k0 += kCholNB) launch_trsv_fwd_step(bm, k0, Linv, lstride, Wv, Zv, ystride, s);
   for (int k0 = (nblk - 1) * kCholNB; k0 >= 0; k0 -= kCholNB)
     launch_trsv_bwd_step(bm, k0, Linv, lstride, Zv, Xv, ystride, s);
   ctx->launches += 1 + 2 * nblk;
-  *X_out = Xv;
   return MBD_OK;
 }
 
@@ -1090,6 +1095,7 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
   }
   MBD_CUDA(init_device_constants());
   MBD_CUDA(init_cholflow_attributes());
+  MBD_CUDA(init_trsv_attributes());
   MBD_CUDA(init_cg_attributes());
   MBD_CUDA(init_eigval_attributes());
   MBD_CUDA(init_tc3_attributes());

@@ -98,6 +98,12 @@ constexpr int kCholFlowHead = 32;
 size_t chol_flow_sync_ints(int n, int batch);
 cudaError_t init_cholflow_attributes();
 cudaError_t launch_chol_flow(const CholFlowArgs& a, int num_sms, cudaStream_t s);
+// X = (L L^T)^-1 [I;I;..;I] in one launch, for n <= kTrsvMaxN (the solution is
+// held in shared memory); larger matrices take the steps below, a launch each.
+constexpr int kTrsvMaxN = 8064;
+cudaError_t init_trsv_attributes();
+cudaError_t launch_trsv_cluster(const BatchMat& m, const double* Linv, size_t linv_stride, double* X, size_t ystride,
+                                cudaStream_t s);
 // Y (n x 3 per matrix, row-major, stride ystride) := stacked identities [I;I;..;I].
 void launch_init_rhs(double* Y, size_t ystride, int n, int batch, cudaStream_t s);
 // Forward step: reads W at block k0, writes Z at block k0, updates W below it.
