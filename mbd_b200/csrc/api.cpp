@@ -19,6 +19,7 @@
 #include <limits>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -32,7 +33,10 @@ namespace mbd {
 namespace {
 
 // Symmetric 3x3 eigenvalues from the upper triangle (DSYEV('V','U'), UTILS.f90:273),
-// cyclic Jacobi in FP64, ascending.
+// cyclic Jacobi in FP64, ascending.  From the fifth sweep on, an off-diagonal
+// entry that adds nothing to either diagonal one at a hundredfold counts as
+// zero (Rutishauser's criterion): waiting for exact zeros took up to 50
+// sweeps, 106 us for a geometry's 21 tensors (27 ms for a batch of 256).
 void sym3_eigenvalues_upper(const double* M, double out[3]) {
   double a[3][3];
   for (int r = 0; r < 3; ++r)
@@ -43,6 +47,12 @@ void sym3_eigenvalues_upper(const double* M, double out[3]) {
     for (int p = 0; p < 2; ++p)
       for (int q = p + 1; q < 3; ++q) {
         if (a[p][q] == 0.0) continue;
+        const double g = 100.0 * std::fabs(a[p][q]);
+        if (sweep >= 4 && std::fabs(a[p][p]) + g == std::fabs(a[p][p]) &&
+            std::fabs(a[q][q]) + g == std::fabs(a[q][q])) {
+          a[p][q] = a[q][p] = 0.0;
+          continue;
+        }
         double theta = (a[q][q] - a[p][p]) / (2.0 * a[p][q]);
         double t = (theta >= 0 ? 1.0 : -1.0) / (std::fabs(theta) + std::sqrt(theta * theta + 1.0));
         double c = 1.0 / std::sqrt(t * t + 1.0), s = t * c;
@@ -64,101 +74,94 @@ void sym3_eigenvalues_upper(const double* M, double out[3]) {
   std::sort(out, out + 3);
 }
 
-int upload_geometry(mbd_ctx* ctx, const mbd_geom& g, GeomDev* gd) {
-  int st = build_plan(g, &gd->plan);
-  if (st != MBD_OK) return st;
+// Sections of a buffer, each 256-byte aligned.
+struct Sections {
+  size_t size = 0;
+  size_t add(size_t bytes) {
+    const size_t at = size;
+    size += (bytes + 255) & ~size_t(255);
+    return at;
+  }
+};
+
+// One geometry's device arrays: its inputs, the results the host reads back
+// and the rest, as sections of the batch's three regions.  fill(dst, src,
+// bytes) copies an input into the staging memory.
+template <class Place, class Fill>
+void lay_out(GeomDev* gd, Sections& in, Sections& out, Sections& work, Place place, Fill fill) {
   const GeomPlan& p = gd->plan;
-  const int N = p.N;
-  const int nshift_s = (int)p.scs_shifts.size() / 3, nshift_c = (int)p.cfdm_shifts.size() / 3;
-  const int ndiff = (int)p.diff_is_zero.size();
-  const int nplace = (int)p.place_rc.size();
-  // inputs
-  size_t off = 0;
-  std::vector<size_t> offs;
-  auto add = [&](size_t b) { offs.push_back(off); off += b; };
-  add(bytes_of<double>(3 * N));             // coords
-  add(bytes_of<double>(N));                 // alpha0
-  add(bytes_of<double>(N));                 // c6free
-  add(bytes_of<double>(N));                 // r0
-  add(bytes_of<double>(N));                 // hirsh
-  add(bytes_of<double>(3 * nshift_s));
-  add(bytes_of<double>(3 * nshift_c));
-  add(bytes_of<double>(3 * ndiff));
-  add(bytes_of<int>(ndiff));
-  add(bytes_of<int>(ndiff + 1));
-  add(bytes_of<int>(nplace));
-  add(bytes_of<int>(nplace));
-  MBD_CUDA(gd->inputs.reserve(off));
-  char* base = gd->inputs.as<char>();
-  std::vector<char> host(off, 0);
-  auto put = [&](int idx, const void* src, size_t b) { std::memcpy(host.data() + offs[idx], src, b); };
-  put(0, p.coords.data(), sizeof(double) * 3 * N);
-  put(1, p.alpha0.data(), sizeof(double) * N);
-  put(2, p.c6free.data(), sizeof(double) * N);
-  put(3, p.r0.data(), sizeof(double) * N);
-  put(4, p.hirsh.data(), sizeof(double) * N);
-  put(5, p.scs_shifts.data(), sizeof(double) * 3 * nshift_s);
-  put(6, p.cfdm_shifts.data(), sizeof(double) * 3 * nshift_c);
-  put(7, p.diff_shift.data(), sizeof(double) * 3 * ndiff);
-  put(8, p.diff_is_zero.data(), sizeof(int) * ndiff);
-  put(9, p.place_offset.data(), sizeof(int) * (ndiff + 1));
-  put(10, p.place_rc.data(), sizeof(int) * nplace);
-  put(11, p.place_cc.data(), sizeof(int) * nplace);
-  MBD_CUDA(cudaMemcpyAsync(base, host.data(), off, cudaMemcpyHostToDevice, ctx->stream));
-  ctx->h2d_bytes += (double)off;
-  gd->coords = reinterpret_cast<const double*>(base + offs[0]);
-  gd->alpha0 = reinterpret_cast<const double*>(base + offs[1]);
-  gd->c6free = reinterpret_cast<const double*>(base + offs[2]);
-  gd->r0 = reinterpret_cast<const double*>(base + offs[3]);
-  gd->hirsh = reinterpret_cast<const double*>(base + offs[4]);
-  gd->scs_shifts = reinterpret_cast<const double*>(base + offs[5]);
-  gd->cfdm_shifts = reinterpret_cast<const double*>(base + offs[6]);
-  gd->diff_shift = reinterpret_cast<const double*>(base + offs[7]);
-  gd->diff_is_zero = reinterpret_cast<const int*>(base + offs[8]);
-  gd->place_offset = reinterpret_cast<const int*>(base + offs[9]);
-  gd->place_rc = reinterpret_cast<const int*>(base + offs[10]);
-  gd->place_cc = reinterpret_cast<const int*>(base + offs[11]);
-  // results
-  off = 0;
-  offs.clear();
-  add(bytes_of<double>(21 * N));   // 0 alpha_w
-  add(bytes_of<double>(21 * N));   // 1 sgm
-  add(bytes_of<double>(N));        // 2 rvdw_iso
-  add(bytes_of<double>(21 * N));   // 3 alpha_iw
-  add(bytes_of<double>(21 * 9));   // 4 molpol
-  add(bytes_of<double>(N));        // 5 c6_eff
-  add(bytes_of<double>(N));        // 6 alpha_eff
-  add(bytes_of<double>(N));        // 7 omega
-  add(bytes_of<double>(N));        // 8 rvdw_eff
-  add(bytes_of<double>(8));        // 9 scalars
-  add(bytes_of<double>(8));        // 10 energy
-  add(bytes_of<double>(p.nH));     // 11 d
-  add(bytes_of<double>(p.nH));     // 12 e
-  add(bytes_of<double>(2 * (size_t)p.nH));   // 13 ev (+ e^2 scratch of the bisection)
-  add(bytes_of<int>(32));          // 14 info
-  add(bytes_of<double>(32));       // 15 rnorm2 (squared refinement residual per frequency)
-  add(bytes_of<double>(kNFreq * kCgState));   // 16 block-CG state
-  MBD_CUDA(gd->results.reserve(off));
-  base = gd->results.as<char>();
-  MBD_CUDA(cudaMemsetAsync(base, 0, off, ctx->stream));
-  gd->alpha_w = reinterpret_cast<double*>(base + offs[0]);
-  gd->sgm = reinterpret_cast<double*>(base + offs[1]);
-  gd->rvdw_iso = reinterpret_cast<double*>(base + offs[2]);
-  gd->alpha_iw = reinterpret_cast<double*>(base + offs[3]);
-  gd->molpol = reinterpret_cast<double*>(base + offs[4]);
-  gd->c6_eff = reinterpret_cast<double*>(base + offs[5]);
-  gd->alpha_eff = reinterpret_cast<double*>(base + offs[6]);
-  gd->omega = reinterpret_cast<double*>(base + offs[7]);
-  gd->rvdw_eff = reinterpret_cast<double*>(base + offs[8]);
-  gd->scalars = reinterpret_cast<double*>(base + offs[9]);
-  gd->energy = reinterpret_cast<double*>(base + offs[10]);
-  gd->d = reinterpret_cast<double*>(base + offs[11]);
-  gd->e = reinterpret_cast<double*>(base + offs[12]);
-  gd->ev = reinterpret_cast<double*>(base + offs[13]);
-  gd->info = reinterpret_cast<int*>(base + offs[14]);
-  gd->rnorm2 = reinterpret_cast<double*>(base + offs[15]);
-  gd->cgstate = reinterpret_cast<double*>(base + offs[16]);
+  const size_t N = p.N;
+  auto input = [&](auto*& dev, const auto& v) {
+    const size_t bytes = sizeof(v[0]) * v.size(), at = in.add(bytes);
+    place(0, at, dev);
+    fill(at, v.data(), bytes);
+  };
+  input(gd->coords, p.coords);
+  input(gd->alpha0, p.alpha0);
+  input(gd->c6free, p.c6free);
+  input(gd->r0, p.r0);
+  input(gd->hirsh, p.hirsh);
+  input(gd->scs_shifts, p.scs_shifts);
+  input(gd->cfdm_shifts, p.cfdm_shifts);
+  input(gd->diff_shift, p.diff_shift);
+  input(gd->diff_is_zero, p.diff_is_zero);
+  input(gd->place_offset, p.place_offset);
+  input(gd->place_rc, p.place_rc);
+  input(gd->place_cc, p.place_cc);
+  gd->out_at = out.size;
+  auto result = [&](auto*& dev, size_t n) { place(1, out.add(sizeof(*dev) * n), dev); };
+  result(gd->alpha_iw, 21 * N);
+  result(gd->molpol, 21 * 9);
+  result(gd->c6_eff, N);
+  result(gd->alpha_eff, N);
+  result(gd->scalars, 8);
+  result(gd->energy, 8);
+  result(gd->info, 32);
+  result(gd->rnorm2, 32);                         // squared relay residual per frequency
+  result(gd->cgstate, (size_t)kNFreq * kCgState);
+  gd->out_bytes = out.size - gd->out_at;
+  auto scratch = [&](double*& dev, size_t n) { place(2, work.add(sizeof(double) * n), dev); };
+  scratch(gd->alpha_w, 21 * N);
+  scratch(gd->sgm, 21 * N);
+  scratch(gd->rvdw_iso, N);
+  scratch(gd->omega, N);
+  scratch(gd->rvdw_eff, N);
+  scratch(gd->d, p.nH);
+  scratch(gd->e, p.nH);
+  scratch(gd->ev, 2 * (size_t)p.nH);              // + e^2 scratch of the bisection
   gd->n_edges = -1;   // the learned-mode graph of the new geometry is built on first use
+}
+
+// Plans and uploads every geometry: one staging copy, one clearing.
+int upload_geometries(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms) {
+  Sections in, out, work;
+  auto nowhere = [](int, size_t, auto*&) {};
+  auto nothing = [](size_t, const void*, size_t) {};
+  for (int g = 0; g < n_geom; ++g) {
+    GeomDev* gd = ctx->geoms[g].get();
+    gd->status_host = build_plan(geoms[g], &gd->plan);
+    if (gd->status_host == MBD_OK) lay_out(gd, in, out, work, nowhere, nothing);
+  }
+  if (in.size == 0) return MBD_OK;
+  MBD_CUDA(ctx->inputs.reserve(in.size));
+  MBD_CUDA(ctx->results.reserve(out.size + work.size));
+  MBD_CUDA(ctx->in_staging.reserve(in.size));
+  char* const region[3] = {ctx->inputs.as<char>(), ctx->results.as<char>(), ctx->results.as<char>() + out.size};
+  char* const host = ctx->in_staging.as<char>();
+  auto place = [&](int r, size_t at, auto*& dev) {
+    dev = reinterpret_cast<std::remove_reference_t<decltype(dev)>>(region[r] + at);
+  };
+  auto fill = [&](size_t at, const void* src, size_t bytes) { std::memcpy(host + at, src, bytes); };
+  const size_t in_bytes = in.size;
+  ctx->out_bytes = out.size;
+  in = out = Sections{};
+  const size_t work_bytes = work.size;
+  work = Sections{};
+  for (int g = 0; g < n_geom; ++g)
+    if (ctx->geoms[g]->status_host == MBD_OK) lay_out(ctx->geoms[g].get(), in, out, work, place, fill);
+  MBD_CUDA(cudaMemcpyAsync(ctx->inputs.p, host, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+  MBD_CUDA(cudaMemsetAsync(ctx->results.p, 0, ctx->out_bytes + work_bytes, ctx->stream));
+  ctx->h2d_bytes += (double)in_bytes;
   return MBD_OK;
 }
 
@@ -380,6 +383,37 @@ int relay_mixed(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cudaEv
 
 }  // namespace
 
+// Stage timings of the last downloaded compute, from its events (some 3 us an
+// interval on the host, so not on every download): relay/CFDM stages summed
+// over geometries (they overlap on the slots' streams), the batch-wide stages
+// and the total from batch events.
+void resolve_timings(mbd_ctx* ctx) {
+  if (!ctx->timed.pending) return;
+  ctx->timed.pending = false;
+  for (int k = 0; k < Stage::kCount; ++k) ctx->last_ms[k] = 0.0;
+  auto elapsed = [](cudaEvent_t a, cudaEvent_t b) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, a, b) == cudaSuccess) return (double)ms;
+    cudaGetLastError();
+    return 0.0;
+  };
+  const cudaEvent_t* bev = ctx->bev[ctx->timed.set];
+  ctx->last_ms[Stage::kTotal] = elapsed(bev[0], bev[3]);
+  ctx->last_ms[Stage::kTridiag] = elapsed(bev[1], bev[2]);
+  ctx->last_band_ms = ctx->last_trace_ms = 0.0;
+  ctx->last_chase_ms = ctx->last_ms[Stage::kTridiag];
+  ctx->last_onestage_ms = elapsed(bev[1], bev[4]);
+  ctx->last_sb2st_ms = elapsed(bev[4], bev[2]);
+  ctx->last_ms[Stage::kEig] = elapsed(bev[2], bev[3]);
+  for (const auto& [g, trace] : ctx->timed.geoms) {
+    const cudaEvent_t* evs = ctx->events[ctx->timed.set].data() + (size_t)g * kGeomEvents;
+    for (int k = 1; k + 1 < kGeomEvents; ++k) ctx->last_ms[k] += elapsed(evs[k - 1], evs[k]);
+    const double last = elapsed(evs[kGeomEvents - 2], evs[kGeomEvents - 1]);
+    ctx->last_ms[trace ? Stage::kEig : Stage::kTridiag] += last;
+    (trace ? ctx->last_trace_ms : ctx->last_band_ms) += last;
+  }
+}
+
 void drop_graphs(mbd_ctx* ctx, bool keep_first) {
   for (int m = 0; m < 3; ++m) {
     cudaGraphExec_t& g = ctx->graph[m];
@@ -445,7 +479,7 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   RelaySlot& sl = *ctx->slots[gd->slot];
   cudaStream_t s = sl.stream;
   const int N = p.N, n = p.n;
-  cudaEvent_t* ev = ctx->events.data() + (size_t)gi * kGeomEvents;
+  cudaEvent_t* ev = ctx->events[ctx->event_set].data() + (size_t)gi * kGeomEvents;
   auto mark = [&](int k) { record_timing(ctx, ev[k], s); };
   const bool mixed = mode == MBD_MODE_MIXED;
   const bool direct = mixed && mixed_direct(*gd, sl);
@@ -499,19 +533,19 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   CfdmBuildArgs cb{N, p.nsl, p.ldH, gd->coords, gd->omega, gd->alpha_eff, gd->rvdw_eff, gd->cfdm_shifts,
                    (int)p.cfdm_shifts.size() / 3, gd->diff_shift, gd->diff_is_zero, gd->place_offset,
                    gd->place_rc, gd->place_cc, (int)p.diff_is_zero.size(), p.beta, p.cfdm_cut,
-                   gd->hmat.as<double>()};
+                   gd->hmat};
   launch_cfdm_build(cb, s);
   ctx->launches += 1;
   mark(5);
   // 6. the energy from shifted Cholesky factors, or dense -> band (stage 1 of
   // the two-stage tridiagonalisation)
   if (gd->trace) {
-    TraceArgs ta{gd->hmat.as<double>(), p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
+    TraceArgs ta{gd->hmat, p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
                  sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag};
     MBD_CUDA(launch_trace_energy(ta, ctx->num_sms, s));
     ctx->launches += kTraceLaunches;
   } else if (two_stage(ctx, p.nH)) {
-    MBD_CUDA(launch_sy2sb(gd->hmat.as<double>(), p.ldH, p.nH, sl.trd_ws.as<double>(), gd->band.as<double>(),
+    MBD_CUDA(launch_sy2sb(gd->hmat, p.ldH, p.nH, sl.trd_ws.as<double>(), gd->band.as<double>(),
                           ctx->num_sms, s, tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),
                           lookahead_for(ctx, sl.la)));
     ctx->launches += sy2sb_launches(p.nH);
@@ -533,7 +567,7 @@ int run_tail_single(mbd_ctx* ctx, GeomDev* gd, cudaStream_t s) {
       MBD_CUDA(ctx->fb_band.reserve(sizeof(double) * (size_t)p.nH * kBandLd));
       MBD_CUDA(ctx->fb_trd.reserve(sizeof(double) * sy2sb_workspace_doubles(p.nH)));
       band = ctx->fb_band.as<double>();
-      MBD_CUDA(launch_sy2sb(gd->hmat.as<double>(), p.ldH, p.nH, ctx->fb_trd.as<double>(), band, ctx->num_sms, s,
+      MBD_CUDA(launch_sy2sb(gd->hmat, p.ldH, p.nH, ctx->fb_trd.as<double>(), band, ctx->num_sms, s,
                             tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),
                             lookahead_for(ctx, ctx->slots[gd->slot]->la)));
       ctx->launches += sy2sb_launches(p.nH);
@@ -541,7 +575,7 @@ int run_tail_single(mbd_ctx* ctx, GeomDev* gd, cudaStream_t s) {
     int st = band_to_tridiag_single(ctx, band, p.nH, gd->d, gd->e, ctx->fb_ws, s);
     if (st != MBD_OK) return st;
   } else {
-    TridiagJob job{gd->hmat.as<double>(), p.nH, p.ldH, gd->d, gd->e};
+    TridiagJob job{gd->hmat, p.nH, p.ldH, gd->d, gd->e};
     MBD_CUDA(cudaMemcpyAsync(ctx->job_dev, &job, sizeof(job), cudaMemcpyHostToDevice, s));
     const int G = tridiag_group_ctas(ctx, p.nH);
     const size_t wsb = tridiag_workspace_bytes(p.nH, G);
@@ -596,44 +630,68 @@ size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, siz
 // slot, load = (3N)^3), with as many slots as fit in the device memory share.
 int plan_slots(mbd_ctx* ctx, bool eigen) {
   const int ng = (int)ctx->order.size();
-  size_t free_b = 0, total_b = 0;
-  MBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  size_t held = 0;
-  for (auto& s : ctx->slots) held += s->held();
-  const double budget = kSlotMemoryShare * (double)(free_b + held);
+  int S = std::max(1, std::min(kMaxSlots, ng));
+  std::vector<int> slot_of(ctx->geoms.size(), 0);
+  auto deal = [&](int slots) {
+    std::vector<double> load(slots, 0.0);
+    for (int g : ctx->order) {
+      const int s = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      slot_of[g] = s;
+      load[s] += std::pow((double)ctx->geoms[g]->plan.n, 3.0);
+    }
+  };
   // Energies as traces: not while an eigenvalue kernel is asked for (its
-  // environment switches, the stalled chase of the failure tests), nor for
-  // Hamiltonians so large that the factors would not fit a share of the memory
+  // environment switches, the stalled chase of the failure tests)
   for (auto& gd : ctx->geoms) gd->trace = false;
   if (eigen && ctx->trace_form && !ctx->test_stall_wait)
+    for (int g : ctx->order) ctx->geoms[g]->trace = ctx->geoms[g]->plan.nH <= kTraceMaxN;
+  // A batch whose buffers are all there already (a program's second call of a
+  // size) does not ask how much memory is free: that query goes through the
+  // driver's kernel part, 0.05 to 2 ms depending on what else the host runs.
+  deal(S);
+  bool held = (int)ctx->slots.size() >= S;
+  for (int g : ctx->order) {
+    if (!held) break;
+    const GeomDev& gd = *ctx->geoms[g];
+    const RelaySlot& sl = *ctx->slots[slot_of[g]];
+    size_t a, b, c, d;
+    plain_bytes(gd.plan, &a, &b, &c, &d);
+    held = a <= sl.relay64.bytes && b <= sl.linv.bytes && c <= sl.rhs.bytes && d <= sl.chol_sync.bytes;
+    if (!held || !gd.trace) continue;
+    trace_bytes(gd.plan, &a, &b, &c);
+    held = a <= sl.relay64.bytes && b <= sl.linv.bytes && c <= sl.trace_ws.bytes;
+  }
+  if (!held) {
+    size_t free_b = 0, total_b = 0;
+    MBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    size_t own = 0;
+    for (auto& s : ctx->slots) own += s->held();
+    const double budget = kSlotMemoryShare * (double)(free_b + own);
+    // no trace form for Hamiltonians whose factors would not fit a share of the memory
     for (int g : ctx->order) {
       size_t a, b, c;
       GeomDev& gd = *ctx->geoms[g];
-      gd.trace = gd.plan.nH <= kTraceMaxN && (double)trace_bytes(gd.plan, &a, &b, &c) <= 0.5 * budget;
+      gd.trace = gd.trace && (double)trace_bytes(gd.plan, &a, &b, &c) <= 0.5 * budget;
     }
-  int S = std::max(1, std::min(kMaxSlots, ng));
-  std::vector<int> slot_of(ctx->geoms.size(), 0);
-  for (; S >= 1; --S) {
-    std::vector<double> load(S, 0.0);
-    std::vector<size_t> need(S, 0);
-    for (int g : ctx->order) {
-      const GeomPlan& p = ctx->geoms[g]->plan;
-      const int s = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-      slot_of[g] = s;
-      load[s] += std::pow((double)p.n, 3.0);
-      size_t a, b, c, d, e, f, h;
-      size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a, p.n <= kMixedDirectMaxN);
-      // the trace form's factors past what the relay's matrices leave
-      if (ctx->geoms[g]->trace) {
-        plain_bytes(p, &a, &b, &c, &h);
-        bytes += trace_bytes(p, &d, &e, &f);
-        bytes -= std::min(a, d) + std::min(b, e);
+    for (; S >= 1; --S) {
+      std::vector<size_t> need(S, 0);
+      deal(S);
+      for (int g : ctx->order) {
+        const GeomPlan& p = ctx->geoms[g]->plan;
+        size_t a, b, c, d, e, f, h;
+        size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a, p.n <= kMixedDirectMaxN);
+        // the trace form's factors past what the relay's matrices leave
+        if (ctx->geoms[g]->trace) {
+          plain_bytes(p, &a, &b, &c, &h);
+          bytes += trace_bytes(p, &d, &e, &f);
+          bytes -= std::min(a, d) + std::min(b, e);
+        }
+        need[slot_of[g]] = std::max(need[slot_of[g]], bytes);
       }
-      need[s] = std::max(need[s], bytes);
+      double total = 0.0;
+      for (size_t x : need) total += (double)x;
+      if (total <= budget || S == 1) break;
     }
-    double total = 0.0;
-    for (size_t x : need) total += (double)x;
-    if (total <= budget || S == 1) break;
   }
   for (int g : ctx->order) ctx->geoms[g]->slot = slot_of[g];
   while ((int)ctx->slots.size() < S) {
@@ -670,16 +728,24 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   ctx->two_stage_batch = ctx->two_stage_force != 0;
   std::stable_sort(ctx->order.begin(), ctx->order.end(),
                    [&](int a, int b) { return ctx->geoms[a]->plan.n > ctx->geoms[b]->plan.n; });
-  for (int g : ctx->order) {
-    const GeomPlan& p = ctx->geoms[g]->plan;
-    if (eigen) MBD_CUDA(ctx->geoms[g]->hmat.reserve(sizeof(double) * (size_t)p.nH * p.ldH));
+  if (eigen) {
+    Sections h;
+    std::vector<size_t> at;
+    for (int g : ctx->order) {
+      const GeomPlan& p = ctx->geoms[g]->plan;
+      at.push_back(h.add(sizeof(double) * (size_t)p.nH * p.ldH));
+    }
+    MBD_CUDA(ctx->hmats.reserve(h.size));
+    for (size_t k = 0; k < at.size(); ++k)
+      ctx->geoms[ctx->order[k]]->hmat = reinterpret_cast<double*>(ctx->hmats.as<char>() + at[k]);
   }
   const size_t nev = ctx->geoms.size() * kGeomEvents;
-  while (ctx->events.size() < nev) {
-    cudaEvent_t e;
-    MBD_CUDA(cudaEventCreate(&e));
-    ctx->events.push_back(e);
-  }
+  for (auto& set : ctx->events)
+    while (set.size() < nev) {
+      cudaEvent_t e;
+      MBD_CUDA(cudaEventCreate(&e));
+      set.push_back(e);
+    }
   if (ctx->order.empty()) {
     ctx->n_slots = 0;
     ctx->n_trd_groups = ctx->trd_total_ctas = ctx->n_eig_jobs = ctx->n_eig_batch = 0;
@@ -752,7 +818,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
     for (int j : tp.bins[b]) {
       GeomDev* gd = ctx->geoms[one_stage[j]].get();
       const GeomPlan& p = gd->plan;
-      jobs.push_back(TridiagJob{gd->hmat.as<double>(), p.nH, p.ldH, gd->d, gd->e});
+      jobs.push_back(TridiagJob{gd->hmat, p.nH, p.ldH, gd->d, gd->e});
       gr.nmax = std::max(gr.nmax, p.nH);
     }
     gr.job_end = (int)jobs.size();
@@ -853,7 +919,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   std::memcpy(host.data() + b_jobs + b_groups, eig.data(), sizeof(EigJob) * eig.size());
   std::memcpy(host.data() + b_jobs + b_groups + b_eig, bjobs.data(), sizeof(BandJob) * bjobs.size());
   std::memcpy(host.data() + b_jobs + b_groups + b_eig + b_bj, items.data(), sizeof(SweepItem) * items.size());
-  MBD_CUDA(h2d_ordered(ctx, base, host.data(), host.size()));
+  if (!host.empty()) MBD_CUDA(h2d_ordered(ctx, base, host.data(), host.size()));
   ctx->h2d_bytes += (double)host.size();
   return MBD_OK;
 }
@@ -910,11 +976,12 @@ int reserve_mixed(mbd_ctx* ctx) {
 // cleared and its epochs restarted on every run.
 int enqueue_batch(mbd_ctx* ctx, int mode) {
   cudaStream_t s = ctx->stream;
+  const cudaEvent_t* bev = ctx->bev[ctx->event_set];
   ctx->launches = 0;
   MBD_CUDA(cudaMemsetAsync(ctx->err_flag, 0, sizeof(int), s));
-  record_timing(ctx, ctx->bev[0], s);
+  record_timing(ctx, bev[0], s);
   if (ctx->order.empty()) {
-    for (int k = 1; k < 5; ++k) record_timing(ctx, ctx->bev[k], s);
+    for (int k = 1; k < 5; ++k) record_timing(ctx, bev[k], s);
     return cuda_status(cudaGetLastError());
   }
   // relay and CFDM stages, geometries spread over the slots' streams
@@ -935,7 +1002,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
     MBD_CUDA(cudaEventRecord(ctx->slots[k]->done, ctx->slots[k]->stream));
     MBD_CUDA(cudaStreamWaitEvent(s, ctx->slots[k]->done, 0));
   }
-  record_timing(ctx, ctx->bev[1], s);
+  record_timing(ctx, bev[1], s);
   // bands -> tridiagonal in one persistent launch; matrices too large for the
   // two-stage path in one grouped one-stage launch
   if (ctx->n_trd_groups > 0) {
@@ -943,7 +1010,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
                                    ctx->tridiag_ws.p, ctx->err_flag, s));
     ctx->launches += 2;
   }
-  record_timing(ctx, ctx->bev[4], s);
+  record_timing(ctx, bev[4], s);
   if (ctx->n_band_cluster > 0) {
     MBD_CUDA(launch_sb2st_cluster(ctx->band_jobs, ctx->n_band_cluster, ctx->band_cluster_max_n,
                                   ctx->band_cluster_C, s));
@@ -955,7 +1022,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
                           ctx->num_sms, ctx->band_max_n, ctx->sweeps_in_flight, ctx->test_stall_wait ? 0 : -1, s));
     ctx->launches += 3;
   }
-  record_timing(ctx, ctx->bev[2], s);
+  record_timing(ctx, bev[2], s);
   // eigenvalues and energies
   launch_eigen_batch(ctx->eig_jobs, ctx->n_eig_batch, ctx->eig_batch_max_n, s);
   ctx->launches += ctx->n_eig_batch > 0 ? 1 : 0;
@@ -966,7 +1033,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
   }
   launch_energy_batch(ctx->eig_jobs, ctx->n_eig_jobs, s);
   ctx->launches += ctx->n_eig_jobs > 0 ? 1 : 0;
-  record_timing(ctx, ctx->bev[3], s);
+  record_timing(ctx, bev[3], s);
   return cuda_status(cudaGetLastError());
 }
 
@@ -1015,6 +1082,7 @@ bool capture_batch(mbd_ctx* ctx, int mode, bool first) {
     return false;
   }
   ctx->graph[mode] = exec;
+  ctx->graph_events[mode] = ctx->event_set;
   ctx->graph_first[mode] = first;
   ctx->graph_launches[mode] = ctx->launches;
   return true;
@@ -1058,7 +1126,8 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
   MBD_CUDA(cudaSetDevice(device));
   ctx->num_sms = prop.multiProcessorCount;
   MBD_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-  for (auto& e : ctx->bev) MBD_CUDA(cudaEventCreate(&e));
+  for (auto& set : ctx->bev)
+    for (auto& e : set) MBD_CUDA(cudaEventCreate(&e));
   MBD_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
   MBD_CUDA(create_lookahead(&ctx->la_ctx));
   {
@@ -1133,10 +1202,12 @@ void mbd_rsscs_destroy(mbd_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
-  for (auto e : ctx->events) cudaEventDestroy(e);
+  for (auto& set : ctx->events)
+    for (auto e : set) cudaEventDestroy(e);
   drop_graphs(ctx);
-  for (auto e : ctx->bev)
-    if (e) cudaEventDestroy(e);
+  for (auto& set : ctx->bev)
+    for (auto e : set)
+      if (e) cudaEventDestroy(e);
   if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   if (ctx->la_ctx.ready) cudaEventDestroy(ctx->la_ctx.ready);
   if (ctx->la_ctx.done) cudaEventDestroy(ctx->la_ctx.done);
@@ -1167,14 +1238,12 @@ int upload_batch(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms, bool eigen) {
   ctx->h2d_bytes = 0;
   while ((int)ctx->geoms.size() < n_geom) ctx->geoms.emplace_back(new GeomDev());
   ctx->geoms.resize(n_geom);
+  if (!eigen) resolve_timings(ctx);   // a training batch's stages record the same events
+  int st = upload_geometries(ctx, n_geom, geoms);
+  if (st != MBD_OK) return st;
   int first = MBD_OK;
-  for (int g = 0; g < n_geom; ++g) {
-    int st = upload_geometry(ctx, geoms[g], ctx->geoms[g].get());
-    ctx->geoms[g]->status_host = st;
-    if (st != MBD_OK && first == MBD_OK) first = st;
-    if (st == MBD_ERR_OUT_OF_MEMORY || st == MBD_ERR_DEVICE) return st;
-  }
-  int st = prepare_batch(ctx, eigen);
+  for (int g = 0; g < n_geom && first == MBD_OK; ++g) first = ctx->geoms[g]->status_host;
+  st = prepare_batch(ctx, eigen);
   if (st != MBD_OK) return st;
   ctx->have_batch = eigen;
   return first;
@@ -1212,6 +1281,11 @@ int mbd_rsscs_compute(mbd_ctx* ctx, int mode) {
   // the iterations seen instead and the first graph is kept for the next
   // batch.
   const bool repeat = ctx->mode_runs[mode]++ > 0;
+  // this compute's timing events: a replay's are those of its capture; else
+  // the set that the last compute did not use
+  const int events = ctx->use_graphs && repeat && ctx->graph[mode] ? ctx->graph_events[mode] : 1 - ctx->event_set;
+  if (ctx->timed.pending && ctx->timed.set == events) resolve_timings(ctx);
+  ctx->event_set = events;
   if (ctx->use_graphs && repeat && ctx->graph[mode] && ctx->graph_first[mode] &&
       mode == MBD_MODE_MIXED_LEARNED) {
     if (ctx->graph_prev[mode]) cudaGraphExecDestroy(ctx->graph_prev[mode]);
@@ -1243,73 +1317,29 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
   NvtxRange nvtx("mbd_b200 download");
   if (!ctx || !ctx->have_batch || !out) return MBD_ERR_ARG;
   MBD_CUDA(cudaSetDevice(ctx->device));
-  // Every geometry's results in one pass into page-locked memory: the block
-  // alpha_iw .. energy and the block info .. CG state of its results buffer,
-  // queued behind the batch on the context stream, one synchronisation.
-  struct Range {
-    const char* lo;
-    size_t bytes, at;
-  };
-  auto range = [](const void* a, const void* b_end) {
-    const char* lo = static_cast<const char*>(a);
-    return Range{lo, (size_t)(static_cast<const char*>(b_end) - lo), 0};
-  };
-  std::vector<Range> r1(ctx->geoms.size()), r2(ctx->geoms.size());
-  size_t stage = 256;
-  for (size_t g = 0; g < ctx->geoms.size(); ++g) {
-    const GeomDev* gd = ctx->geoms[g].get();
-    if (gd->status_host != MBD_OK) continue;
-    r1[g] = range(gd->alpha_iw, gd->energy + 8);
-    r2[g] = range(gd->info, gd->cgstate + (size_t)kNFreq * kCgState);
-    r1[g].at = stage;
-    stage += (r1[g].bytes + 255) & ~size_t(255);
-    r2[g].at = stage;
-    stage += (r2[g].bytes + 255) & ~size_t(255);
-  }
-  MBD_CUDA(ctx->staging.reserve(stage));
+  // Every geometry's results in one copy into page-locked memory, queued
+  // behind the batch on the context stream, one synchronisation.
+  constexpr size_t kHead = 256;   // the error flag
+  MBD_CUDA(ctx->staging.reserve(kHead + ctx->out_bytes));
   char* hs = ctx->staging.as<char>();
+  const char* dev_out = ctx->results.as<char>();
   MBD_CUDA(cudaMemcpyAsync(hs, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   ctx->d2h_bytes = sizeof(int);
-  auto fetch = [&](size_t g, cudaStream_t s) -> cudaError_t {
-    for (const Range* r : {&r1[g], &r2[g]}) {
-      cudaError_t e = cudaMemcpyAsync(hs + r->at, r->lo, r->bytes, cudaMemcpyDeviceToHost, s);
-      if (e != cudaSuccess) return e;
-      ctx->d2h_bytes += (double)r->bytes;
-    }
-    return cudaSuccess;
+  auto fetch = [&](size_t at, size_t bytes, cudaStream_t s) -> cudaError_t {
+    ctx->d2h_bytes += (double)bytes;
+    return cudaMemcpyAsync(hs + kHead + at, dev_out + at, bytes, cudaMemcpyDeviceToHost, s);
   };
-  for (size_t g = 0; g < ctx->geoms.size(); ++g)
-    if (ctx->geoms[g]->status_host == MBD_OK) MBD_CUDA(fetch(g, ctx->stream));
+  auto fetch_one = [&](const GeomDev* gd, cudaStream_t s) { return fetch(gd->out_at, gd->out_bytes, s); };
+  if (!ctx->order.empty()) MBD_CUDA(fetch(0, ctx->out_bytes, ctx->stream));
   MBD_CUDA(cudaStreamSynchronize(ctx->stream));
   int err = 0;
   std::memcpy(&err, hs, sizeof(int));
-  // host copy of a device array inside geometry g's two blocks
-  auto host = [&](size_t g, const void* dev) -> const char* {
-    const char* d = static_cast<const char*>(dev);
-    const Range& r = (d >= r1[g].lo && d < r1[g].lo + r1[g].bytes) ? r1[g] : r2[g];
-    return hs + r.at + (d - r.lo);
-  };
-  // stage timings: relay/CFDM stages summed over geometries (they overlap on
-  // the slots' streams), the batch-wide stages and the total from batch events
-  for (int k = 0; k < Stage::kCount; ++k) ctx->last_ms[k] = 0.0;
-  auto elapsed = [](cudaEvent_t a, cudaEvent_t b) {
-    float ms = 0.f;
-    return cudaEventElapsedTime(&ms, a, b) == cudaSuccess ? (double)ms : 0.0;
-  };
-  ctx->last_ms[Stage::kTotal] = elapsed(ctx->bev[0], ctx->bev[3]);
-  ctx->last_ms[Stage::kTridiag] = elapsed(ctx->bev[1], ctx->bev[2]);
-  ctx->last_band_ms = ctx->last_trace_ms = 0.0;
-  ctx->last_chase_ms = ctx->last_ms[Stage::kTridiag];
-  ctx->last_onestage_ms = elapsed(ctx->bev[1], ctx->bev[4]);
-  ctx->last_sb2st_ms = elapsed(ctx->bev[4], ctx->bev[2]);
-  ctx->last_ms[Stage::kEig] = elapsed(ctx->bev[2], ctx->bev[3]);
-  for (int g : ctx->order) {
-    cudaEvent_t* evs = ctx->events.data() + (size_t)g * kGeomEvents;
-    for (int k = 1; k + 1 < kGeomEvents; ++k) ctx->last_ms[k] += elapsed(evs[k - 1], evs[k]);
-    const double last = elapsed(evs[kGeomEvents - 2], evs[kGeomEvents - 1]);
-    ctx->last_ms[ctx->geoms[g]->trace ? Stage::kEig : Stage::kTridiag] += last;
-    (ctx->geoms[g]->trace ? ctx->last_trace_ms : ctx->last_band_ms) += last;
-  }
+  auto host = [&](const void* dev) -> const char* { return hs + kHead + (static_cast<const char*>(dev) - dev_out); };
+  // the stage timings are read from their events when someone asks for them
+  ctx->timed.pending = true;
+  ctx->timed.set = ctx->event_set;
+  ctx->timed.geoms.clear();
+  for (int g : ctx->order) ctx->timed.geoms.emplace_back(g, ctx->geoms[g]->trace);
   int first = MBD_OK;
   for (size_t g = 0; g < ctx->geoms.size(); ++g) {
     GeomDev* gd = ctx->geoms[g].get();
@@ -1330,13 +1360,13 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
     if (ctx->last_mode != MBD_MODE_PLAIN_FP64) {
       // residual gate of the mixed relay solve; a miss re-runs this geometry
       // with the direct FP64 solve (the plain path) before reading results
-      const double* rn = reinterpret_cast<const double*>(host(g, gd->rnorm2));
+      const double* rn = reinterpret_cast<const double*>(host(gd->rnorm2));
       double worst = 0.0;
       for (int f = 0; f < 21; ++f) worst = std::max(worst, std::sqrt(rn[f] / (3.0 * N)));
       r.err_est[0] = r.err_est[1] = r.err_est[2] = worst;
       r.refine_iters = mixed_direct(*gd, *ctx->slots[gd->slot]) ? 1 : kRefineIters;
       if (ctx->last_mode == MBD_MODE_MIXED_LEARNED) {
-        const double* cs = reinterpret_cast<const double*>(host(g, gd->cgstate));
+        const double* cs = reinterpret_cast<const double*>(host(gd->cgstate));
         double most = 0.0, most1 = 0.0;
         bool indefinite = false;
         for (int f = 0; f < kNFreq; ++f) {
@@ -1358,7 +1388,7 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
         if (st == MBD_OK && !gd->trace) st = run_tail_single(ctx, gd, ctx->slots[gd->slot]->stream);
         if (st != MBD_OK) return st;
         const cudaStream_t ss = ctx->slots[gd->slot]->stream;
-        MBD_CUDA(fetch(g, ss));   // the re-run's results replace the staged ones
+        MBD_CUDA(fetch_one(gd, ss));   // the re-run's results replace the staged ones
         MBD_CUDA(cudaStreamSynchronize(ss));
         r.refine_iters = -1;
       }
@@ -1366,24 +1396,24 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
     if (gd->trace && err == 0) {
       // a refused trace form (an imaginary mode, or a Hamiltonian too near
       // one): the eigenvalues, if the relay gave a Hamiltonian at all
-      const double* sc = reinterpret_cast<const double*>(host(g, gd->scalars));
-      const int* fi = reinterpret_cast<const int*>(host(g, gd->info));
+      const double* sc = reinterpret_cast<const double*>(host(gd->scalars));
+      const int* fi = reinterpret_cast<const int*>(host(gd->info));
       bool relay_ok = sc[2] == 0.0;
       for (int f = 0; f < 21; ++f) relay_ok = relay_ok && fi[f] == 0;
-      if (relay_ok && reinterpret_cast<const double*>(host(g, gd->energy))[3] != kTraceOk) {
+      if (relay_ok && reinterpret_cast<const double*>(host(gd->energy))[3] != kTraceOk) {
         const cudaStream_t ss = ctx->slots[gd->slot]->stream;
         int st = run_tail_single(ctx, gd, ss);
         if (st != MBD_OK) return st;
         MBD_CUDA(cudaMemcpyAsync(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ss));
-        MBD_CUDA(fetch(g, ss));
+        MBD_CUDA(fetch_one(gd, ss));
         MBD_CUDA(cudaStreamSynchronize(ss));
       }
     }
-    const double* aiw = reinterpret_cast<const double*>(host(g, gd->alpha_iw));
-    const double* molpol = reinterpret_cast<const double*>(host(g, gd->molpol));
-    const double* scal = reinterpret_cast<const double*>(host(g, gd->scalars));
-    const double* en = reinterpret_cast<const double*>(host(g, gd->energy));
-    const int* info = reinterpret_cast<const int*>(host(g, gd->info));
+    const double* aiw = reinterpret_cast<const double*>(host(gd->alpha_iw));
+    const double* molpol = reinterpret_cast<const double*>(host(gd->molpol));
+    const double* scal = reinterpret_cast<const double*>(host(gd->scalars));
+    const double* en = reinterpret_cast<const double*>(host(gd->energy));
+    const int* info = reinterpret_cast<const int*>(host(gd->info));
     int status = MBD_OK;
     for (int f = 0; f < 21; ++f)
       if (info[f] != 0) status = MBD_ERR_RELAY_NOT_SPD;
@@ -1404,11 +1434,11 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
       for (int q = 0; q < N; ++q)
         for (int f = 0; f < 21; ++f) r.alpha_iw[f + 21 * (size_t)pm[q]] = aiw[(size_t)f * N + q];
     if (r.alpha_eff) {
-      const double* a = reinterpret_cast<const double*>(host(g, gd->alpha_eff));
+      const double* a = reinterpret_cast<const double*>(host(gd->alpha_eff));
       for (int q = 0; q < N; ++q) r.alpha_eff[pm[q]] = a[q];
     }
     if (r.c6_eff) {
-      const double* c = reinterpret_cast<const double*>(host(g, gd->c6_eff));
+      const double* c = reinterpret_cast<const double*>(host(gd->c6_eff));
       for (int q = 0; q < N; ++q) r.c6_eff[pm[q]] = c[q];
     }
     if (r.molpol_eig)
@@ -1743,6 +1773,7 @@ int mbd_rsscs_get_option(mbd_ctx* ctx, int option, double* value) {
 
 int mbd_rsscs_last_timings(mbd_ctx* ctx, double* ms, int n) {
   if (!ctx || !ms || n < Stage::kCount) return MBD_ERR_ARG;
+  resolve_timings(ctx);
   for (int k = 0; k < Stage::kCount; ++k) ms[k] = ctx->last_ms[k];
   if (n >= Stage::kCount + 2) {
     ms[Stage::kCount] = ctx->last_band_ms;        // dense -> band, summed over geometries

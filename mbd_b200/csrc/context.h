@@ -6,6 +6,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "gnn.h"
@@ -78,14 +79,13 @@ struct HostBuf {
 // Per-geometry device state that must survive until download.
 struct GeomDev {
   GeomPlan plan;
-  DevBuf inputs;     // coords, alpha0, c6free, r0, hirsh, shifts, diff data
-  DevBuf results;    // alpha_w, sgm, rvdw_iso, alpha_iw, molpol, c6_eff, alpha_eff, omega, rvdw_eff, scalars, energy, info, d, e, ev
-  DevBuf hmat;       // CFDM Hamiltonian (nH x ldH, lower blocks), reduced in place
+  double* hmat = nullptr;   // CFDM Hamiltonian (nH x ldH, lower blocks), in the context's hmats
+  size_t out_at = 0, out_bytes = 0;   // this geometry's part of the results that go back to the host
   DevBuf band;       // two-stage reduction: the band, nH x kBandLd
-  // offsets into inputs (doubles unless noted)
+  // in the context's inputs
   const double *coords, *alpha0, *c6free, *r0, *hirsh, *scs_shifts, *cfdm_shifts, *diff_shift;
   const int *diff_is_zero, *place_offset, *place_rc, *place_cc;
-  // results
+  // in the context's results
   double *alpha_w, *sgm, *rvdw_iso, *alpha_iw, *molpol, *c6_eff, *alpha_eff, *omega, *rvdw_eff;
   double *scalars, *energy, *d, *e, *ev, *rnorm2;
   double* cgstate;   // [21][kCgState] block-CG recurrence state (MIXED_LEARNED)
@@ -168,7 +168,9 @@ struct mbd_ctx {
   int n_slots = 0;                           // slots in use for the current batch
   mbd::DevBuf tridiag_ws, tables, misc, fb_ws;
   mbd::DevBuf fb_band, fb_trd;   // a refused trace form's reduction (never part of a graph)
-  mbd::HostBuf staging;   // download: every geometry's results in one pass
+  mbd::DevBuf inputs, results, hmats;   // the batch's geometries: inputs; results (first what goes back); Hamiltonians
+  size_t out_bytes = 0;                 // of results, what goes back to the host
+  mbd::HostBuf in_staging, staging;     // upload and download: one copy for the batch
   mbd::Sy2sbLookAhead la_ctx{};   // look-ahead stream and events of the context-stream reductions
   bool lookahead = true;     // dense -> band look-ahead (MBD_B200_LOOKAHEAD=0: off)
   bool priorities = true;    // stream and graph-node priorities (MBD_B200_PRIORITY=0: off)
@@ -203,9 +205,18 @@ struct mbd_ctx {
   double* loss_dev = nullptr;
   int* err_flag = nullptr;
   mbd::TridiagJob* job_dev = nullptr;
-  std::vector<cudaEvent_t> events;           // kGeomEvents per geometry
-  // start, relay done, tridiag done, end, one-stage launch done
-  cudaEvent_t bev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  // timing events, two sets used in turn (a download's timings are read from
+  // theirs when asked for, which may be after the next compute): kGeomEvents
+  // per geometry; start, relay done, tridiag done, end, one-stage launch done
+  std::vector<cudaEvent_t> events[2];
+  cudaEvent_t bev[2][5] = {};
+  int event_set = 0;
+  int graph_events[3] = {0, 0, 0};           // the set each captured graph records
+  struct {
+    bool pending = false;
+    int set = 0;
+    std::vector<std::pair<int, bool>> geoms; // geometries that ran, and whether by the trace form
+  } timed;                                   // the last download's timings, not read yet
   cudaEvent_t fork_ev = nullptr;             // releases the slot streams at the start of a compute
   // one captured graph of mbd_rsscs_compute per mode, valid until the next
   // upload or workspace reallocation
@@ -320,6 +331,7 @@ inline int tuned_chase_c(const mbd_ctx* ctx, int n) { return ctx->tune[tune_clas
 // uploaded batch and its buffers).  keep_first: a graph captured at a first
 // compute is kept for the next batch's first compute to update.
 void drop_graphs(mbd_ctx* ctx, bool keep_first = false);
+void resolve_timings(mbd_ctx* ctx);
 int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only = false);
 int upload_batch(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms, bool eigen);
 // learn.cpp

@@ -208,6 +208,7 @@ int reserve_learned(mbd_ctx* ctx) {
     bool fp32 = ctx->cg_fp32_mode == 1;
     if (ctx->cg_fp32_mode < 0) {
       size_t need = 0, held = 0, free_b = 0, total_b = 0;
+      bool there = true;   // the copies' memory is there: no question of how much is free
       for (int s = 0; s < ctx->n_slots; ++s) {
         size_t r32 = 0;
         for (int g : ctx->order)
@@ -215,9 +216,13 @@ int reserve_learned(mbd_ctx* ctx) {
             r32 = std::max(r32, sizeof(float) * (size_t)kNFreq * ctx->geoms[g]->plan.n * ctx->geoms[g]->plan.ld);
         need += r32;
         held += ctx->slots[s]->relay32.bytes;
+        there = there && r32 <= ctx->slots[s]->relay32.bytes;
       }
-      MBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      fp32 = (double)need <= 0.5 * (double)(free_b + held);
+      fp32 = there;
+      if (!there) {
+        MBD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        fp32 = (double)need <= 0.5 * (double)(free_b + held);
+      }
     }
     moved = fp32 != ctx->cg_fp32;   // the captured launches carry the choice
     ctx->cg_fp32 = fp32;

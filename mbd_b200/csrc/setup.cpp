@@ -247,11 +247,12 @@ int build_plan(const mbd_geom& g, GeomPlan* p) {
   // reference's own r <= mbd_scs_dip_cutoff test (UTILS.f90:574,623) still
   // applies inside it.
   // sigma = (alpha / 3 sqrt(2 / pi))^(1/3) rises with alpha: its extremes
-  // come from the extremes of alpha over atoms and frequencies
+  // come from the extremes of alpha over atoms and frequencies, and alpha
+  // falls with the frequency: the grid's first and last
   double rmax_iso = 0.0, amax = 0.0, amin = 1e300;
   for (int i = 0; i < N; ++i) {
     rmax_iso = std::max(rmax_iso, std::pow(p->hirsh[i], kOtd) * p->r0[i]);
-    for (int f = 0; f < kNFreq; ++f) {
+    for (int f : {0, kNFreq - 1}) {
       double w = kCasimirOmega[f];
       double wp = (4.0 / 3.0) * p->c6free[i] / (p->alpha0[i] * p->alpha0[i]);
       double aw = (p->hirsh[i] * p->alpha0[i]) / (1.0 + (w * w) / (wp * wp));

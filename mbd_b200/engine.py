@@ -232,8 +232,10 @@ class _Packed:
     """Host arrays of one geometry kept alive for the duration of a call."""
 
     def __init__(self, geo: Geometry, st: Settings, z: np.ndarray | None = None):
-        self.z = np.ascontiguousarray(z if z is not None else
-                                      np.array([element_z(s) for s in geo.names], dtype=np.int32))
+        if z is None:
+            known = {s: element_z(s) for s in set(geo.names)}
+            z = np.array([known[s] for s in geo.names], dtype=np.int32)
+        self.z = np.ascontiguousarray(z)
         self.coords = np.ascontiguousarray(geo.coords / BOHR, dtype=np.float64)   # MBD_rsSCS.f90:211
         self.hirsh = np.ascontiguousarray(geo.hirshfeld, dtype=np.float64)
         # lattice(3,3) column-major, columns = vectors == rows of geo.lattice in C order
