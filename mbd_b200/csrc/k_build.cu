@@ -57,6 +57,11 @@ __device__ __forceinline__ bool folded_row(int N, int* i, int* j0) {
   return true;
 }
 
+// Beyond r = kFarX beta R the Fermi exponential exp(-6 (x - 1)) is below
+// 5.2e-17 < 2^-53: 1 + exp(..) is 1, so the short-range damping is exactly 0
+// (the image adds nothing) and the long-range one exactly 1.
+constexpr double kFarX = 1.0 + 37.5 / 6.0;
+
 // Value type of the tensor arithmetic: FP64, or FP32 from FP64 displacements
 // (the image set is always selected in FP64: r <= cut exactly as
 // UTILS.f90:574,623 test it).
@@ -80,7 +85,10 @@ struct TensorMath<true> {
 // (scs_offdiag_block 591-633, scs_diag_block 543-587).  The 3x3 blocks of a
 // warp's 32 consecutive pairs go out through shared memory as whole block
 // rows: 96 contiguous doubles (FP64, double2 stores) or floats (FP32, float4
-// stores) per matrix row.
+// stores) per matrix row.  Bound by the FP64 arithmetic of the images in
+// range: those whose damping is exactly 0 are left out (20 A instead of the 32 A
+// of the image list), and an image out of range costs no square root.
+// Periodic box of 2000 atoms 11.6 -> 4.4 ms; 256 atoms 1.8 -> 0.54.
 template <int FCH, bool F32>
 __global__ void __launch_bounds__(kBuildThreads) relay_build_kernel(RelayBuildArgs a) {
   using M = TensorMath<F32>;
@@ -101,6 +109,8 @@ __global__ void __launch_bounds__(kBuildThreads) relay_build_kernel(RelayBuildAr
   const double d0x = xi - a.coords[3 * jj], d0y = yi - a.coords[3 * jj + 1], d0z = zi - a.coords[3 * jj + 2];
   const double rv12 = diag ? 2.0 * a.rvdw_iso[i] : a.rvdw_iso[i] + a.rvdw_iso[jj];
   const T inv_brv = (T)(1.0 / (a.beta * rv12));
+  const double far = kFarX * a.beta * rv12, lim = fmin(a.cut, far);
+  const double lim2 = lim * lim * (1.0 + 1e-14);   // r2 beyond it: sqrt(r2) > lim for certain
   const T c4pi = (T)sqrt(4.0 / kPiD), c16pi = (T)sqrt(16.0 / kPiD);
 
   T sg[FCH];
@@ -124,7 +134,7 @@ __global__ void __launch_bounds__(kBuildThreads) relay_build_kernel(RelayBuildAr
   for (int s = diag ? 1 : 0; s < a.n_shifts; ++s) {
     const double dxd = d0x + a.shifts[3 * s], dyd = d0y + a.shifts[3 * s + 1], dzd = d0z + a.shifts[3 * s + 2];
     const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
-    if (!(sqrt(r2d) <= a.cut)) continue;
+    if (!(r2d <= lim2) || !(sqrt(r2d) <= a.cut)) continue;
     const T dx = (T)dxd, dy = (T)dyd, dz = (T)dzd;
     const T r2 = (T)r2d;
     const T r = F32 ? (T)sqrt(r2d) : sqrt(r2);
@@ -204,6 +214,9 @@ __global__ void __launch_bounds__(kBuildThreads) relay_build_kernel(RelayBuildAr
 }
 
 // One thread: atom pair (r = blockIdx.y, c), cell difference blockIdx.z.
+// Bound by the FP64 arithmetic of the images in range; an image out of range
+// costs no square root and a far one no exponential (box of 2000 atoms 3.6 ->
+// 2.4 ms).
 // lr_bare_dipole_tensor (UTILS.f90:1098-1153) summed over supercell images
 // (cfdm_diag_block 998-1043 / cfdm_offdiag_block 1047-1094), then placed at
 // every (row cell, col cell) with that difference (supercell_*_block 883-994).
@@ -223,12 +236,15 @@ __global__ void __launch_bounds__(128) cfdm_build_kernel(CfdmBuildArgs a) {
   // UTILS.f90:1028 (same atom, same cell) and 1086 (all other blocks)
   const double pref = self ? wr * wr * a.alpha_eff[r] : wr * wc * sqrt(a.alpha_eff[r] * a.alpha_eff[c]);
   double acc[6] = {0, 0, 0, 0, 0, 0};
+  const double cut2 = a.cut * a.cut * (1.0 + 1e-14);   // r2 beyond it: sqrt(r2) > cut for certain
   for (int s = self ? 1 : 0; s < a.n_shifts; ++s) {
     const double dx = d0x + a.shifts[3 * s], dy = d0y + a.shifts[3 * s + 1], dz = d0z + a.shifts[3 * s + 2];
     const double r2 = dx * dx + dy * dy + dz * dz;
+    if (!(r2 <= cut2)) continue;
     const double rr = sqrt(r2);
     if (!(rr <= a.cut)) continue;
-    const double fermi = 1.0 / (1.0 + exp(-6.0 * (rr * inv_brv - 1.0)));
+    const double x = rr * inv_brv;
+    const double fermi = x > kFarX ? 1.0 : 1.0 / (1.0 + exp(-6.0 * (x - 1.0)));
     const double s5 = fermi / (r2 * r2 * rr);
     const double ca = -3.0 * s5, cb = r2 * s5;   // (r^2 I - 3 dd)/r^5 * fermi
     acc[0] += ca * dx * dx + cb;
