@@ -543,7 +543,7 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
     TraceArgs ta{gd->hmat, p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
                  sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag};
     MBD_CUDA(launch_trace_energy(ta, ctx->num_sms, s));
-    ctx->launches += kTraceLaunches;
+    ctx->launches += trace_launches(p.nH);
   } else if (two_stage(ctx, p.nH)) {
     MBD_CUDA(launch_sy2sb(gd->hmat, p.ldH, p.nH, sl.trd_ws.as<double>(), gd->band.as<double>(),
                           ctx->num_sms, s, tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),

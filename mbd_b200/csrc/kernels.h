@@ -290,7 +290,7 @@ struct TraceArgs {
 };
 constexpr double kTraceOk = 1.0, kTraceRefused = 2.0;
 size_t trace_ws_bytes(int n);
-constexpr int kTraceLaunches = 5;
+int trace_launches(int n);
 cudaError_t launch_trace_energy(const TraceArgs& a, int num_sms, cudaStream_t s);
 
 // ---- block-CG relay solve of the MIXED_LEARNED mode (UTILS.f90:469-473) ----
