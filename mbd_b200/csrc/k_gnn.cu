@@ -67,28 +67,34 @@ __global__ void features_kernel(const int* species, const double* hirsh, const d
   xo[7] = (float)log1p(omega[f]);
 }
 
-// filt[l][e][k] = Wf_l[k] . e_e (l = 0..2), g[e] = wg . e_e
-__global__ void filter_kernel(const float* P, const float* efeat, int E, float* filt, float* g) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)E * (kGnnLayers * H + 1);
-  if (idx >= total) return;
-  const int e = (int)(idx / (kGnnLayers * H + 1));
-  const int c = (int)(idx % (kGnnLayers * H + 1));
-  const float* ee = efeat + (size_t)e * NR;
-  if (c == kGnnLayers * H) {
-    const float* wg = P + kGnnOffWg;
+// filt[l][e][k] = Wf_l[k] . e_e (l = 0..2), g[e] = wg . e_e.  A thread keeps
+// the weights of one output in registers and takes the CTA's edges in turn
+// (their features broadcast from shared memory); bound by the stores.  With
+// the weights and features read from global memory for every output: 74 us at
+// 15 000 edges, 8 now.
+constexpr int kFilterEdges = 32;
+constexpr int kFilterOut = kGnnLayers * H + 1;
+__global__ void __launch_bounds__(224) filter_kernel(const float* P, const float* efeat, int E, float* filt, float* g) {
+  __shared__ __align__(16) float es[kFilterEdges][NR];
+  const int e0 = blockIdx.x * kFilterEdges, ne = min(kFilterEdges, E - e0), c = threadIdx.x;
+  for (int t = threadIdx.x; t < ne * NR; t += blockDim.x) es[t / NR][t % NR] = efeat[(size_t)e0 * NR + t];
+  const int l = c / H, k = c % H;
+  float W[NR];
+  if (c < kFilterOut) {
+    const float* Wg = c == kGnnLayers * H ? P + kGnnOffWg : P + kGnnOffWf(l) + k * NR;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) W[q] = Wg[q];
+  }
+  __syncthreads();
+  if (c >= kFilterOut) return;
+  float* out = c == kGnnLayers * H ? g + e0 : filt + ((size_t)l * E + e0) * H + k;
+  const int stride = c == kGnnLayers * H ? 1 : H;
+  for (int e = 0; e < ne; ++e) {
     float s = 0.f;
 #pragma unroll
-    for (int q = 0; q < NR; ++q) s += wg[q] * ee[q];
-    g[e] = s;
-    return;
+    for (int q = 0; q < NR; ++q) s += W[q] * es[e][q];
+    out[(size_t)e * stride] = s;
   }
-  const int l = c / H, k = c % H;
-  const float* W = P + kGnnOffWf(l) + k * NR;
-  float s = 0.f;
-#pragma unroll
-  for (int q = 0; q < NR; ++q) s += W[q] * ee[q];
-  filt[((size_t)l * E + e) * H + k] = s;
 }
 
 __global__ void embed_kernel(const float* P, const float* x, int M, float* pre0, float* h0) {
@@ -104,41 +110,78 @@ __global__ void embed_kernel(const float* P, const float* x, int M, float* pre0,
   h0[idx] = silu(s);
 }
 
-// m[f*N+i][k] = sum_{e in nbr(i)} filt[e][k] h[f*N+nbr[e]][k]
-__global__ void conv_kernel(const float* h, const float* filt, const int* off, const int* nbr, int N, int F,
-                            float* m) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)N * F * H) return;
-  const int node = (int)(idx / H), k = (int)(idx % H);
-  const int f = node / N, i = node % N;
-  const float* hf = h + (size_t)f * N * H;
-  float s = 0.f;
-  for (int e = off[i]; e < off[i + 1]; ++e) s += filt[(size_t)e * H + k] * hf[(size_t)nbr[e] * H + k];
-  m[idx] = s;
-}
-
-// u = Wu m + bu; h_out = h_in + silu(u).  256 threads = 4 nodes x 64 outputs.
-__global__ void __launch_bounds__(256) dense_kernel(const float* P, int l, const float* m, const float* h_in,
-                                                    float* u, float* h_out, int M) {
-  __shared__ float Wt[H][H + 1];   // Wt[q][k] = Wu[k][q]
-  __shared__ float ms[4][H];
-  const float* W = P + kGnnOffWu(l);
-  for (int t = threadIdx.x; t < H * H; t += blockDim.x) Wt[t % H][t / H] = W[t];
-  const float bk = P[kGnnOffBu(l) + threadIdx.x % H];
-  const int k = threadIdx.x % H, sub = threadIdx.x / H;
-  for (int n0 = blockIdx.x * 4; n0 < M; n0 += gridDim.x * 4) {
-    __syncthreads();
-    const int node = n0 + sub;
-    ms[sub][k] = node < M ? m[(size_t)node * H + k] : 0.f;
-    __syncthreads();
-    if (node < M) {
-      float s = bk;
-#pragma unroll 16
-      for (int q = 0; q < H; ++q) s += Wt[q][k] * ms[sub][q];
-      u[(size_t)node * H + k] = s;
-      h_out[(size_t)node * H + k] = h_in[(size_t)node * H + k] + silu(s);
+// m[f*N+i][k] = sum_{e in nbr(i)} filt[e][k] h[f*N+nbr[e]][k] (plus start[f*N+i][k]
+// where given).  A CTA takes an atom and kConvGroups * kConvF frequencies: a
+// filter entry is read once for a thread's kConvF frequencies, and the loads
+// of four edges are in flight together.
+constexpr int kConvGroups = 4, kConvF = 2;
+__global__ void __launch_bounds__(64 * kConvGroups) conv_kernel(const float* h, const float* filt, const int* off,
+                                                               const int* nbr, int N, int F, const float* start,
+                                                               float* m) {
+  const int i = blockIdx.x, k = threadIdx.x % H, fg = threadIdx.x / H;
+  const int e0 = off[i], e1 = off[i + 1];
+  const int f0 = blockIdx.y * kConvGroups * kConvF;
+  float s[kConvF];
+#pragma unroll
+  for (int u = 0; u < kConvF; ++u) {
+    const int f = f0 + fg + kConvGroups * u;
+    s[u] = start && f < F ? start[((size_t)f * N + i) * H + k] : 0.f;
+  }
+#pragma unroll 4
+  for (int e = e0; e < e1; ++e) {
+    const float w = filt[(size_t)e * H + k];
+    const float* hj = h + (size_t)nbr[e] * H + k;
+#pragma unroll
+    for (int u = 0; u < kConvF; ++u) {
+      const int f = f0 + fg + kConvGroups * u;
+      if (f < F) s[u] += w * hj[(size_t)f * N * H];
     }
   }
+#pragma unroll
+  for (int u = 0; u < kConvF; ++u) {
+    const int f = f0 + fg + kConvGroups * u;
+    if (f < F) m[((size_t)f * N + i) * H + k] = s[u];
+  }
+}
+
+// Y[16 nodes][64] = (init +) X W^T-like products from shared memory: thread =
+// one node x 4 outputs.  Ws[q][k].
+constexpr int kDenseNodes = 16;
+__device__ __forceinline__ void dense_tile(const float (&Ws)[H][H + 4], const float (&Xs)[kDenseNodes][H + 1], int k4,
+                                           int node, float (&acc)[4]) {
+#pragma unroll 8
+  for (int q = 0; q < H; ++q) {
+    const float4 w = *reinterpret_cast<const float4*>(&Ws[q][k4]);
+    const float x = Xs[node][q];
+    acc[0] += w.x * x;
+    acc[1] += w.y * x;
+    acc[2] += w.z * x;
+    acc[3] += w.w * x;
+  }
+}
+
+// u = Wu m + bu; h_out = h_in + silu(u)
+__global__ void __launch_bounds__(256) dense_kernel(const float* P, int l, const float* m, const float* h_in,
+                                                    float* u, float* h_out, int M) {
+  __shared__ __align__(16) float Wt[H][H + 4];   // Wt[q][k] = Wu[k][q]
+  __shared__ float ms[kDenseNodes][H + 1];
+  const float* W = P + kGnnOffWu(l);
+  const int n0 = blockIdx.x * kDenseNodes;
+  for (int t = threadIdx.x; t < H * H; t += 256) Wt[t % H][t / H] = W[t];
+  for (int t = threadIdx.x; t < kDenseNodes * H; t += 256)
+    ms[t / H][t % H] = n0 + t / H < M ? m[(size_t)n0 * H + t] : 0.f;
+  __syncthreads();
+  const int k4 = 4 * (threadIdx.x & 15), node = threadIdx.x >> 4;
+  float acc[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] = P[kGnnOffBu(l) + k4 + c];
+  dense_tile(Wt, ms, k4, node, acc);
+  if (n0 + node >= M) return;
+  const size_t o = (size_t)(n0 + node) * H + k4;
+  const float4 hi = *reinterpret_cast<const float4*>(h_in + o);
+  *reinterpret_cast<float4*>(u + o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  *reinterpret_cast<float4*>(h_out + o) =
+      make_float4(hi.x + silu(acc[0]), hi.y + silu(acc[1]), hi.z + silu(acc[2]), hi.w + silu(acc[3]));
 }
 
 // s = ws.h + bs, a = wa.h + ca (one warp per node)
@@ -159,18 +202,29 @@ __global__ void sa_kernel(const float* P, const float* h, int M, float* s, float
   }
 }
 
-// S (row-major 3x3) per node
+// Sum over the 8 lanes of a node.
+__device__ __forceinline__ float sum8(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v + __shfl_xor_sync(0xffffffffu, v, 4);
+}
+
+// S (row-major 3x3) per node; 8 lanes share a node's edges
 __global__ void tensor_kernel(const float* s, const float* a, const float* g, const float* eproj, const int* off,
                               const int* nbr, int N, int F, float* S) {
-  const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= N * F) return;
-  const int f = node / N, i = node % N;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, node = idx >> 3, sub = idx & 7;
+  const bool live = node < N * F;
+  const int f = live ? node / N : 0, i = live ? node % N : 0;
   float p[6] = {0, 0, 0, 0, 0, 0};
-  for (int e = off[i]; e < off[i + 1]; ++e) {
-    const float w = a[(size_t)f * N + nbr[e]] * g[e];
+  if (live)
+    for (int e = off[i] + sub; e < off[i + 1]; e += 8) {
+      const float w = a[(size_t)f * N + nbr[e]] * g[e];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) p[c] += w * eproj[(size_t)e * 6 + c];
-  }
+      for (int c = 0; c < 6; ++c) p[c] += w * eproj[(size_t)e * 6 + c];
+    }
+#pragma unroll
+  for (int c = 0; c < 6; ++c) p[c] = sum8(p[c]);
+  if (!live || sub != 0) return;
   const float d = 1.0f + s[node];
   float* o = S + (size_t)node * 9;
   o[0] = d + p[0];
@@ -212,18 +266,21 @@ __device__ __forceinline__ float dot_proj(const float* dS, const float* p) {
 __global__ void readout_bwd_kernel(const float* dS, const float* a, const float* g, const float* eproj,
                                    const int* off, const int* nbr, int N, int F, int E, float* ds, float* da,
                                    float* cw) {
-  const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= N * F) return;
-  const int f = node / N, i = node % N;
-  const float* dSi = dS + (size_t)node * 9;
-  ds[node] = dSi[0] + dSi[4] + dSi[8];
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, node = idx >> 3, sub = idx & 7;   // 8 lanes a node
+  const bool live = node < N * F;
+  const int f = live ? node / N : 0, i = live ? node % N : 0;
+  const float* dSi = dS + (size_t)(live ? node : 0) * 9;
   float acc = 0.f;
-  for (int e = off[i]; e < off[i + 1]; ++e) {
-    const int j = f * N + nbr[e];
-    const float* pe = eproj + (size_t)e * 6;
-    acc += g[e] * dot_proj(dS + (size_t)j * 9, pe);
-    cw[(size_t)f * E + e] = dot_proj(dSi, pe) * a[j];
-  }
+  if (live)
+    for (int e = off[i] + sub; e < off[i + 1]; e += 8) {
+      const int j = f * N + nbr[e];
+      const float* pe = eproj + (size_t)e * 6;
+      acc += g[e] * dot_proj(dS + (size_t)j * 9, pe);
+      cw[(size_t)f * E + e] = dot_proj(dSi, pe) * a[j];
+    }
+  acc = sum8(acc);
+  if (!live || sub != 0) return;
+  ds[node] = dSi[0] + dSi[4] + dSi[8];
   da[node] = acc;
 }
 
@@ -235,44 +292,28 @@ __global__ void readout_dh_kernel(const float* P, const float* ds, const float* 
   dh[idx] = ds[node] * P[kGnnOffWs + k] + da[node] * P[kGnnOffWa + k];
 }
 
-// du = dh * silu'(u); dm = Wu^T du.  256 threads = 4 nodes x 64.
+// du = dh * silu'(u); dm = Wu^T du
 __global__ void __launch_bounds__(256) dense_bwd_kernel(const float* P, int l, const float* dh, const float* u,
                                                         float* du, float* dm, int M) {
-  __shared__ float W[H][H + 1];   // W[k][q]
-  __shared__ float ds_[4][H];
+  __shared__ __align__(16) float W[H][H + 4];   // W[k][q]
+  __shared__ float ds_[kDenseNodes][H + 1];
   const float* Wg = P + kGnnOffWu(l);
-  for (int t = threadIdx.x; t < H * H; t += blockDim.x) W[t / H][t % H] = Wg[t];
-  const int q = threadIdx.x % H, sub = threadIdx.x / H;
-  for (int n0 = blockIdx.x * 4; n0 < M; n0 += gridDim.x * 4) {
-    __syncthreads();
-    const int node = n0 + sub;
+  const int n0 = blockIdx.x * kDenseNodes;
+  for (int t = threadIdx.x; t < H * H; t += 256) W[t / H][t % H] = Wg[t];
+  for (int t = threadIdx.x; t < kDenseNodes * H; t += 256) {
     float d = 0.f;
-    if (node < M) {
-      d = dh[(size_t)node * H + q] * dsilu(u[(size_t)node * H + q]);
-      du[(size_t)node * H + q] = d;
+    if (n0 + t / H < M) {
+      d = dh[(size_t)n0 * H + t] * dsilu(u[(size_t)n0 * H + t]);
+      du[(size_t)n0 * H + t] = d;
     }
-    ds_[sub][q] = d;
-    __syncthreads();
-    if (node < M) {
-      float s = 0.f;
-#pragma unroll 16
-      for (int k = 0; k < H; ++k) s += W[k][q] * ds_[sub][k];
-      dm[(size_t)node * H + q] = s;
-    }
+    ds_[t / H][t % H] = d;
   }
-}
-
-// dh_out[j] = dh_next[j] + sum_{e in nbr(j)} filt[e] * dm[nbr_e]
-__global__ void conv_bwd_kernel(const float* dh_next, const float* dm, const float* filt, const int* off,
-                                const int* nbr, int N, int F, float* dh_out) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)N * F * H) return;
-  const int node = (int)(idx / H), k = (int)(idx % H);
-  const int f = node / N, i = node % N;
-  const float* dmf = dm + (size_t)f * N * H;
-  float s = dh_next[idx];
-  for (int e = off[i]; e < off[i + 1]; ++e) s += filt[(size_t)e * H + k] * dmf[(size_t)nbr[e] * H + k];
-  dh_out[idx] = s;
+  __syncthreads();
+  const int k4 = 4 * (threadIdx.x & 15), node = threadIdx.x >> 4;
+  float acc[4] = {};
+  dense_tile(W, ds_, k4, node, acc);
+  if (n0 + node < M)
+    *reinterpret_cast<float4*>(dm + (size_t)(n0 + node) * H + k4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
 // dfilt[e][k] = sum_f dm[f, src_e][k] h[f, nbr_e][k]
@@ -294,45 +335,123 @@ __global__ void embed_bwd_kernel(float* dh, const float* pre0, int M) {
   dh[idx] *= dsilu(pre0[idx]);
 }
 
-// out[k1][k2] += sum_r A[r][k1] B[r % bmod][k2]  (B == nullptr: B = 1, K2 = 1).
-// Each CTA sums a chunk of 64 rows in registers, then adds atomically.
+// out[k1][k2] += sum_r A[r][k1] B[r][k2] and, where given, bias[k1] += sum_r
+// A[r][k1], for K1 = 64.  A CTA stages 64 rows at a time; a thread keeps a
+// TM x 4 block of the outputs, sums 64 rows, adds them to its total and the
+// totals atomically at the end.  One output per thread and row read both
+// operands from shared memory for every product (17 us a launch, 9 now).
 constexpr int kOuterRows = 64;
-__global__ void __launch_bounds__(256) outer_kernel(const float* A, int K1, const float* B, int K2, long long rows,
-                                                    long long bmod, float* out) {
+template <int K2>
+__global__ void __launch_bounds__(256) outer_kernel(const float* A, const float* B, int rows, float* out, float* bias) {
+  constexpr int TX = K2 / 4, TM = K2 >= 16 ? H * TX / 256 : 1;
   __shared__ float As[kOuterRows][H + 1];
-  __shared__ float Bs[kOuterRows][H + 1];
-  const int nout = K1 * K2;
-  float acc[16];
+  __shared__ __align__(16) float Bs[kOuterRows][K2 + 4];
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;   // outputs k1 = TM ty .., k2 = 4 tx ..
+  const bool work = TM * ty < H;
+  float acc[TM][4], ab[TM];
 #pragma unroll
-  for (int t = 0; t < 16; ++t) acc[t] = 0.f;
-  for (long long r0 = (long long)blockIdx.x * kOuterRows; r0 < rows; r0 += (long long)gridDim.x * kOuterRows) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < kOuterRows * K1; t += blockDim.x) {
-      const int rr = t / K1, c = t % K1;
-      const long long r = r0 + rr;
-      As[rr][c] = r < rows ? A[r * K1 + c] : 0.f;
-    }
-    for (int t = threadIdx.x; t < kOuterRows * K2; t += blockDim.x) {
-      const int rr = t / K2, c = t % K2;
-      const long long r = r0 + rr;
-      Bs[rr][c] = (r < rows) ? (B ? B[(r % bmod) * K2 + c] : 1.0f) : 0.f;
-    }
-    __syncthreads();
+  for (int t = 0; t < TM; ++t) {
+    ab[t] = 0.f;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const int o = threadIdx.x + 256 * t;
-      if (o < nout) {
-        const int k1 = o / K2, k2 = o % K2;
-        float s = 0.f;
-        for (int rr = 0; rr < kOuterRows; ++rr) s += As[rr][k1] * Bs[rr][k2];
-        acc[t] += s;
+    for (int c = 0; c < 4; ++c) acc[t][c] = 0.f;
+  }
+  for (int r0 = blockIdx.x * kOuterRows; r0 < rows; r0 += gridDim.x * kOuterRows) {
+    __syncthreads();
+    const int nr = min(kOuterRows, rows - r0);
+    for (int t = threadIdx.x; t < kOuterRows * H; t += 256)
+      As[t / H][t % H] = t < nr * H ? A[(size_t)r0 * H + t] : 0.f;
+    for (int t = threadIdx.x; t < kOuterRows * K2; t += 256)
+      Bs[t / K2][t % K2] = t < nr * K2 ? B[(size_t)r0 * K2 + t] : 0.f;
+    __syncthreads();
+    if (!work) continue;
+    float s[TM][4], sb[TM];
+#pragma unroll
+    for (int t = 0; t < TM; ++t) {
+      sb[t] = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s[t][c] = 0.f;
+    }
+#pragma unroll 8
+    for (int rr = 0; rr < kOuterRows; ++rr) {
+      const float4 b = *reinterpret_cast<const float4*>(&Bs[rr][4 * tx]);
+#pragma unroll
+      for (int t = 0; t < TM; ++t) {
+        const float x = As[rr][TM * ty + t];
+        sb[t] += x;
+        s[t][0] += x * b.x;
+        s[t][1] += x * b.y;
+        s[t][2] += x * b.z;
+        s[t][3] += x * b.w;
       }
     }
-  }
 #pragma unroll
-  for (int t = 0; t < 16; ++t) {
-    const int o = threadIdx.x + 256 * t;
-    if (o < nout) atomicAdd(out + o, acc[t]);
+    for (int t = 0; t < TM; ++t) {
+      ab[t] += sb[t];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[t][c] += s[t][c];
+    }
+  }
+  if (!work) return;
+#pragma unroll
+  for (int t = 0; t < TM; ++t) {
+    const int k1 = TM * ty + t;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) atomicAdd(out + k1 * K2 + 4 * tx + c, acc[t][c]);
+    if (bias && tx == 0) atomicAdd(bias + k1, ab[t]);
+  }
+}
+
+// The readout's gradients: ws += ds^T h, wa += da^T h, bs += sum ds, ca += sum da.
+__global__ void __launch_bounds__(256) readout_grad_kernel(const float* ds, const float* da, const float* h, int M,
+                                                           float* ws, float* wa, float* bs, float* ca) {
+  __shared__ float red[4][2][H], one[4][2];
+  const int k = threadIdx.x % H, sub = threadIdx.x / H;
+  float s = 0.f, a = 0.f, s1 = 0.f, a1 = 0.f;
+  for (int r0 = blockIdx.x * kOuterRows; r0 < M; r0 += gridDim.x * kOuterRows) {
+    float cs = 0.f, cw = 0.f, c1 = 0.f, c2 = 0.f;
+#pragma unroll 4
+    for (int r = r0 + sub; r < min(M, r0 + kOuterRows); r += 4) {
+      const float x = h[(size_t)r * H + k], u = ds[r], v = da[r];
+      cs += u * x;
+      cw += v * x;
+      c1 += u;
+      c2 += v;
+    }
+    s += cs;
+    a += cw;
+    s1 += c1;
+    a1 += c2;
+  }
+  red[sub][0][k] = s;
+  red[sub][1][k] = a;
+  if (k == 0) {
+    one[sub][0] = s1;
+    one[sub][1] = a1;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * H) {
+    const int w = threadIdx.x / H;
+    atomicAdd((w ? wa : ws) + k, (red[0][w][k] + red[1][w][k]) + (red[2][w][k] + red[3][w][k]));
+    if (k == 0) atomicAdd(w ? ca : bs, (one[0][w] + one[1][w]) + (one[2][w] + one[3][w]));
+  }
+}
+
+// wg += sum over frequencies and edges of cw[f][e] efeat[e]
+__global__ void __launch_bounds__(256) edge_grad_kernel(const float* cw, const float* efeat, int F, int E, float* wg) {
+  __shared__ float red[16][NR];
+  const int q = threadIdx.x % NR, sub = threadIdx.x / NR;
+  float t = 0.f;
+  for (int e = blockIdx.x * 16 + sub; e < E; e += gridDim.x * 16) {
+    float c = 0.f;
+    for (int f = 0; f < F; ++f) c += cw[(size_t)f * E + e];
+    t += c * efeat[(size_t)e * NR + q];
+  }
+  red[sub][q] = t;
+  __syncthreads();
+  if (threadIdx.x < NR) {
+    float v = 0.f;
+    for (int u = 0; u < 16; ++u) v += red[u][q];
+    atomicAdd(wg + q, v);
   }
 }
 
@@ -475,12 +594,15 @@ __global__ void __launch_bounds__(1024) graph_scan_kernel(int* a, int N, int* E)
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-void outer(const float* A, int K1, const float* B, int K2, long long rows, long long bmod, float* out,
-           cudaStream_t s) {
+dim3 conv_grid(const GnnGraph& g) {
+  return dim3(g.N, (g.F + kConvGroups * kConvF - 1) / (kConvGroups * kConvF));
+}
+
+template <int K2>
+void outer(const float* A, const float* B, int rows, float* out, float* bias, cudaStream_t s) {
   if (rows <= 0) return;
-  const long long chunks = (rows + kOuterRows - 1) / kOuterRows;
-  const unsigned g = (unsigned)(chunks < 592 ? chunks : 592);
-  outer_kernel<<<g, 256, 0, s>>>(A, K1, B, K2, rows, bmod, out);
+  const int chunks = (rows + kOuterRows - 1) / kOuterRows;
+  outer_kernel<K2><<<chunks < 592 ? chunks : 592, 256, 0, s>>>(A, B, rows, out, bias);
 }
 
 }  // namespace
@@ -552,16 +674,15 @@ void gnn_features(const int* species, const double* hirsh, const double* alpha_w
 int gnn_forward(const float* P, const GnnGraph& g, const GnnWork& w, cudaStream_t s) {
   const int M = g.N * g.F;
   if (g.E > 0)
-    filter_kernel<<<blocks((long long)g.E * (kGnnLayers * H + 1), 256), 256, 0, s>>>(P, g.efeat, g.E, w.filt, w.g);
+    filter_kernel<<<blocks(g.E, kFilterEdges), 224, 0, s>>>(P, g.efeat, g.E, w.filt, w.g);
   embed_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(P, g.x, M, w.pre0, w.h[0]);
-  const unsigned dg = blocks(M, 4) < 1184 ? blocks(M, 4) : 1184;
   for (int l = 0; l < kGnnLayers; ++l) {
-    conv_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(w.h[l], w.filt + (size_t)l * g.E * H, g.off, g.nbr,
-                                                              g.N, g.F, w.m[l]);
-    dense_kernel<<<dg, 256, 0, s>>>(P, l, w.m[l], w.h[l], w.u[l], w.h[l + 1], M);
+    conv_kernel<<<conv_grid(g), 64 * kConvGroups, 0, s>>>(w.h[l], w.filt + (size_t)l * g.E * H, g.off, g.nbr, g.N, g.F,
+                                                 nullptr, w.m[l]);
+    dense_kernel<<<blocks(M, kDenseNodes), 256, 0, s>>>(P, l, w.m[l], w.h[l], w.u[l], w.h[l + 1], M);
   }
   sa_kernel<<<blocks((long long)M * 32, 256), 256, 0, s>>>(P, w.h[kGnnLayers], M, w.s, w.a);
-  tensor_kernel<<<blocks(M, 128), 128, 0, s>>>(w.s, w.a, w.g, g.eproj, g.off, g.nbr, g.N, g.F, w.S);
+  tensor_kernel<<<blocks(8LL * M, 128), 128, 0, s>>>(w.s, w.a, w.g, g.eproj, g.off, g.nbr, g.N, g.F, w.S);
   return 3 + 2 * kGnnLayers + (g.E > 0 ? 1 : 0);
 }
 
@@ -569,31 +690,30 @@ int gnn_loss_backward(const float* P, const GnnGraph& g, const GnnWork& w, float
   const int M = g.N * g.F;
   int launches = 0;
   loss_kernel<<<blocks(M, 256), 256, 0, s>>>(w.S, w.S_true, M, w.dS, loss);
-  readout_bwd_kernel<<<blocks(M, 128), 128, 0, s>>>(w.dS, w.a, w.g, g.eproj, g.off, g.nbr, g.N, g.F, g.E, w.ds, w.da,
+  readout_bwd_kernel<<<blocks(8LL * M, 128), 128, 0, s>>>(w.dS, w.a, w.g, g.eproj, g.off, g.nbr, g.N, g.F, g.E, w.ds, w.da,
                                                      w.cw);
   readout_dh_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(P, w.ds, w.da, M, w.dh);
   launches += 3;
   const float* h3 = w.h[kGnnLayers];
-  outer(w.ds, 1, h3, H, M, M, G + kGnnOffWs, s);
-  outer(w.ds, 1, nullptr, 1, M, 1, G + kGnnOffBs, s);
-  outer(w.da, 1, h3, H, M, M, G + kGnnOffWa, s);
-  outer(w.da, 1, nullptr, 1, M, 1, G + kGnnOffCa, s);
-  if (g.E > 0) outer(w.cw, 1, g.efeat, kGnnRbf, (long long)g.F * g.E, g.E, G + kGnnOffWg, s);
-  launches += 5;
-  const unsigned dg = blocks(M, 4) < 1184 ? blocks(M, 4) : 1184;
+  readout_grad_kernel<<<blocks(M, kOuterRows) < 592 ? blocks(M, kOuterRows) : 592, 256, 0, s>>>(
+      w.ds, w.da, h3, M, G + kGnnOffWs, G + kGnnOffWa, G + kGnnOffBs, G + kGnnOffCa);
+  if (g.E > 0)
+    edge_grad_kernel<<<blocks(g.E, 16) < 296 ? blocks(g.E, 16) : 296, 256, 0, s>>>(w.cw, g.efeat, g.F, g.E,
+                                                                                  G + kGnnOffWg);
+  launches += 2;
   float* dh = w.dh;
   float* dh_alt = w.dh2;
   for (int l = kGnnLayers - 1; l >= 0; --l) {
-    dense_bwd_kernel<<<dg, 256, 0, s>>>(P, l, dh, w.u[l], w.du, w.dm, M);
-    outer(w.du, H, w.m[l], H, M, M, G + kGnnOffWu(l), s);
-    outer(w.du, H, nullptr, 1, M, 1, G + kGnnOffBu(l), s);
-    conv_bwd_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(dh, w.dm, w.filt + (size_t)l * g.E * H, g.off,
-                                                                  g.nbr, g.N, g.F, dh_alt);
-    launches += 4;
+    dense_bwd_kernel<<<blocks(M, kDenseNodes), 256, 0, s>>>(P, l, dh, w.u[l], w.du, w.dm, M);
+    outer<H>(w.du, w.m[l], M, G + kGnnOffWu(l), G + kGnnOffBu(l), s);
+    // dh_out[j] = dh[j] + sum_{e in nbr(j)} filt[e] dm[nbr_e] (the lists are symmetric)
+    conv_kernel<<<conv_grid(g), 64 * kConvGroups, 0, s>>>(w.dm, w.filt + (size_t)l * g.E * H, g.off, g.nbr, g.N, g.F, dh,
+                                                 dh_alt);
+    launches += 3;
     if (g.E > 0) {
       dfilt_kernel<<<blocks((long long)g.E * H, 256), 256, 0, s>>>(w.dm, w.h[l], g.src, g.nbr, g.N, g.F, g.E,
                                                                    w.dfilt);
-      outer(w.dfilt, H, g.efeat, kGnnRbf, g.E, g.E, G + kGnnOffWf(l), s);
+      outer<kGnnRbf>(w.dfilt, g.efeat, g.E, G + kGnnOffWf(l), nullptr, s);
       launches += 2;
     }
     float* t = dh;
@@ -601,9 +721,8 @@ int gnn_loss_backward(const float* P, const GnnGraph& g, const GnnWork& w, float
     dh_alt = t;
   }
   embed_bwd_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(dh, w.pre0, M);
-  outer(dh, H, g.x, kGnnIn, M, M, G + kGnnOffW0, s);
-  outer(dh, H, nullptr, 1, M, 1, G + kGnnOffB0, s);
-  return launches + 3;
+  outer<kGnnIn>(dh, g.x, M, G + kGnnOffW0, G + kGnnOffB0, s);
+  return launches + 2;
 }
 
 void gnn_adam(float* P, float* G, float* m1, float* m2, int step, float lr, cudaStream_t s) {
