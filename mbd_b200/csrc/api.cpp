@@ -1165,6 +1165,7 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
   MBD_CUDA(init_device_constants());
   MBD_CUDA(init_cholflow_attributes());
   MBD_CUDA(init_trsv_attributes());
+  MBD_CUDA(init_eigvec_attributes());
   MBD_CUDA(init_cg_attributes());
   MBD_CUDA(init_eigval_attributes());
   MBD_CUDA(init_tc3_attributes());
@@ -1519,14 +1520,15 @@ int mbd_rsscs_eigh(mbd_ctx* ctx, const double* H, int n, int ld, double* w, doub
   if (!ctx || !H || !w || !Z || n < 1 || ld < n || ldz < n) return MBD_ERR_ARG;
   MBD_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  constexpr int NBW = 128;   // reflectors per compact-WY block of the back-transformation
+  constexpr int NBW = kWyNB;   // reflectors per compact-WY block of the back-transformation
+  const size_t nwy = (n + NBW - 1) / NBW;
   const size_t ldp = round_up(n, 32);
   const size_t nn = (size_t)n * ldp;
   const int G = tridiag_group_ctas(ctx, n);
   const size_t wsb = tridiag_workspace_bytes(n, G);
   MBD_CUDA(ctx->eig_ws.reserve(wsb));
   // A, V (reflectors), X, X2 (vectors), Gram; scratch; W, W2 (NBW x n);
-  // S, T (NBW x NBW); tau, d, e, ev (2n); the deviation word
+  // S, T (NBW x NBW a block); tau, d, e, ev (2n); the deviation word
   size_t off = 0;
   std::vector<size_t> o;
   auto add = [&](size_t doubles) { o.push_back(off); off += (doubles + 31) & ~size_t(31); };
@@ -1538,8 +1540,8 @@ int mbd_rsscs_eigh(mbd_ctx* ctx, const double* H, int n, int ld, double* w, doub
   add(eigh_scratch_doubles(n));
   add((size_t)NBW * n);
   add((size_t)NBW * n);
-  add((size_t)NBW * NBW);
-  add((size_t)NBW * NBW);
+  add(nwy * NBW * NBW);
+  add(nwy * NBW * NBW);
   add(n);
   add(n);
   add(n);
@@ -1608,15 +1610,19 @@ int mbd_rsscs_eigh(mbd_ctx* ctx, const double* H, int n, int ld, double* w, doub
   // the last block first; V^T of a block is row-major (kb x m) at
   // V + c0 * ldp + c0 + 1
   const int nr = n - 1;
+  for (int c0 = 0; c0 < nr; c0 += NBW) {   // S = V^T V of every block, then every T
+    const int kb = std::min(NBW, nr - c0);
+    const double* Vt = V + (size_t)c0 * ldp + c0 + 1;
+    dgemm_rm(false, true, kb, kb, n - c0 - 1, 1.0, Vt, ldp, Vt, ldp, 0.0, Sg + (size_t)(c0 / NBW) * NBW * NBW, NBW, s);
+  }
+  launch_wy_t(Sg, tau, nr, Tb, s);
   for (int c0 = nr > 0 ? ((nr - 1) / NBW) * NBW : -1; c0 >= 0; c0 -= NBW) {
     const int kb = std::min(NBW, nr - c0);
     const int m = n - c0 - 1;
     const double* Vt = V + (size_t)c0 * ldp + c0 + 1;
     double* Xs = X + (size_t)(c0 + 1) * ldp;
-    dgemm_rm(false, true, kb, kb, m, 1.0, Vt, ldp, Vt, ldp, 0.0, Sg, NBW, s);    // S = V^T V
-    launch_wy_t(Sg, tau + c0, kb, NBW, Tb, s);
     dgemm_rm(false, false, kb, n, m, 1.0, Vt, ldp, Xs, ldp, 0.0, W, n, s);       // W = V^T X
-    dgemm_rm(false, false, kb, n, kb, 1.0, Tb, NBW, W, n, 0.0, W2, n, s);        // W2 = T W
+    dgemm_rm(false, false, kb, n, kb, 1.0, Tb + (size_t)(c0 / NBW) * NBW * NBW, NBW, W, n, 0.0, W2, n, s);   // W2 = T W
     dgemm_rm(true, false, m, n, kb, -1.0, Vt, ldp, W2, n, 1.0, Xs, ldp, s);      // X -= V W2
   }
   MBD_CUDA(cudaGetLastError());

@@ -296,22 +296,36 @@ __global__ void ns_prepare_kernel(double* G, int n, unsigned long long* dev) {
 // T (nb x nb, row-major, upper) of the forward compact-WY form
 // H_0 ... H_{kb-1} = I - V T V^T from the Gram matrix S = V^T V (row-major,
 // ld nb) and the taus: T(j,j) = tau_j, T(0:j, j) = -tau_j T(0:j, 0:j) S(0:j, j).
-__global__ void wy_t_kernel(const double* __restrict__ S, const double* __restrict__ tau, int kb, int nb, double* T) {
-  const int i = threadIdx.x;   // blockDim.x == nb
-  for (int c = 0; c < nb; ++c) T[i * nb + c] = 0.0;
-  __syncthreads();
+// One CTA per block of reflectors, T in shared memory, eight threads to a row
+// of it; bound by the nb dependent columns (340 us a block with a thread per
+// row and T in global memory, and one block after the other).
+constexpr int kWyThreads = 1024;
+static_assert(kWyThreads / 8 == kWyNB, "eight threads to a row");
+constexpr size_t kWySmem = sizeof(double) * (kWyNB * (kWyNB + 1) + kWyNB);
+__global__ void __launch_bounds__(kWyThreads) wy_t_kernel(const double* __restrict__ S0,
+                                                         const double* __restrict__ tau0, int n_refl, double* T0) {
+  extern __shared__ double sh[];
+  double (*Ts)[kWyNB + 1] = reinterpret_cast<double (*)[kWyNB + 1]>(sh);
+  double* sj = sh + kWyNB * (kWyNB + 1);
+  constexpr int nb = kWyNB;
+  const double* S = S0 + (size_t)blockIdx.x * nb * nb;
+  const double* tau = tau0 + (size_t)blockIdx.x * nb;
+  double* T = T0 + (size_t)blockIdx.x * nb * nb;
+  const int kb = min(nb, n_refl - (int)blockIdx.x * nb), i = threadIdx.x >> 3, q = threadIdx.x & 7;
+  for (int t = threadIdx.x; t < nb * nb; t += kWyThreads) Ts[t / nb][t % nb] = 0.0;
   for (int j = 0; j < kb; ++j) {
+    if ((int)threadIdx.x < j) sj[threadIdx.x] = S[threadIdx.x * nb + j];
+    __syncthreads();
     double v = 0.0;
-    if (i < j) {
-      for (int l = i; l < j; ++l) v += T[i * nb + l] * S[l * nb + j];
-      v *= -tau[j];
-    } else if (i == j) {
-      v = tau[j];
-    }
+    for (int l = q; l < j; l += 8) v += Ts[i][l] * sj[l];   // T(i, l) = 0 for l < i
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
     __syncthreads();
-    if (i <= j) T[i * nb + j] = v;
-    __syncthreads();
+    if (q == 0 && i <= j) Ts[i][j] = i == j ? tau[j] : -tau[j] * v;
   }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nb * nb; t += kWyThreads) T[t] = Ts[t / nb][t % nb];
 }
 
 }  // namespace
@@ -347,8 +361,12 @@ void launch_ns_prepare(double* G, int n, unsigned long long* dev, cudaStream_t s
   ns_prepare_kernel<<<std::max(1u, blocks), 256, 0, s>>>(G, n, dev);
 }
 
-void launch_wy_t(const double* S, const double* tau, int kb, int nb, double* T, cudaStream_t s) {
-  wy_t_kernel<<<1, nb, 0, s>>>(S, tau, kb, nb, T);
+cudaError_t init_eigvec_attributes() {
+  return cudaFuncSetAttribute(wy_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWySmem);
+}
+
+void launch_wy_t(const double* S, const double* tau, int n_refl, double* T, cudaStream_t s) {
+  if (n_refl > 0) wy_t_kernel<<<(n_refl + kWyNB - 1) / kWyNB, kWyThreads, kWySmem, s>>>(S, tau, n_refl, T);
 }
 
 }  // namespace mbd

@@ -193,8 +193,12 @@ void launch_tri_vectors(const double* d, const double* e, const double* ev, int 
                         double* scratch, cudaStream_t s);
 // G (n x n) <- 3/2 I - G/2, *dev = max |G - I| as bits (atomic max; zero it first)
 void launch_ns_prepare(double* G, int n, unsigned long long* dev, cudaStream_t s);
-// T (nb x nb row-major upper) of I - V T V^T = H_0 ... H_{kb-1} from S = V^T V (ld nb)
-void launch_wy_t(const double* S, const double* tau, int kb, int nb, double* T, cudaStream_t s);
+// Per block b of kWyNB reflectors (the last may be short): T_b (row-major
+// upper) of I - V T V^T = H_0 H_1 ... from S_b = V^T V and the block's taus; S
+// and T hold kWyNB x kWyNB entries a block.
+constexpr int kWyNB = 128;
+cudaError_t init_eigvec_attributes();
+void launch_wy_t(const double* S, const double* tau, int n_refl, double* T, cudaStream_t s);
 // energy = 0.5*sum_{ev>=0} sqrt(ev)/nsl - 0.5*sum_nonint; out[0]=E, out[1]=sum sqrt, out[2]=nimag
 void launch_energy(const double* ev, int n, int nsl, const double* scalars, double* out,
                    cudaStream_t s);
