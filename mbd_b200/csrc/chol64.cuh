@@ -1,5 +1,5 @@
 // Cholesky factor and inverse of one 64 x 64 block in shared memory by a CTA
-// of 256 threads, and the FP64 tensor-core product they are built on
+// of 128 or 256 threads, and the FP64 tensor-core product they are built on
 // (k_cholflow.cu, k_cg.cu).
 #pragma once
 
@@ -12,7 +12,6 @@ namespace {
 
 constexpr int NB = kCholNB;      // 64
 constexpr int FS = NB + 4;       // row stride of 64-wide shared blocks: a half-warp's 8 x 4 fragment loads hit 16 bank pairs
-constexpr int kDiagThreads = 256;
 
 // D = A B + D with A 8x4 (row), B 4x8 (col), D 8x8 in FP64:
 // a = A[lane/4][lane%4], b = B[lane%4][lane/4], d = D[lane/4][2*(lane%4) + {0,1}].
@@ -102,6 +101,22 @@ __device__ __forceinline__ void update8(double* S, int i, int j, int s, int g, i
   *c = v;
 }
 
+// The same for two block rows at once.
+__device__ __forceinline__ void update8x2(double* S, int i0, int i1, int j, int s, int g, int q) {
+  double2* c0 = reinterpret_cast<double2*>(S + (8 * i0 + g) * FS + 8 * j + 2 * q);
+  double2* c1 = reinterpret_cast<double2*>(S + (8 * i1 + g) * FS + 8 * j + 2 * q);
+  const double *a0 = S + (8 * i0 + g) * FS + 8 * s + q, *a1 = S + (8 * i1 + g) * FS + 8 * s + q;
+  const double* b = S + (8 * j + g) * FS + 8 * s + q;
+  double2 v0 = *c0, v1 = *c1;
+  const double b0 = b[0], b1 = b[4], x0 = a0[0], y0 = a0[4], x1 = a1[0], y1 = a1[4];
+  dmma(v0.x, v0.y, -x0, b0);
+  dmma(v1.x, v1.y, -x1, b0);
+  dmma(v0.x, v0.y, -y0, b1);
+  dmma(v1.x, v1.y, -y1, b1);
+  *c0 = v0;
+  *c1 = v1;
+}
+
 // X(s, s) = L(s, s)^-1, a column per lane; one warp.
 __device__ __forceinline__ void inverse8(const double* S, const double* dinv, double* X, int s, int lane) {
   double x[8];
@@ -134,34 +149,42 @@ __device__ __forceinline__ void inverse_row8(const double* S, double* X, int s, 
 }
 
 // Factors S and inverts the factor into X; dinv, diagx: 64 doubles each.
-// All 256 threads.
+// All THREADS threads of the CTA.
+template <int THREADS>
 __device__ __forceinline__ void diag_factor(double* S, double* X, double* dinv, double* diagx, int tid, int col0,
                                             int n, int* bad, double shift) {
+  constexpr int W = THREADS / 32;
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  for (int e = tid; e < NB * FS / 2; e += kDiagThreads) reinterpret_cast<double2*>(X)[e] = make_double2(0.0, 0.0);
+  for (int e = tid; e < NB * FS / 2; e += THREADS) reinterpret_cast<double2*>(X)[e] = make_double2(0.0, 0.0);
   __syncthreads();
 #pragma unroll 1
   for (int s = 0; s < 10; ++s) {
-    // warp 0: panel s.  The others: what panel s - 1 does to the columns
-    // past s, the inverse of diagonal block s - 1, row s - 2 of the inverse
-    if (warp == 0) {
-      if (s < 8) panel8(S, s, lane, shift, col0, n, bad, dinv, diagx);
+    // warp 0: panel s, while there is one.  The others: what panel s - 1 does to
+    // the columns past s, the inverse of diagonal block s - 1, row s - 2 of the inverse
+    const int h = s < 8 ? warp - 1 : warp, nh = s < 8 ? W - 1 : W;
+    if (h < 0) {
+      panel8(S, s, lane, shift, col0, n, bad, dinv, diagx);
     } else {
-      if (warp == 1 && s >= 1 && s <= 8) inverse8(S, dinv, X, s - 1, lane);
-      if (s >= 2 && warp <= s - 2) inverse_row8(S, X, s - 2, warp - 1, g, q);
+      if (h == 0 && s >= 1 && s <= 8) inverse8(S, dinv, X, s - 1, lane);
+      for (int j = nh - 1 - h; j < s - 2; j += nh) inverse_row8(S, X, s - 2, j, g, q);
       if (s >= 1 && s < 8) {
-        int t = 7 - warp;   // tiles (i, j), s < j <= i < 8, dealt from warp 7 down
+        int t = nh - 1 - h;   // tiles (i, j), s < j <= i < 8, dealt from the last warp down
         for (int j = s + 1; j < 8; ++j)
           for (int i = j; i < 8; ++i)
             if (--t < 0) {
               update8(S, i, j, s - 1, g, q);
-              t = 6;
+              t = nh - 1;
             }
       }
     }
     __syncthreads();
     if (s < 7) {   // panel s on the columns of panel s + 1
-      if (s + 1 + warp < 8) update8(S, s + 1 + warp, s + 1, s, g, q);
+      const int i = s + 1 + warp;
+      if (W < 7 && i + W < 8) {
+        update8x2(S, i, i + W, s + 1, s, g, q);
+      } else if (i < 8) {
+        update8(S, i, s + 1, s, g, q);
+      }
       __syncthreads();
     }
   }

@@ -140,8 +140,9 @@ __device__ __forceinline__ bool stopped(const CgArgs& a, int f) { return a.state
 // sends the geometry to the direct solve).  Bound by the factor's chain of 64
 // pivots; a column-at-a-time factor with dot products by single threads took
 // 153 us a launch (300-atom clusters) against 28.
+constexpr int kTileInvThreads = 256;
 constexpr size_t kTileInvSmem = sizeof(double) * 2 * NB * FS;
-__global__ void __launch_bounds__(kDiagThreads) cg_tile_inv_kernel(CgArgs a) {
+__global__ void __launch_bounds__(kTileInvThreads) cg_tile_inv_kernel(CgArgs a) {
   extern __shared__ __align__(16) double dsm[];
   __shared__ double s_dinv[NB], s_diagx[NB];
   __shared__ int s_bad;
@@ -149,13 +150,13 @@ __global__ void __launch_bounds__(kDiagThreads) cg_tile_inv_kernel(CgArgs a) {
   double* X = dsm + NB * FS;
   const int I = blockIdx.x, f = blockIdx.y, tid = threadIdx.x;
   const double* A = a.A + (size_t)f * a.a_stride;
-  for (int e = tid; e < NB * NB; e += kDiagThreads) {
+  for (int e = tid; e < NB * NB; e += kTileInvThreads) {
     const int r = e / NB, c = e % NB, gr = I * NB + r, gc = I * NB + c;
     S[r * FS + c] = (c <= r && gr < a.n) ? A[(size_t)gr * a.ld + gc] : (r == c ? 1.0 : 0.0);
   }
   if (tid == 0) s_bad = 0;
   __syncthreads();
-  diag_factor(S, X, s_dinv, s_diagx, tid, 0, NB, &s_bad, 0.0);
+  diag_factor<kTileInvThreads>(S, X, s_dinv, s_diagx, tid, 0, NB, &s_bad, 0.0);
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   double o[8][2];
 #pragma unroll
@@ -1047,7 +1048,7 @@ void launch_cg_setup(const CgArgs& a, cudaStream_t s) {
   const long long items = (long long)a.nt * (a.nt + 1) / 2 * a.batch;
   const int tgrid = (int)std::min<long long>(cg_tile_grid<double>(), items);
   cudaMemsetAsync(a.state, 0, sizeof(double) * kCgState * a.batch, s);
-  cg_tile_inv_kernel<<<dim3(a.nt, a.batch), kDiagThreads, kTileInvSmem, s>>>(a);
+  cg_tile_inv_kernel<<<dim3(a.nt, a.batch), kTileInvThreads, kTileInvSmem, s>>>(a);
   cg_tile_kernel<double><<<tgrid, TT, 0, s>>>(a, a.A, a.X);
   cg_rows_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1);
   cg_init_tiles_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a);
