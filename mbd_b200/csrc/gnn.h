@@ -51,7 +51,7 @@ struct GnnWork {
   float *s, *a;            // [M]
   float* S;                // [M][9] prediction
   // training only
-  float *dS, *dh, *dh2, *du, *dm, *ds, *da, *dfilt, *cw, *S_true;
+  float *dS, *dh, *dh2, *du, *du2, *dm, *ds, *da, *dfilt, *cw, *S_true;
 };
 
 // Radius graph of one geometry (the network's neighbour lists): edges

@@ -13,6 +13,9 @@
 // is written as a gather over the receiving node's own list.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <utility>
+
 #include "gnn.h"
 
 namespace mbd {
@@ -115,12 +118,11 @@ __global__ void embed_kernel(const float* P, const float* x, int M, float* pre0,
 // filter entry is read once for a thread's kConvF frequencies, and the loads
 // of four edges are in flight together.
 constexpr int kConvGroups = 4, kConvF = 2;
-__global__ void __launch_bounds__(64 * kConvGroups) conv_kernel(const float* h, const float* filt, const int* off,
-                                                               const int* nbr, int N, int F, const float* start,
-                                                               float* m) {
-  const int i = blockIdx.x, k = threadIdx.x % H, fg = threadIdx.x / H;
+__device__ __forceinline__ void conv(const float* h, const float* filt, const int* off, const int* nbr, int N, int F,
+                                     const float* start, float* m, int i, int fblock) {
+  const int k = threadIdx.x % H, fg = threadIdx.x / H;
   const int e0 = off[i], e1 = off[i + 1];
-  const int f0 = blockIdx.y * kConvGroups * kConvF;
+  const int f0 = fblock * kConvGroups * kConvF;
   float s[kConvF];
 #pragma unroll
   for (int u = 0; u < kConvF; ++u) {
@@ -144,11 +146,16 @@ __global__ void __launch_bounds__(64 * kConvGroups) conv_kernel(const float* h, 
   }
 }
 
+__global__ void __launch_bounds__(64 * kConvGroups) conv_kernel(const float* h, const float* filt, const int* off,
+                                                               const int* nbr, int N, int F, float* m) {
+  conv(h, filt, off, nbr, N, F, nullptr, m, blockIdx.x, blockIdx.y);
+}
+
 // Y[16 nodes][64] = (init +) X W^T-like products from shared memory: thread =
 // one node x 4 outputs.  Ws[q][k].
 constexpr int kDenseNodes = 16;
-__device__ __forceinline__ void dense_tile(const float (&Ws)[H][H + 4], const float (&Xs)[kDenseNodes][H + 1], int k4,
-                                           int node, float (&acc)[4]) {
+__device__ __forceinline__ void dense_tile(const float (*Ws)[H + 4], const float (*Xs)[H + 1], int k4, int node,
+                                           float (&acc)[4]) {
 #pragma unroll 8
   for (int q = 0; q < H; ++q) {
     const float4 w = *reinterpret_cast<const float4*>(&Ws[q][k4]);
@@ -293,12 +300,11 @@ __global__ void readout_dh_kernel(const float* P, const float* ds, const float* 
 }
 
 // du = dh * silu'(u); dm = Wu^T du
-__global__ void __launch_bounds__(256) dense_bwd_kernel(const float* P, int l, const float* dh, const float* u,
-                                                        float* du, float* dm, int M) {
-  __shared__ __align__(16) float W[H][H + 4];   // W[k][q]
-  __shared__ float ds_[kDenseNodes][H + 1];
-  const float* Wg = P + kGnnOffWu(l);
-  const int n0 = blockIdx.x * kDenseNodes;
+__device__ __forceinline__ void dense_bwd(const float* Wg, const float* dh, const float* u, float* du, float* dm, int M,
+                                          int block, float* smem) {
+  float(*W)[H + 4] = reinterpret_cast<float(*)[H + 4]>(smem);   // W[k][q]
+  float(*ds_)[H + 1] = reinterpret_cast<float(*)[H + 1]>(smem + H * (H + 4));
+  const int n0 = block * kDenseNodes;
   for (int t = threadIdx.x; t < H * H; t += 256) W[t / H][t % H] = Wg[t];
   for (int t = threadIdx.x; t < kDenseNodes * H; t += 256) {
     float d = 0.f;
@@ -317,9 +323,9 @@ __global__ void __launch_bounds__(256) dense_bwd_kernel(const float* P, int l, c
 }
 
 // dfilt[e][k] = sum_f dm[f, src_e][k] h[f, nbr_e][k]
-__global__ void dfilt_kernel(const float* dm, const float* h, const int* src, const int* nbr, int N, int F, int E,
-                             float* dfilt) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void filter_grad(const float* dm, const float* h, const int* src, const int* nbr, int N,
+                                            int F, int E, float* dfilt, int block) {
+  const long long idx = (long long)block * 256 + threadIdx.x;
   if (idx >= (long long)E * H) return;
   const int e = (int)(idx / H), k = (int)(idx % H);
   const int i = src[e], j = nbr[e];
@@ -328,24 +334,18 @@ __global__ void dfilt_kernel(const float* dm, const float* h, const int* src, co
   dfilt[idx] = s;
 }
 
-// dpre = dh * silu'(pre0) (in place into dh)
-__global__ void embed_bwd_kernel(float* dh, const float* pre0, int M) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)M * H) return;
-  dh[idx] *= dsilu(pre0[idx]);
-}
-
 // out[k1][k2] += sum_r A[r][k1] B[r][k2] and, where given, bias[k1] += sum_r
-// A[r][k1], for K1 = 64.  A CTA stages 64 rows at a time; a thread keeps a
+// A[r][k1], for K1 = 64; with pre, A[r][k1] silu'(pre[r][k1]) for A.  A CTA stages 64 rows at a time; a thread keeps a
 // TM x 4 block of the outputs, sums 64 rows, adds them to its total and the
 // totals atomically at the end.  One output per thread and row read both
 // operands from shared memory for every product (17 us a launch, 9 now).
 constexpr int kOuterRows = 64;
 template <int K2>
-__global__ void __launch_bounds__(256) outer_kernel(const float* A, const float* B, int rows, float* out, float* bias) {
+__device__ __forceinline__ void outer(const float* A, const float* pre, const float* B, int rows, float* out, float* bias,
+                                      int block, int nblocks, float* smem) {
   constexpr int TX = K2 / 4, TM = K2 >= 16 ? H * TX / 256 : 1;
-  __shared__ float As[kOuterRows][H + 1];
-  __shared__ __align__(16) float Bs[kOuterRows][K2 + 4];
+  float(*As)[H + 1] = reinterpret_cast<float(*)[H + 1]>(smem);
+  float(*Bs)[K2 + 4] = reinterpret_cast<float(*)[K2 + 4]>(smem + kOuterRows * (H + 1));   // 16-byte aligned
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;   // outputs k1 = TM ty .., k2 = 4 tx ..
   const bool work = TM * ty < H;
   float acc[TM][4], ab[TM];
@@ -355,11 +355,12 @@ __global__ void __launch_bounds__(256) outer_kernel(const float* A, const float*
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[t][c] = 0.f;
   }
-  for (int r0 = blockIdx.x * kOuterRows; r0 < rows; r0 += gridDim.x * kOuterRows) {
+  for (int r0 = block * kOuterRows; r0 < rows; r0 += nblocks * kOuterRows) {
     __syncthreads();
     const int nr = min(kOuterRows, rows - r0);
     for (int t = threadIdx.x; t < kOuterRows * H; t += 256)
-      As[t / H][t % H] = t < nr * H ? A[(size_t)r0 * H + t] : 0.f;
+      As[t / H][t % H] =
+          t < nr * H ? (pre ? A[(size_t)r0 * H + t] * dsilu(pre[(size_t)r0 * H + t]) : A[(size_t)r0 * H + t]) : 0.f;
     for (int t = threadIdx.x; t < kOuterRows * K2; t += 256)
       Bs[t / K2][t % K2] = t < nr * K2 ? B[(size_t)r0 * K2 + t] : 0.f;
     __syncthreads();
@@ -402,12 +403,13 @@ __global__ void __launch_bounds__(256) outer_kernel(const float* A, const float*
 }
 
 // The readout's gradients: ws += ds^T h, wa += da^T h, bs += sum ds, ca += sum da.
-__global__ void __launch_bounds__(256) readout_grad_kernel(const float* ds, const float* da, const float* h, int M,
-                                                           float* ws, float* wa, float* bs, float* ca) {
-  __shared__ float red[4][2][H], one[4][2];
+__device__ __forceinline__ void readout_grad(const float* ds, const float* da, const float* h, int M, float* ws,
+                                             float* wa, float* bs, float* ca, int block, int nblocks, float* smem) {
+  float(*red)[2][H] = reinterpret_cast<float(*)[2][H]>(smem);
+  float(*one)[2] = reinterpret_cast<float(*)[2]>(smem + 4 * 2 * H);
   const int k = threadIdx.x % H, sub = threadIdx.x / H;
   float s = 0.f, a = 0.f, s1 = 0.f, a1 = 0.f;
-  for (int r0 = blockIdx.x * kOuterRows; r0 < M; r0 += gridDim.x * kOuterRows) {
+  for (int r0 = block * kOuterRows; r0 < M; r0 += nblocks * kOuterRows) {
     float cs = 0.f, cw = 0.f, c1 = 0.f, c2 = 0.f;
 #pragma unroll 4
     for (int r = r0 + sub; r < min(M, r0 + kOuterRows); r += 4) {
@@ -437,11 +439,12 @@ __global__ void __launch_bounds__(256) readout_grad_kernel(const float* ds, cons
 }
 
 // wg += sum over frequencies and edges of cw[f][e] efeat[e]
-__global__ void __launch_bounds__(256) edge_grad_kernel(const float* cw, const float* efeat, int F, int E, float* wg) {
-  __shared__ float red[16][NR];
+__device__ __forceinline__ void edge_grad(const float* cw, const float* efeat, int F, int E, float* wg, int block,
+                                          int nblocks, float* smem) {
+  float(*red)[NR] = reinterpret_cast<float(*)[NR]>(smem);
   const int q = threadIdx.x % NR, sub = threadIdx.x / NR;
   float t = 0.f;
-  for (int e = blockIdx.x * 16 + sub; e < E; e += gridDim.x * 16) {
+  for (int e = block * 16 + sub; e < E; e += nblocks * 16) {
     float c = 0.f;
     for (int f = 0; f < F; ++f) c += cw[(size_t)f * E + e];
     t += c * efeat[(size_t)e * NR + q];
@@ -453,6 +456,56 @@ __global__ void __launch_bounds__(256) edge_grad_kernel(const float* cw, const f
     for (int u = 0; u < 16; ++u) v += red[u][q];
     atomicAdd(wg + q, v);
   }
+}
+
+// The backward pass in launches of independent parts, a range of blocks each:
+// a part alone leaves most of the device idle (some 20 M = 5000 nodes or
+// 10 000 edges, 10-15 us of latency whatever its size).  A layer is
+//   bwd_kernel       du, dm of the layer; behind them the weight gradients that
+//                    the layer above left (from its du and dfilt), or those of
+//                    the readout
+//   bwd_conv_kernel  dh of the layer below and dfilt, both from dm
+// Training of 16 clusters of 54 to 356 atoms, two epochs: 16.7 -> 14.2 ms against a
+// launch for every part (22 launches a backward pass, 10 now).
+struct BwdJobs {
+  // blocks of each part, in this order
+  int dense, embed, unit, filt, readout, edge;
+  const float *Wu, *dh, *u;                 // dense: du = dh silu'(u), dm = Wu^T du
+  float *du, *dm;
+  const float *pre0, *x;                    // embed: W0, b0 from dh silu'(pre0) and x
+  float *g_w0, *g_b0;
+  const float *du_above, *m_above;          // unit: Wu, bu of the layer above
+  float *g_wu, *g_bu;
+  const float *dfilt, *efeat;               // filt: Wf of the layer above
+  float* g_wf;
+  const float *ds, *da, *h, *cw;            // readout and edge
+  float *g_ws, *g_wa, *g_bs, *g_ca, *g_wg;
+  int M, E, F;
+};
+__global__ void __launch_bounds__(256) bwd_kernel(BwdJobs j) {
+  __shared__ __align__(16) float smem[kOuterRows * (H + 1) + kOuterRows * (H + 4)];
+  int b = blockIdx.x;
+  if (b < j.dense) return dense_bwd(j.Wu, j.dh, j.u, j.du, j.dm, j.M, b, smem);
+  b -= j.dense;
+  if (b < j.embed) return outer<kGnnIn>(j.dh, j.pre0, j.x, j.M, j.g_w0, j.g_b0, b, j.embed, smem);
+  b -= j.embed;
+  if (b < j.unit) return outer<H>(j.du_above, nullptr, j.m_above, j.M, j.g_wu, j.g_bu, b, j.unit, smem);
+  b -= j.unit;
+  if (b < j.filt) return outer<kGnnRbf>(j.dfilt, nullptr, j.efeat, j.E, j.g_wf, nullptr, b, j.filt, smem);
+  b -= j.filt;
+  if (b < j.readout)
+    return readout_grad(j.ds, j.da, j.h, j.M, j.g_ws, j.g_wa, j.g_bs, j.g_ca, b, j.readout, smem);
+  b -= j.readout;
+  edge_grad(j.cw, j.efeat, j.F, j.E, j.g_wg, b, j.edge, smem);
+}
+
+// dh_out[j] = dh[j] + sum_{e in nbr(j)} filt[e] dm[nbr_e] (the lists are
+// symmetric) on the first conv_blocks blocks, dfilt on the rest.
+__global__ void __launch_bounds__(256) bwd_conv_kernel(const float* dm, const float* filt, const float* h, const int* off,
+                                                       const int* nbr, const int* src, int N, int F, int E,
+                                                       const float* dh, float* dh_out, float* dfilt, int conv_blocks) {
+  if ((int)blockIdx.x < conv_blocks) return conv(dm, filt, off, nbr, N, F, dh, dh_out, blockIdx.x % N, blockIdx.x / N);
+  filter_grad(dm, h, src, nbr, N, F, E, dfilt, blockIdx.x - conv_blocks);
 }
 
 __global__ void adam_kernel(float* P, float* G, float* m1, float* m2, int n, float lr, float b1, float b2, float eps,
@@ -598,12 +651,8 @@ dim3 conv_grid(const GnnGraph& g) {
   return dim3(g.N, (g.F + kConvGroups * kConvF - 1) / (kConvGroups * kConvF));
 }
 
-template <int K2>
-void outer(const float* A, const float* B, int rows, float* out, float* bias, cudaStream_t s) {
-  if (rows <= 0) return;
-  const int chunks = (rows + kOuterRows - 1) / kOuterRows;
-  outer_kernel<K2><<<chunks < 592 ? chunks : 592, 256, 0, s>>>(A, B, rows, out, bias);
-}
+// Blocks of a part that sums over rows.
+int sum_blocks(int rows, int per, int most) { return std::min((rows + per - 1) / per, most); }
 
 }  // namespace
 
@@ -612,7 +661,7 @@ size_t gnn_work_floats(int N, int F, int E, bool train) {
   size_t f = M * H * (1 + 4 + 3 + 3)          // pre0, h0..h3, m0..m2, u0..u2
              + (size_t)kGnnLayers * E * H + E // filt, g
              + 2 * M + 9 * M;                 // s, a, S
-  if (train) f += 9 * M + 4 * M * H + 2 * M + (size_t)E * H + (size_t)F * E + 9 * M;   // dS, dh*, ds/da, dfilt, cw, S_true
+  if (train) f += 9 * M + 5 * M * H + 2 * M + (size_t)E * H + (size_t)F * E + 9 * M;   // dS, dh*, ds/da, dfilt, cw, S_true
   return f + 512;   // 8-float alignment of every array of the layout
 }
 
@@ -639,6 +688,7 @@ GnnWork gnn_work_layout(float* base, int N, int F, int E, bool train) {
     w.dh = take(M * H);
     w.dh2 = take(M * H);
     w.du = take(M * H);
+    w.du2 = take(M * H);
     w.dm = take(M * H);
     w.ds = take(M);
     w.da = take(M);
@@ -678,7 +728,7 @@ int gnn_forward(const float* P, const GnnGraph& g, const GnnWork& w, cudaStream_
   embed_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(P, g.x, M, w.pre0, w.h[0]);
   for (int l = 0; l < kGnnLayers; ++l) {
     conv_kernel<<<conv_grid(g), 64 * kConvGroups, 0, s>>>(w.h[l], w.filt + (size_t)l * g.E * H, g.off, g.nbr, g.N, g.F,
-                                                 nullptr, w.m[l]);
+                                                          w.m[l]);
     dense_kernel<<<blocks(M, kDenseNodes), 256, 0, s>>>(P, l, w.m[l], w.h[l], w.u[l], w.h[l + 1], M);
   }
   sa_kernel<<<blocks((long long)M * 32, 256), 256, 0, s>>>(P, w.h[kGnnLayers], M, w.s, w.a);
@@ -694,35 +744,64 @@ int gnn_loss_backward(const float* P, const GnnGraph& g, const GnnWork& w, float
                                                      w.cw);
   readout_dh_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(P, w.ds, w.da, M, w.dh);
   launches += 3;
-  const float* h3 = w.h[kGnnLayers];
-  readout_grad_kernel<<<blocks(M, kOuterRows) < 592 ? blocks(M, kOuterRows) : 592, 256, 0, s>>>(
-      w.ds, w.da, h3, M, G + kGnnOffWs, G + kGnnOffWa, G + kGnnOffBs, G + kGnnOffCa);
-  if (g.E > 0)
-    edge_grad_kernel<<<blocks(g.E, 16) < 296 ? blocks(g.E, 16) : 296, 256, 0, s>>>(w.cw, g.efeat, g.F, g.E,
-                                                                                  G + kGnnOffWg);
-  launches += 2;
+  const int outer_blocks = sum_blocks(M, kOuterRows, 592), filt_blocks = sum_blocks(g.E, kOuterRows, 592);
+  const dim3 cg = conv_grid(g);
   float* dh = w.dh;
   float* dh_alt = w.dh2;
-  for (int l = kGnnLayers - 1; l >= 0; --l) {
-    dense_bwd_kernel<<<blocks(M, kDenseNodes), 256, 0, s>>>(P, l, dh, w.u[l], w.du, w.dm, M);
-    outer<H>(w.du, w.m[l], M, G + kGnnOffWu(l), G + kGnnOffBu(l), s);
-    // dh_out[j] = dh[j] + sum_{e in nbr(j)} filt[e] dm[nbr_e] (the lists are symmetric)
-    conv_kernel<<<conv_grid(g), 64 * kConvGroups, 0, s>>>(w.dm, w.filt + (size_t)l * g.E * H, g.off, g.nbr, g.N, g.F, dh,
-                                                 dh_alt);
-    launches += 3;
-    if (g.E > 0) {
-      dfilt_kernel<<<blocks((long long)g.E * H, 256), 256, 0, s>>>(w.dm, w.h[l], g.src, g.nbr, g.N, g.F, g.E,
-                                                                   w.dfilt);
-      outer<kGnnRbf>(w.dfilt, g.efeat, g.E, G + kGnnOffWf(l), nullptr, s);
-      launches += 2;
+  BwdJobs j{};
+  j.M = M;
+  j.E = g.E;
+  j.F = g.F;
+  j.dfilt = w.dfilt;
+  j.efeat = g.efeat;
+  j.dm = w.dm;
+  for (int l = kGnnLayers; l >= 0; --l) {
+    // launch l: layer l - 1 (the embedding below layer 0) and the gradients layer l left
+    j.dense = l > 0 ? (int)blocks(M, kDenseNodes) : 0;
+    j.embed = l > 0 ? 0 : outer_blocks;
+    j.unit = l < kGnnLayers ? outer_blocks : 0;
+    j.filt = l < kGnnLayers ? filt_blocks : 0;
+    j.readout = l < kGnnLayers ? 0 : outer_blocks;
+    j.edge = l < kGnnLayers ? 0 : sum_blocks(g.E, 16, 296);
+    j.dh = dh;
+    if (l < kGnnLayers) {
+      j.du_above = j.du;
+      j.m_above = w.m[l];
+      j.g_wu = G + kGnnOffWu(l);
+      j.g_bu = G + kGnnOffBu(l);
+      j.g_wf = G + kGnnOffWf(l);
+    } else {
+      j.ds = w.ds;
+      j.da = w.da;
+      j.h = w.h[kGnnLayers];
+      j.cw = w.cw;
+      j.g_ws = G + kGnnOffWs;
+      j.g_wa = G + kGnnOffWa;
+      j.g_bs = G + kGnnOffBs;
+      j.g_ca = G + kGnnOffCa;
+      j.g_wg = G + kGnnOffWg;
     }
-    float* t = dh;
-    dh = dh_alt;
-    dh_alt = t;
+    if (l > 0) {
+      j.Wu = P + kGnnOffWu(l - 1);
+      j.u = w.u[l - 1];
+      j.du = l % 2 ? w.du : w.du2;
+    } else {
+      j.pre0 = w.pre0;
+      j.x = g.x;
+      j.g_w0 = G + kGnnOffW0;
+      j.g_b0 = G + kGnnOffB0;
+    }
+    bwd_kernel<<<j.dense + j.embed + j.unit + j.filt + j.readout + j.edge, 256, 0, s>>>(j);
+    ++launches;
+    if (l == 0) break;
+    const int conv_blocks = (int)(cg.x * cg.y);
+    bwd_conv_kernel<<<conv_blocks + blocks((long long)g.E * H, 256), 256, 0, s>>>(
+        w.dm, w.filt + (size_t)(l - 1) * g.E * H, w.h[l - 1], g.off, g.nbr, g.src, g.N, g.F, g.E, dh, dh_alt, w.dfilt,
+        conv_blocks);
+    ++launches;
+    std::swap(dh, dh_alt);
   }
-  embed_bwd_kernel<<<blocks((long long)M * H, 256), 256, 0, s>>>(dh, w.pre0, M);
-  outer<kGnnIn>(dh, g.x, M, G + kGnnOffW0, G + kGnnOffB0, s);
-  return launches + 2;
+  return launches;
 }
 
 void gnn_adam(float* P, float* G, float* m1, float* m2, int step, float lr, cudaStream_t s) {
