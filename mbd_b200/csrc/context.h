@@ -341,16 +341,18 @@ int reserve_learned(mbd_ctx* ctx);
 int band_to_tridiag_single(mbd_ctx* ctx, double* Br, int n, double* d, double* e, DevBuf& scratch, cudaStream_t s);
 int relay_learned(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cudaEvent_t ev_net, double** X_out);
 
-// Largest Hamiltonian the trace form takes: past it the reduction to a band,
-// (4/3) n^3 operations against ~4 n^3, is the faster one.
+// Largest Hamiltonian the trace form takes: its 21 factors need 14 GB there,
+// and the work grows as 5 to 7 n^3 against (4/3) n^3 of the reduction to a
+// band.  Energy of one cluster (ms, trace form / reduction): n = 1500 0.9 / 17,
+// 3000 4.7 / 37, 6000 37 / 87, 7500 55 / 123, 9000 96 / 165.
 constexpr int kTraceMaxN = 9216;
 
 // Relay matrices the mixed mode solves by the FP64 factors instead of 3xTF32
-// factors and refinement.  Factor + solve (ms, direct / 3xTF32): N = 61 0.14 /
-// 0.76, 533 2.3 / 6.9, 1000 8.8 / 15.4, 2000 54 / 49: the refinement's
-// triangular sweeps and the FP32 panels' chain cost more than the tensor cores
-// save below ~1700 atoms.
-constexpr int kMixedDirectMaxN = 5000;
+// factors and refinement.  Factor + solve + residual (ms, direct / 3xTF32): n =
+// 183 0.14 / 0.76, 1599 2.3 / 6.9, 3000 8.1 / 15.4, 5100 30.0 / 36.2, 6000 47.6 /
+// 48.6, 6600 62 / 59, 7500 90 / 76: the refinement's triangular sweeps and the
+// FP32 panels' chain cost more than the tensor cores save below that.
+constexpr int kMixedDirectMaxN = 5700;
 inline bool mixed_direct(const GeomDev& gd, const RelaySlot& sl) {
   return sl.mixed_direct && gd.plan.n <= kMixedDirectMaxN;
 }
