@@ -46,6 +46,7 @@ METRIC = "MBD energies/s, mixed+batched+learned vs plain FP64 on 1 B200, |dE|<=1
 SIZES = (500, 1000, 2000)
 BOX_SIZES = (2000, 4000, 6000)
 FP64_NOMINAL_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12   # 148 SMs x 64 DFMA/clk x 2 x 1965 MHz
+MIXED_DIRECT_MAX_N = 5700   # largest relay matrix the mixed mode solves by FP64 factors
 TWO_STAGE_MAX_N = 1152 * 16 + 32   # largest Hamiltonian the two-stage reduction takes (panel rows x cluster CTAs + a panel)
 
 
@@ -364,7 +365,7 @@ def roofline(stage_ms, sizes, mode):
     """Roofline of the dominant stage of the last timed step."""
     peaks, src = load_peaks()
     sub = ("total", "tridiag_dense_to_band", "tridiag_to_tridiagonal", "tridiag_one_stage_launch",
-           "tridiag_band_chase_launch")
+           "tridiag_band_chase_launch", "trace_form")
     stages = {k: v for k, v in stage_ms.items() if k not in sub}
     dom = max(stages, key=stages.get)
     one_ms = stage_ms.get("tridiag_one_stage_launch", 0.0)
@@ -410,11 +411,23 @@ def roofline(stage_ms, sizes, mode):
                 "peak_source": f"{src} copy bandwidth (MEASURED_PEAKS.json hbm_gbs)",
                 "algorithmic": "(3N)^3/6 * 8 B per energy (SYMV reads of the trailing lower triangle)",
                 "stage_ms": stages}
+    trace_ms = stage_ms.get("trace_form", 0.0)
+    if dom == "eig_energy" and trace_ms > 0.5 * stages[dom]:
+        achieved = sum(4.0 / 3.0 * (3.0 * n) ** 3 for n in sizes) / (trace_ms / 1000.0) / 1e12
+        return {"bound": "tensor", "kernel": "chol_flow_kernel (FP64 tensor cores; the energy's trace form)",
+                "achieved": achieved, "peak": FP64_NOMINAL_TFLOPS, "unit": "TFLOP/s",
+                "frac": achieved / FP64_NOMINAL_TFLOPS, "traffic": load_traffic().get("chol_flow_kernel"),
+                "kernel_ms": trace_ms,
+                "peak_source": "nominal FP64 (148 SM x 64 DFMA/clk x 1965 MHz); no FP64 entry in MEASURED_PEAKS.json",
+                "algorithmic": "(4/3)(3N)^3 flop per energy, the reduction that the trace form replaces; it does "
+                               "15 to 21 factors of (3N)^3/3 at 25 to 34 TFLOP/s instead (the stage time is summed "
+                               "over the slots' overlapping streams)",
+                "stage_ms": stages}
     if dom == "relay_factor":
         fl = sum(21 * (3.0 * n) ** 3 / 3.0 for n in sizes)
-        if mode == "plain":
+        if mode == "plain" or (mode == "mixed" and all(3 * n <= MIXED_DIRECT_MAX_N for n in sizes)):
             achieved = fl / (stages[dom] / 1000.0) / 1e12
-            return {"bound": "tensor", "kernel": "syrk_lower/trsm_panel/potrf_diag (FP64 DFMA)",
+            return {"bound": "tensor", "kernel": "chol_flow_kernel (FP64 tensor cores)",
                     "achieved": achieved, "peak": FP64_NOMINAL_TFLOPS, "unit": "TFLOP/s",
                     "frac": achieved / FP64_NOMINAL_TFLOPS, "traffic": None,
                     "peak_source": "nominal FP64 (148 SM x 64 DFMA/clk x 1965 MHz); no FP64 entry in MEASURED_PEAKS.json",
@@ -428,8 +441,8 @@ def roofline(stage_ms, sizes, mode):
     note = None
     if dom == "relay_solve" and mode == "mixed_learned":
         note = ("block-CG over the slots' overlapping streams (the stage time is summed over geometries); no "
-                "per-launch timing of its matrix pass cg_tile_kernel here (ncu: 4.72 TB/s, 72 % of the measured "
-                "copy bandwidth on an n = 3000 relay batch)")
+                "per-launch timing of its matrix pass cg_strip_kernel here (3.4 TB/s, 53 % of the measured copy "
+                "bandwidth on an n = 6000 relay batch)")
     return {"bound": "hbm", "kernel": dom, "achieved": None, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
             "frac": None, "traffic": None, "peak_source": src, "note": note, "stage_ms": stages}
 
