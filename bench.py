@@ -441,7 +441,7 @@ def roofline(stage_ms, sizes, mode):
     note = None
     if dom == "relay_solve" and mode == "mixed_learned":
         note = ("block-CG over the slots' overlapping streams (the stage time is summed over geometries); no "
-                "per-launch timing of its matrix pass cg_strip_kernel here (3.4 TB/s, 53 % of the measured copy "
+                "per-launch timing of its matrix pass strip_kernel here (3.4 TB/s, 53 % of the measured copy "
                 "bandwidth on an n = 6000 relay batch)")
     return {"bound": "hbm", "kernel": dom, "achieved": None, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
             "frac": None, "traffic": None, "peak_source": src, "note": note, "stage_ms": stages}

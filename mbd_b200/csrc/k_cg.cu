@@ -10,8 +10,7 @@
 //   Q = A P;  alpha = (P^T Q)^-1 (Z^T R);  X += P alpha;  R -= Q alpha
 //   Z = M^-1 R;  beta = (Z_old^T R_old)^-1 (Z^T R);  P = Z + P beta
 // Four launches per iteration, all frequencies at once (grid.y = f):
-//   cg_strip   partials of A P from the FP32 copy (the lower half serves both
-//              triangles); cg_tile from the FP64 matrix
+//   strip      partials of A P (k_strip.cu; the lower half serves both triangles)
 //   cg_rows    Q = sum of the partials of each 64-row block; partials of P^T Q
 //   cg_update  alpha; X, R, Z = M^-1 R of one 64-row tile per CTA; partials
 //              of Z^T R, R^T R
@@ -23,15 +22,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "chol64.cuh"
 #include "kernels.h"
+#include "strip.cuh"
 
 namespace mbd {
 namespace {
 
-constexpr int CT = 64;       // tile edge (rows)
+constexpr int CT = kStripRows;   // tile edge (rows)
 constexpr int AT = 64;       // atoms per CTA in the per-atom kernels
 constexpr int kRed = 10;     // per-CTA partial sums: a 3x3 matrix and one scalar
 // state[f][kCgState]: [0] stop (0 run, 1 converged, 2 breakdown, 3 negative
@@ -39,14 +38,6 @@ constexpr int kRed = 10;     // per-CTA partial sums: a 3x3 matrix and one scala
 // (odd), [20] R^T R, [kCgIndefinite] 1 when the relay matrix is shown not to
 // be positive definite
 constexpr int kZR0 = 2, kRR = 20;
-
-__device__ __forceinline__ void cg_tri(int t, int* ti, int* tj) {
-  int i = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-  while ((i + 1) * (i + 2) / 2 <= t) ++i;
-  while (i * (i + 1) / 2 > t) --i;
-  *ti = i;
-  *tj = t - i * (i + 1) / 2;
-}
 
 // out = m^-1 (3x3, row-major) by cofactors; false when singular or not finite.
 __device__ __forceinline__ bool inv3(const double* m, double* out) {
@@ -182,429 +173,18 @@ __global__ void __launch_bounds__(kTileInvThreads) cg_tile_inv_kernel(CgArgs a) 
   }
 }
 
-// partial[f][I][J][64 x 3] = A_IJ v_J, and A_IJ^T v_I into [J][I] (I > J).
-// Grid-stride over (tile, frequency) items, so that the launches after every
-// frequency has converged cost a few microseconds.  Thread (ty, tx) of 16 x 16
-// holds the 16 tile entries of rows ty + 16 i and columns {2 tx, 2 tx + 1,
-// 32 + 2 tx, 33 + 2 tx} in registers (16-byte loads, a warp reads two 256-byte
-// row segments per instruction), forms their row and column products with v
-// (6 FMAs per entry) and the 16 partial sums of every output meet in shared
-// memory (fixed order).
-constexpr int TT = 256;           // threads of cg_tile
-constexpr int RP = CT * 3 + 1;    // row stride of the partial-sum buffer (bank spread)
-
-// A float as a double by integer operations: the conversion instruction has an
-// eighth of the ALU's rate, and its queue can set a pass's time.  Zeros
-// and denormals come out as some 1e-38, infinities and NaN as some 1e38 (the
-// residual gate turns such a solve away).
-__device__ __forceinline__ double widen(float x) {
-  const int b = __float_as_int(x);
-  return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
-}
-
-__global__ void __launch_bounds__(TT, 3) cg_tile_kernel(CgArgs a, const double* in) {
-  __shared__ __align__(16) double xI[CT * 3], xJ[CT * 3];
-  __shared__ double buf[16 * RP];
-  const int ntiles = a.nt * (a.nt + 1) / 2;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int n = a.n;
-  const long long items = (long long)ntiles * a.batch;
-  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
-    const int f = (int)(item / ntiles);
-    if (stopped(a, f)) {
-      // skip to this CTA's first item of the next frequency (uniform over the CTA)
-      const long long next = (long long)(f + 1) * ntiles;
-      item += (next - item - 1) / gridDim.x * gridDim.x;
-      continue;
-    }
-    int ti, tj;
-    cg_tri((int)(item % ntiles), &ti, &tj);
-    const bool diag = ti == tj;
-    const double* A = a.A + (size_t)f * a.a_stride;
-    const double* x = in + (size_t)f * a.ystride;
-    // the 16 entries (pair loads; rows start 16-byte aligned, ld a multiple
-    // of 32; an entry beyond n or above the diagonal reads as zero)
-    double t[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i, gr = ti * CT + r;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = 2 * tx + 32 * h, gc = tj * CT + c;
-        double2 v = make_double2(0.0, 0.0);
-        if (gr < n && gc < n && (!diag || c <= r)) v = *reinterpret_cast<const double2*>(A + (size_t)gr * a.ld + gc);
-        t[i][2 * h] = v.x;
-        t[i][2 * h + 1] = (gc + 1 < n && (!diag || c + 1 <= r)) ? v.y : 0.0;
-      }
-    }
-    __syncthreads();   // the previous item's reads of xI / xJ / buf are done
-    for (int idx = tid; idx < CT * 3; idx += TT) {
-      const int gi = ti * CT + idx / 3, gj = tj * CT + idx / 3;
-      xI[idx] = gi < n ? x[(size_t)ti * CT * 3 + idx] : 0.0;
-      xJ[idx] = gj < n ? x[(size_t)tj * CT * 3 + idx] : 0.0;
-    }
-    __syncthreads();
-    double rs[4][3], cs[4][3];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) rs[k][q] = cs[k][q] = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      double xi[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) xi[q] = xI[3 * r + q];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = 2 * tx + 32 * (j >> 1) + (j & 1);
-        const double e = t[i][j];
-        const double ec = (!diag || c < r) ? e : 0.0;   // the diagonal counts once (row side)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          rs[i][q] += e * xJ[3 * c + q];
-          cs[j][q] += ec * xi[q];
-        }
-      }
-    }
-    double* pr = a.partial + (size_t)f * a.nt * a.nt * CT * 3;
-    // row sums: the 16 column groups of each row
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) buf[tx * RP + 3 * (ty + 16 * i) + q] = rs[i][q];
-    __syncthreads();
-    double y = 0.0;
-    if (tid < CT * 3) {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) y += buf[k * RP + tid];
-    }
-    __syncthreads();
-    // column sums: the 16 row groups of each column
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = 2 * tx + 32 * (j >> 1) + (j & 1);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) buf[ty * RP + 3 * c + q] = cs[j][q];
-    }
-    __syncthreads();
-    if (tid < CT * 3) {
-      double z = 0.0;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) z += buf[k * RP + tid];
-      if (!diag) {
-        pr[((size_t)ti * a.nt + tj) * CT * 3 + tid] = y;
-        pr[((size_t)tj * a.nt + ti) * CT * 3 + tid] = z;
-      } else {
-        pr[((size_t)ti * a.nt + ti) * CT * 3 + tid] = y + z;
-      }
-    }
-  }
-}
-
-// ---- FP32 matrix pass ---------------------------------------------------------
-// The same partials from the FP32 copy in chunks of 64 x 128 entries, row
-// block after row block, frequency after frequency; every CTA (one an SM)
-// takes an equal run of chunks.  A warp has 8 rows of a chunk, four entries of
-// every row per lane, brought by 16-byte asynchronous copies three chunks
-// ahead (512 bytes of a row each; a lane reads what it copied itself).  Row
-// sums stay in registers to the end of the row block or the run; column sums
-// cross the eight warps in shared memory, added up while the next chunk is
-// worked on, with one barrier a chunk.  Four products are summed in FP32, two
-// to an instruction (the pass would otherwise stay bound by its 12 FP64 FMAs
-// per entry, not by its halved bytes), everything beyond in FP64: the sums
-// carry a relative error of a few 1e-7, below what either phase of that solve
-// resolves (rms against the FP64 pass 2.6e-8 of the largest entry, as the
-// 64 x 64 tile kernel before).
-// Slots (the three vectors apart) written in partial[f], row block I: [I][2 c]
-// by a run's piece of the row block that begins at chunk c, [I][I] by the last
-// piece together with the diagonal block's columns, and [J][I] with the
-// columns of the blocks J < I.
-// Bound: instruction issue and the FP64 conversions of the sums; the bytes
-// alone (half a matrix per frequency) take half the time.  21 matrices of
-// n = 6000 (1.5 GB): 0.69 ms by tiles with all sums through shared memory,
-// 0.45 now, 0.23 without the arithmetic; an iteration 775 -> 523 us, of
-// n = 3000 223 -> 171 us, of n = 2100 126 -> 105 us.
-constexpr int RW = 8;                       // rows of a warp
-constexpr int ST = 32 * CT / RW;            // threads
-constexpr int kStripRing = 4;               // chunks of a CTA in shared memory, one in use
-constexpr int kColsElems = 2 * (CT / 4) * 3 * 128;
-constexpr int kXElems = 3 * 128 + 3 * CT;   // v on a chunk's columns and rows
-constexpr size_t kStripSmem =
-    sizeof(float) * (kColsElems + (size_t)kStripRing * CT * 128) + sizeof(double) * kStripRing * kXElems;
-constexpr int kMaxActive = 32;              // frequencies of a launch
-
-// Chunks of the row blocks before block I, and the row block of chunk t.
-__host__ __device__ inline int chunks_before(int I) { return (I + 1) / 2 * ((I + 2) / 2); }
-__device__ __forceinline__ int chunk_row(int t) {
-  int m, o;
-  cg_tri(t / 2, &m, &o);                    // m (m + 1) <= t < (m + 1) (m + 2)
-  return t < (m + 1) * (m + 1) ? 2 * m : 2 * m + 1;
-}
-// Chunks of a CTA's run when `act` frequencies of nt row blocks take part.
-__device__ __forceinline__ int strip_run(int nt, int act, int ctas) { return (chunks_before(nt) * act + ctas - 1) / ctas; }
-
-// The frequencies that still run, as a mask; all threads of a warp.
-__device__ __forceinline__ unsigned running(const CgArgs& a) {
-  const int lane = threadIdx.x & 31;
-  return __ballot_sync(0xffffffffu, lane < a.batch && !stopped(a, lane));
-}
-
-// Two floats in one register pair, and the instructions that take them.
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
-__device__ __forceinline__ void ring_copy(unsigned dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void ring_copy(float4* dst, const float* src) {
-  ring_copy((unsigned)__cvta_generic_to_shared(dst), src);
-}
-
-__global__ void __launch_bounds__(ST, 1) cg_strip_kernel(CgArgs a, const double* in) {
-  __shared__ __align__(16) float xs[2][3][128], xi[2][CT][8];
-  __shared__ double ys[2][CT * 3];
-  extern __shared__ __align__(16) float dyn[];
-  float* cols = dyn;                                   // [2][16][3 x 128]: sums of four rows
-  float4* ring = reinterpret_cast<float4*>(dyn + kColsElems) + threadIdx.x;   // [kStripRing][RW][ST], each lane's own
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n = a.n, per = chunks_before(a.nt);
-  const unsigned act = running(a);
-  const int run = strip_run(a.nt, __popc(act), gridDim.x);
-  int pos = blockIdx.x * run;
-  const int end = min(pos + run, per * __popc(act));
-  if (pos >= end) return;
-  struct At {                               // chunk c of row block I of frequency f
-    int f, I, c;
-  };
-  auto advance = [&](At& w) {
-    if (w.c++ < w.I / 2) return;
-    w.c = 0;
-    if (++w.I < a.nt) return;
-    w.I = 0;
-    w.f = __fns(act, w.f + 1, 1);           // -1 behind the last one, not used
-  };
-  At w;
-  w.f = __fns(act, 0, pos / per + 1);
-  w.I = chunk_row(pos % per);
-  w.c = pos % per - chunks_before(w.I);
-  int c0 = w.c;                             // where this run's piece of the row block begins
-  At pw = w;
-  int ppos = pos, slot = 0;
-  const unsigned ring_at = (unsigned)__cvta_generic_to_shared(ring);
-  // rows past n and columns past the row's end bring some other entry (masked
-  // in a row block's last chunk, times a zero of v, or never read)
-  constexpr int XC = (3 * 128 + ST - 1) / ST, XR = (3 * CT + ST - 1) / ST;
-  double* xring = reinterpret_cast<double*>(dyn + kColsElems + (size_t)kStripRing * CT * 128) + tid;   // each thread's own
-  auto issue_x = [&](double* dst, int f_, int first, int count) {
-    const int left = min(count, 3 * n - first) - tid;   // elements at tid, tid + ST, ...
-    const double* src = in + (size_t)f_ * a.ystride + (left > 0 ? first + tid : 0);
-    for (int u = 0; ST * u < count; ++u)
-      if (tid + ST * u < count) {
-        const bool ok = ST * u < left;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + ST * u);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(ok ? src + ST * u : src), "r"(ok ? 8 : 0) : "memory");
-      }
-  };
-  auto issue = [&](int to) {                // a chunk of the matrix, and v for the one behind it
-    if (ppos < end) {
-      const float* src = a.A32 + (size_t)pw.f * a.a_stride + (size_t)pw.I * CT * a.ld + min(128 * pw.c + 4 * lane, a.ld - 4);
-      const int rmax = n - 1 - pw.I * CT;
-      const unsigned d = ring_at + to * (RW * ST * 16);
-      if (rmax >= CT - 1) {
-        const float* row = src + (size_t)(RW * warp) * a.ld;
-#pragma unroll
-        for (int r = 0; r < RW; ++r) ring_copy(d + r * (ST * 16), row + (size_t)(unsigned)r * a.ld);
-      } else {
-#pragma unroll
-        for (int r = 0; r < RW; ++r)
-          ring_copy(d + r * (ST * 16), src + (size_t)(unsigned)min(RW * warp + r, rmax) * a.ld);
-      }
-      advance(pw);
-      if (++ppos < end) {
-        issue_x(xring + to * kXElems, pw.f, 128 * 3 * pw.c, 3 * 128);
-        if (pw.c == 0) issue_x(xring + to * kXElems + 3 * 128, pw.f, CT * 3 * pw.I, 3 * CT);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int d = 0; d < kStripRing - 1; ++d) issue(d);
-  // v on the chunk's 128 columns and on the row block, the three vectors apart
-  // (element e: vector e % 3 of row e / 3)
-  auto x_at = [&](int f_, int first, int e, int count) {
-    return e < count && first + e < 3 * n ? in[(size_t)f_ * a.ystride + first + e] : 0.0;
-  };
-  auto put_col = [&](int p, int e, double v) {
-    if (e < 3 * 128) xs[p][e % 3][e / 3] = (float)v;
-  };
-  auto put_row = [&](int p, int e, double v) {
-    if (e < 3 * CT) *reinterpret_cast<float2*>(&xi[p][e / 3][2 * (e % 3)]) = make_float2((float)v, (float)v);
-  };
-#pragma unroll
-  for (int u = 0; u < XC; ++u) put_col(0, tid + ST * u, x_at(w.f, 128 * 3 * w.c, tid + ST * u, 3 * 128));
-#pragma unroll
-  for (int u = 0; u < XR; ++u) put_row(0, tid + ST * u, x_at(w.f, CT * 3 * w.I, tid + ST * u, 3 * CT));
-  // the columns of a chunk whose sums all warps have put into cols[p]
-  auto columns = [&](const At& o, int p) {
-    double* pr = a.partial + (size_t)o.f * a.nt * a.nt * CT * 3;
-#pragma unroll
-    for (int u = 0; u < XC; ++u) {
-      const int e = tid + ST * u, q = e / 128, J = 2 * o.c + e % 128 / CT, k = CT * q + e % CT;
-      if (e >= 3 * 128 || J > o.I) continue;
-      double z[4] = {J == o.I ? ys[p][k] : 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int g = 0; g < CT / 4; ++g)   // half of the conversions on either pipe: 2 % of the pass
-        z[g % 4] += g % 2 ? widen(cols[(CT / 4 * p + g) * 3 * 128 + e]) : (double)cols[(CT / 4 * p + g) * 3 * 128 + e];
-      pr[((size_t)J * a.nt + o.I) * CT * 3 + k] = (z[0] + z[1]) + (z[2] + z[3]);
-    }
-  };
-  __syncthreads();
-  double rs[RW][3];
-#pragma unroll
-  for (int r = 0; r < RW; ++r) rs[r][0] = rs[r][1] = rs[r][2] = 0.0;
-  At prev = w;
-  for (int p = 0, ip = 0, first = 1;; p ^= 1, first = 0) {
-    const bool diag = w.c == w.I / 2, more = ++pos < end, same = more && !diag;
-    At nw = w;
-    advance(nw);
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStripRing - 2) : "memory");
-    const float4* mine = ring + slot * RW * ST;
-    const double* xmine = xring + slot * kXElems;
-    issue(slot == 0 ? kStripRing - 1 : slot - 1);      // the slot of the last chunk
-    slot = slot + 1 == kStripRing ? 0 : slot + 1;
-    ulonglong2 xj[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) xj[q] = *reinterpret_cast<const ulonglong2*>(&xs[p][q][4 * lane]);
-    float* co = cols + (CT / 4 * p + RW / 4 * warp) * 3 * 128 + 4 * lane;
-    auto chunk = [&](auto diag_tag) {
-      ulonglong2 cs[3];
-#pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        ulonglong2 e = *reinterpret_cast<const ulonglong2*>(mine + r * ST), ec = e;
-        if constexpr (decltype(diag_tag)::value) {   // nothing above the diagonal, the diagonal on the row side
-          const int d = 128 * w.c + 4 * lane - (w.I * CT + RW * warp + r);
-          float e0, e1, e2, e3;
-          unpack2(e.x, e0, e1);
-          unpack2(e.y, e2, e3);
-          e0 = d <= 0 ? e0 : 0.f, e1 = d <= -1 ? e1 : 0.f, e2 = d <= -2 ? e2 : 0.f, e3 = d <= -3 ? e3 : 0.f;
-          e = make_ulonglong2(pack2(e0, e1), pack2(e2, e3));
-          ec = make_ulonglong2(pack2(d < 0 ? e0 : 0.f, d < -1 ? e1 : 0.f), pack2(d < -2 ? e2 : 0.f, d < -3 ? e3 : 0.f));
-        }
-        const ulonglong2 x01 = *reinterpret_cast<const ulonglong2*>(&xi[ip][RW * warp + r][0]);
-        const unsigned long long x[3] = {x01.x, x01.y, *reinterpret_cast<const unsigned long long*>(&xi[ip][RW * warp + r][4])};
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          float v0, v1;
-          unpack2(fma2(e.y, xj[q].y, mul2(e.x, xj[q].x)), v0, v1);
-          if constexpr (decltype(diag_tag)::value) {   // the diagonal's product is rounded once
-            rs[r][q] += (double)v0 + (double)v1;
-          } else {
-            rs[r][q] += (double)(v0 + v1);
-          }
-          cs[q].x = r % 4 == 0 ? mul2(ec.x, x[q]) : fma2(ec.x, x[q], cs[q].x);
-          cs[q].y = r % 4 == 0 ? mul2(ec.y, x[q]) : fma2(ec.y, x[q], cs[q].y);
-          if (r % 4 == 3) *reinterpret_cast<ulonglong2*>(co + (r / 4 * 3 + q) * 128) = cs[q];
-        }
-      }
-    };
-    if (diag) {
-      chunk(std::true_type());
-    } else {
-      chunk(std::false_type());
-    }
-    if (!first) columns(prev, p ^ 1);
-    if (!same) {
-      // RW rows over 32 lanes: halves exchanged until every lane has one row, then the lanes of a row add up
-      double* pr = a.partial + (size_t)w.f * a.nt * a.nt * CT * 3;
-      constexpr int L = 32 / RW;            // lanes of a row
-      auto fold = [&](auto half) {
-        constexpr int h = decltype(half)::value;
-        const bool up = lane & (L * h);
-#pragma unroll
-        for (int r = 0; r < h; ++r)
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            const double a0 = rs[r][q], a1 = rs[r + h][q];
-            const double got = __shfl_xor_sync(0xffffffffu, up ? a0 : a1, L * h);
-            rs[r][q] = (up ? a1 : a0) + got;
-          }
-      };
-      fold(std::integral_constant<int, 4>());
-      fold(std::integral_constant<int, 2>());
-      fold(std::integral_constant<int, 1>());
-      const int row = RW * warp + lane / L;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        double y = rs[0][q];
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        if (lane % L == 0) {
-          if (diag) {
-            ys[p][CT * q + row] = y;
-          } else {
-            pr[((size_t)w.I * a.nt + 2 * c0) * CT * 3 + CT * q + row] = y;
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < RW; ++r) rs[r][0] = rs[r][1] = rs[r][2] = 0.0;
-      if (more) {
-#pragma unroll
-        for (int u = 0; u < XR; ++u) if (tid + ST * u < 3 * CT) put_row(ip ^ 1, tid + ST * u, xmine[3 * 128 + ST * u]);
-      }
-    }
-    if (more) {
-#pragma unroll
-      for (int u = 0; u < XC; ++u) if (tid + ST * u < 3 * 128) put_col(p ^ 1, tid + ST * u, xmine[ST * u]);
-    }
-    __syncthreads();   // the other copy of each buffer was last read before this barrier
-    if (!more) {
-      columns(w, p);
-      return;
-    }
-    prev = w;
-    if (!same) ip ^= 1, c0 = nw.c;
-    w = nw;
-  }
-}
-
-// Row sums y = (A v) of 64-row block I.  init: R = B - y.  Otherwise Q = y and
-// the block's partial of P^T Q goes to red[f][I].  The partials are those of
-// cg_strip_kernel or of cg_tile_kernel.
-__global__ void __launch_bounds__(192) cg_rows_kernel(CgArgs a, int init, int strips) {
+// Row sums y = (A v) of 64-row block I from the partials that strip_kernel<T>
+// left on `ctas` CTAs.  init: R = B - y.  Otherwise Q = y and the block's
+// partial of P^T Q goes to red[f][I].
+template <typename T>
+__global__ void __launch_bounds__(192) cg_rows_kernel(CgArgs a, int init, int ctas) {
   const int I = blockIdx.x, f = blockIdx.y;
   if (stopped(a, f)) return;
   __shared__ double sm[kRed * 32];
   const int tid = threadIdx.x;
   const int r = tid / 3, q = tid % 3;
   const int gr = I * CT + r;
-  const double* pr = a.partial + (size_t)f * a.nt * a.nt * CT * 3 + (size_t)I * a.nt * CT * 3 + (strips ? CT * q + r : tid);
-  double y = 0.0;
-  if (strips) {   // the CTA count of that launch: the pieces of this row block but the last
-    const unsigned act = running(a);
-    const int run = strip_run(a.nt, __popc(act), strips);
-    const int first = __popc(act & ((1u << f) - 1)) * chunks_before(a.nt) + chunks_before(I), last = first + I / 2;
-    for (int x = first, end; (end = (x / run + 1) * run) <= last; x = end) y += pr[(size_t)(2 * (x - first)) * CT * 3];
-  } else {
-    for (int J = 0; J < I; ++J) y += pr[(size_t)J * CT * 3];
-  }
-  for (int J = I; J < a.nt; ++J) y += pr[(size_t)J * CT * 3];
+  const double y = strip_row_sum<T>(a.partial, a.state, a.batch, a.nt, f, I, ctas, r, q);
   const bool live = gr < a.n;
   const size_t o = (size_t)f * a.ystride + (size_t)gr * 3;
   if (init) {
@@ -830,7 +410,7 @@ __global__ void __launch_bounds__(AT) cg_dir_kernel(CgArgs a, int it) {
 // An entry off the diagonal blocks is read twice (by its row's and its
 // column's owner): matrices of this size stay in L2, and the symmetric sweep
 // tried first spent more on the exchange than on the products.  Sums as in
-// cg_strip_kernel: four products in FP32, everything beyond in FP64.
+// strip_kernel<float>: four products in FP32, everything beyond in FP64.
 // P is kept in shared memory of every CTA in FP32, written by its owners
 // through the cluster.
 constexpr int CLT = 256;
@@ -1240,17 +820,9 @@ int num_sms() {
   return sms;
 }
 
-// CTAs of the grid-stride tile launch: every resident slot of the device.
-int cg_tile_grid() {
-  static int grid = 0;
-  if (grid == 0) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_tile_kernel, TT, 0);
-    grid = (sms > 0 ? sms : 148) * (per_sm > 0 ? per_sm : 1);
-  }
-  return grid;
+template <typename T>
+StripArgs<T> strip_args(const CgArgs& a, const T* A, const double* in) {
+  return StripArgs<T>{A, a.a_stride, a.ld, a.n, a.nt, a.batch, in, a.ystride, a.partial, a.state};
 }
 
 size_t cg_partial_doubles(int n, int batch) {
@@ -1268,7 +840,7 @@ cudaError_t init_cg_attributes() {
   cudaError_t e = cudaFuncSetAttribute(cg_tile_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kTileInvSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(cg_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripSmem);
+  e = init_strip_attributes();
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)p_shared_bytes((kCgClusterMaxN + CT - 1) / CT));
@@ -1297,38 +869,31 @@ cudaError_t launch_cg_cluster(const CgArgs& a, int it0, int it1, int share, cuda
 }
 
 void launch_cg_setup(const CgArgs& a, cudaStream_t s) {
-  const long long items = (long long)a.nt * (a.nt + 1) / 2 * a.batch;
-  const int tgrid = (int)std::min<long long>(cg_tile_grid(), items);
   cudaMemsetAsync(a.state, 0, sizeof(double) * kCgState * a.batch, s);
   cg_tile_inv_kernel<<<dim3(a.nt, a.batch), kTileInvThreads, kTileInvSmem, s>>>(a);
-  cg_tile_kernel<<<tgrid, TT, 0, s>>>(a, a.X);
-  cg_rows_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1, 0);
+  const int ctas = launch_strip(strip_args(a, a.A, a.X), s);
+  cg_rows_kernel<double><<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1, ctas);
   cg_init_tiles_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a);
   cg_init_final_kernel<<<a.batch, 32, 0, s>>>(a, a.nt);
 }
 
 void launch_cg_restart(const CgArgs& a, cudaStream_t s) {
-  const long long items = (long long)a.nt * (a.nt + 1) / 2 * a.batch;
-  const int tgrid = (int)std::min<long long>(cg_tile_grid(), items);
   cg_reopen_kernel<<<(a.batch + 31) / 32, 32, 0, s>>>(a);
-  cg_tile_kernel<<<tgrid, TT, 0, s>>>(a, a.X);
-  cg_rows_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1, 0);
+  const int ctas = launch_strip(strip_args(a, a.A, a.X), s);
+  cg_rows_kernel<double><<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 1, ctas);
   cg_init_tiles_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a);
   cg_init_final_kernel<<<a.batch, 32, 0, s>>>(a, a.nt);
 }
 
 void launch_cg_iteration(const CgArgs& a, int it, cudaStream_t s, bool fp32) {
   const int nb = (a.N + AT - 1) / AT;
-  const long long items = (long long)a.nt * (a.nt + 1) / 2 * a.batch;
-  const int tgrid = (int)std::min<long long>(cg_tile_grid(), items);
-  int strips = 0;
-  if (fp32 && a.A32 && a.batch <= kMaxActive) {
-    strips = std::min(num_sms(), chunks_before(a.nt) * a.batch);
-    cg_strip_kernel<<<strips, ST, kStripSmem, s>>>(a, a.P);
+  if (fp32 && a.A32) {
+    const int ctas = launch_strip(strip_args(a, a.A32, a.P), s);
+    cg_rows_kernel<float><<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 0, ctas);
   } else {
-    cg_tile_kernel<<<tgrid, TT, 0, s>>>(a, a.P);
+    const int ctas = launch_strip(strip_args(a, a.A, a.P), s);
+    cg_rows_kernel<double><<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 0, ctas);
   }
-  cg_rows_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, 0, strips);
   cg_update_kernel<<<dim3(a.nt, a.batch), 192, 0, s>>>(a, it);
   cg_dir_kernel<<<dim3(nb, a.batch), AT, 0, s>>>(a, it);
 }

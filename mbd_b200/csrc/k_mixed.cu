@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#include "strip.cuh"
 #include "tc3.h"
 #include "wait_limit.cuh"
 #include "../../include/mbd_b200.h"
@@ -267,73 +268,22 @@ __global__ void __launch_bounds__(256) bwd_syncfree_kernel(SolveArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Residual R = B - A X, A lower-stored FP64: tile partials, then row sums.
-constexpr int RT = 64;
-
-__device__ __forceinline__ void rt_index(int t, int* ti, int* tj) {
-  int i = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-  while ((i + 1) * (i + 2) / 2 <= t) ++i;
-  while (i * (i + 1) / 2 > t) --i;
-  *ti = i;
-  *tj = t - i * (i + 1) / 2;
-}
+// Residual R = B - A X, A lower-stored FP64: partials (k_strip.cu), then row sums.
+constexpr int RT = kStripRows;
 
 __global__ void axpy_kernel(double* X, const double* D, size_t total) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total) X[i] += D[i];
 }
 
-// One CTA (192 threads) per lower tile (I, J): row partial (rows of I) and
-// column partial (rows of J), each 64 x 3, into partial[b][I][J] / [b][J][I].
-__global__ void __launch_bounds__(192) res_tile_kernel(const double* A64, size_t a_stride, int ld, int n,
-                                                      const double* X, size_t ystride, double* partial, int nt) {
-  __shared__ double Ts[RT][RT + 1];
-  __shared__ double xI[RT][3], xJ[RT][3];
-  int ti, tj;
-  rt_index(blockIdx.x, &ti, &tj);
-  const int b = blockIdx.y;
-  const double* A = A64 + (size_t)b * a_stride;
-  const double* x = X + (size_t)b * ystride;
-  const int tid = threadIdx.x;
-  const bool diag = ti == tj;
-  for (int idx = tid; idx < RT * RT; idx += blockDim.x) {
-    const int r = idx / RT, c = idx % RT;
-    const int gr = ti * RT + r, gc = tj * RT + c;
-    double v = 0.0;
-    if (gr < n && gc < n && (!diag || c <= r)) v = A[(size_t)gr * ld + gc];
-    Ts[r][c] = v;
-  }
-  for (int idx = tid; idx < RT * 3; idx += blockDim.x) {
-    const int r = idx / 3, q = idx % 3;
-    const int gi = ti * RT + r, gj = tj * RT + r;
-    xI[r][q] = gi < n ? x[(size_t)gi * 3 + q] : 0.0;
-    xJ[r][q] = gj < n ? x[(size_t)gj * 3 + q] : 0.0;
-  }
-  __syncthreads();
-  const int r = tid / 3, q = tid % 3;   // 64 x 3
-  double rs = 0.0, cs = 0.0;
-  for (int c = 0; c < RT; ++c) rs += Ts[r][c] * xJ[c][q];                 // row part
-  for (int c = 0; c < RT; ++c)                                             // column part (strict lower on diag)
-    if (!diag || c > r) cs += Ts[c][r] * xI[c][q];
-  double* pr = partial + (size_t)b * nt * nt * RT * 3;
-  if (!diag) {
-    pr[((size_t)ti * nt + tj) * RT * 3 + tid] = rs;
-    pr[((size_t)tj * nt + ti) * RT * 3 + tid] = cs;
-  } else {
-    pr[((size_t)ti * nt + ti) * RT * 3 + tid] = rs + cs;
-  }
-}
-
-// R[row] = B[row] - sum_J partial[b][I][J][row]; per-block squared norms.
+// R[row] = B[row] - (A X)[row]; per-block squared norms.
 __global__ void __launch_bounds__(192) res_reduce_kernel(const double* partial, int nt, int n, double* R,
-                                                        size_t ystride, double* normpart) {
+                                                        size_t ystride, double* normpart, int ctas) {
   const int I = blockIdx.x, b = blockIdx.y;
   const int tid = threadIdx.x;
   const int r = tid / 3, q = tid % 3;
   const int gr = I * RT + r;
-  const double* pr = partial + (size_t)b * nt * nt * RT * 3 + (size_t)I * nt * RT * 3 + tid;
-  double y = 0.0;
-  for (int J = 0; J < nt; ++J) y += pr[(size_t)J * RT * 3];
+  const double y = strip_row_sum<double>(partial, nullptr, gridDim.y, nt, b, I, ctas, r, q);
   double res = 0.0;
   if (gr < n) {
     res = ((gr % 3) == q ? 1.0 : 0.0) - y;
@@ -397,9 +347,9 @@ void launch_relay_residual(const double* A64, size_t a_stride, int ld, int n, in
     const size_t total = (size_t)batch * ystride;
     axpy_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(X, D, total);
   }
-  res_tile_kernel<<<dim3(nt * (nt + 1) / 2, batch), 192, 0, s>>>(A64, a_stride, ld, n, X, ystride, partial, nt);
+  const int ctas = launch_strip(StripArgs<double>{A64, a_stride, ld, n, nt, batch, X, ystride, partial, nullptr}, s);
   double* normpart = partial + (size_t)batch * nt * nt * RT * 3;
-  res_reduce_kernel<<<dim3(nt, batch), 192, 0, s>>>(partial, nt, n, R, ystride, normpart);
+  res_reduce_kernel<<<dim3(nt, batch), 192, 0, s>>>(partial, nt, n, R, ystride, normpart, ctas);
   norm_final_kernel<<<batch, 32, 0, s>>>(normpart, nt, rnorm2);
 }
 
