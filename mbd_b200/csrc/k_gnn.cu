@@ -209,37 +209,27 @@ __global__ void sa_kernel(const float* P, const float* h, int M, float* s, float
   }
 }
 
-// Sum over the 8 lanes of a node.
-__device__ __forceinline__ float sum8(float v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  return v + __shfl_xor_sync(0xffffffffu, v, 4);
-}
-
-// S (row-major 3x3) per node; 8 lanes share a node's edges
+// S (row-major 3x3) per node, one of its six sums per lane of eight: every sum
+// runs over the edges in their order, so that the prediction keeps its bits
+// (eight lanes that split the edges and add up took as long).
 __global__ void tensor_kernel(const float* s, const float* a, const float* g, const float* eproj, const int* off,
                               const int* nbr, int N, int F, float* S) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x, node = idx >> 3, sub = idx & 7;
-  const bool live = node < N * F;
-  const int f = live ? node / N : 0, i = live ? node % N : 0;
-  float p[6] = {0, 0, 0, 0, 0, 0};
-  if (live)
-    for (int e = off[i] + sub; e < off[i + 1]; e += 8) {
-      const float w = a[(size_t)f * N + nbr[e]] * g[e];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) p[c] += w * eproj[(size_t)e * 6 + c];
-    }
-#pragma unroll
-  for (int c = 0; c < 6; ++c) p[c] = sum8(p[c]);
-  if (!live || sub != 0) return;
-  const float d = 1.0f + s[node];
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, node = idx >> 3, c = idx & 7;
+  if (node >= N * F || c >= 6) return;
+  const int f = node / N, i = node % N;
+  float p = 0.f;
+#pragma unroll 4
+  for (int e = off[i]; e < off[i + 1]; ++e) {
+    const float w = a[(size_t)f * N + nbr[e]] * g[e];
+    p += w * eproj[(size_t)e * 6 + c];
+  }
   float* o = S + (size_t)node * 9;
-  o[0] = d + p[0];
-  o[4] = d + p[1];
-  o[8] = d + p[2];
-  o[1] = o[3] = p[3];
-  o[2] = o[6] = p[4];
-  o[5] = o[7] = p[5];
+  if (c < 3) {
+    o[4 * c] = (1.0f + s[node]) + p;
+  } else {   // xy, xz, yz
+    const int k = c == 5 ? 5 : c - 2;
+    o[k] = o[c == 3 ? 3 : (c == 4 ? 6 : 7)] = p;
+  }
 }
 
 // dS = 2 (S - S_true) / M; loss += ||S - S_true||^2 / M
@@ -277,15 +267,23 @@ __global__ void readout_bwd_kernel(const float* dS, const float* a, const float*
   const bool live = node < N * F;
   const int f = live ? node / N : 0, i = live ? node % N : 0;
   const float* dSi = dS + (size_t)(live ? node : 0) * 9;
+  const int e0 = live ? off[i] : 0, e1 = live ? off[i + 1] : 0;
+  const int rounds = __reduce_max_sync(0xffffffffu, (e1 - e0 + 7) / 8);
   float acc = 0.f;
-  if (live)
-    for (int e = off[i] + sub; e < off[i + 1]; e += 8) {
+  for (int r = 0; r < rounds; ++r) {
+    const int e = e0 + 8 * r + sub;
+    float t = 0.f, ge = 0.f;
+    if (e < e1) {
       const int j = f * N + nbr[e];
       const float* pe = eproj + (size_t)e * 6;
-      acc += g[e] * dot_proj(dS + (size_t)j * 9, pe);
+      ge = g[e];
+      t = dot_proj(dS + (size_t)j * 9, pe);
       cw[(size_t)f * E + e] = dot_proj(dSi, pe) * a[j];
     }
-  acc = sum8(acc);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)   // in the order of the edges; zeros behind the last
+      acc += __shfl_sync(0xffffffffu, ge, u, 8) * __shfl_sync(0xffffffffu, t, u, 8);
+  }
   if (!live || sub != 0) return;
   ds[node] = dSi[0] + dSi[4] + dSi[8];
   da[node] = acc;
