@@ -81,7 +81,7 @@ typedef struct {
     int nimag;                    /* number of negative CFDM eigenvalues, UTILS.f90:850-863 */
     int status;                   /* MBD_OK or an error code for this geometry */
     int supercell[3];             /* supercell multiplicities, UTILS.f90:1252-1283 */
-    int refine_iters;             /* mixed modes: refinement / CG iterations taken (max over freqs) */
+    int refine_iters;             /* mixed modes: refinement sweeps (1: FP64 factors) / CG iterations taken (max over freqs) */
     double err_est[3];            /* [0] max relative relay residual ||b-Ax||/||b|| over freqs (FP64),
                                      [1] estimated relative error of alpha_eff,
                                      [2] estimated relative error of C6 */
