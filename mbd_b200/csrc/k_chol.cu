@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) trsv_bwd_kernel(BatchMat m, int k0, const
 // block, the exchange and the product with the inverse.  Bound by that chain
 // (2 ceil(n/64) steps) and, for large n, by reading L twice.
 constexpr int kTrsvThreads = 256;
-constexpr int kTrsvMaxC = 8;
+constexpr int kTrsvMaxC = 4;
 
 __device__ __forceinline__ double quad_sum(double v) {
   v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -395,7 +395,11 @@ cudaError_t init_trsv_attributes() {
 cudaError_t launch_trsv_cluster(const BatchMat& m, const double* Linv, size_t linv_stride, double* X, size_t ystride,
                                 cudaStream_t s) {
   const int T = (m.n + NB - 1) / NB;
-  const int C = T <= 2 ? 1 : (T <= 6 ? 2 : (T <= 16 || m.n > 3100 ? 4 : 8));
+  // Solve of one cluster (ms) with 1, 2, 4 and 8 CTAs a frequency: n = 126 0.031,
+  // 0.031, 0.031, 0.035; 384 0.055, 0.051, 0.049, 0.059 (two leave more room for
+  // other geometries); 999 0.24, 0.17, 0.14, 0.15; 3000 1.96, 1.12, 0.71, 0.72; 6000
+  // 6.9, 3.8, 2.2, 2.6 (eight: fewer clusters at once, a longer exchange).
+  const int C = T <= 2 ? 1 : (T <= 6 ? 2 : 4);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(m.batch * C);
   cfg.blockDim = dim3(kTrsvThreads);

@@ -328,7 +328,7 @@ void launch_cg_iteration(const CgArgs& a, int it, cudaStream_t s, bool fp32 = fa
 // Iterations [it0, it1) of an FP32-pass phase in one launch, for n <= kCgClusterMaxN
 // (state as launch_cg_iteration leaves it, but for the Z^T R slots).  Relay
 // solve of one cluster, four launches an iteration against this (ms): N = 61
-// 0.54 / 0.41, 200 0.84 / 0.68, 500 2.02 / 1.83, 680 2.76 / 2.26; beyond, a
+// 0.44 / 0.30, 200 0.77 / 0.56, 500 1.63 / 1.66, 680 2.05 / 1.97; beyond, a
 // cluster per frequency leaves too much of the device idle once most
 // frequencies have converged.
 constexpr int kCgClusterMaxN = 2048;
