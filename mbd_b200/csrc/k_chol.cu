@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kTrsvThreads) trsv_cluster_kernel(BatchMat m, 
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int b = blockIdx.x / C;
   extern __shared__ __align__(16) double sh[];
+  cl.barrier_arrive();                              // the cluster's CTAs have started: waited for before the first push
   const int n = m.n, T = (n + NB - 1) / NB, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* Z = sh;                                   // [T * 64][3]: z, overwritten by x
   double* buf = Z + (size_t)T * NB * 3;             // [2][C][192]: the CTAs' partial sums
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(kTrsvThreads) trsv_cluster_kernel(BatchMat m, 
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const double2*>(src + 8 * u);
   };
+  cl.barrier_wait();
   for (int k = 0; k < T; ++k) {
     a0 = quad_sum(a0);
     a1 = quad_sum(a1);

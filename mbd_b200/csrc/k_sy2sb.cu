@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(NW * 32) qr_panel_kernel(PanelArgs a) {
   __shared__ double gs[B];
   __shared__ double Tm[B][B + 1];
   cg::cluster_group cl = cg::this_cluster();
+  cluster_arrive();   // the cluster's CTAs have started: waited for before the first remote store
   // T[0:jc, jc] = -tau_jc T[0:jc, 0:jc] (V^T V)[0:jc, jc], T[jc][jc] = tau_jc
   // (dlarft, forward, columnwise) from column jc's dots dcj (rank 0, warp 0)
   int jprev = -1;
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(NW * 32) qr_panel_kernel(PanelArgs a) {
       if (t == tj) v = x[t];
     return v;
   };
+  cluster_wait();
   // column 0: exact norm and alpha (rank 0, warp 0 owns row 0)
   if (rank == 0 && warp == 0) {
     const double a0 = __shfl_sync(FULL, own_entry(0), 0);
@@ -327,6 +329,7 @@ __global__ void __launch_bounds__(NW * 32) qr_panel2_kernel(PanelArgs a) {
   __shared__ double gs[B];
   __shared__ double Tm[B][B + 1];
   cg::cluster_group cl = cg::this_cluster();
+  cluster_arrive();   // the cluster's CTAs have started: waited for before the first remote store
   // T[0:jc, jc] = -tau_jc T[0:jc, 0:jc] (V^T V)[0:jc, jc], T[jc][jc] = tau_jc
   // (dlarft, forward, columnwise) from column jc's dots dcj (rank 0, warp 0)
   int jprev = -1;
@@ -380,6 +383,7 @@ __global__ void __launch_bounds__(NW * 32) qr_panel2_kernel(PanelArgs a) {
       }
     s_own = s0 + s1;
   }
+  cluster_wait();
   for (int j = 0; j < nref; ++j) {
     const int par = j & 1;
     const double sj = __shfl_sync(FULL, s_own, j);

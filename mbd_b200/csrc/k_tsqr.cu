@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(NT) tsqr_panel_kernel(PanelArgs a) {
   __shared__ double gs[B];
   __shared__ double s_alpha;
   cg::cluster_group cl = cg::this_cluster();
+  cl.barrier_arrive();   // the cluster's CTAs have started: waited for before the first remote store
   const int rank = (int)cl.block_rank();
   const int C = (int)cl.num_blocks();
   const int m = a.m;
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(NT) tsqr_panel_kernel(PanelArgs a) {
   // ---- 1. local Householder QR
   for (int j = 0; j < B; ++j) house_step<RPW>(x, j, nr, nw, &s_alpha, dw, gs, Tl);
   __syncthreads();
+  cl.barrier_wait();
   // local R (rows 0..31) to rank 0; local V rows 0..31 kept for step 3
   double* Rdst = cl.map_shared_rank(Rs, 0) + (size_t)rank * B * LDT;
 #pragma unroll
