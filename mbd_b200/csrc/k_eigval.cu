@@ -204,6 +204,7 @@ __device__ __forceinline__ void energy_block(const double* ev, int n, int nsl, c
     out[0] = (0.5 * e_int) / nsl - (0.5 * e_nonint);     // UTILS.f90:858
     out[1] = e_int;
     out[2] = (double)sn[0];
+    out[3] = kTraceOk;   // where a trace form was refused: that is made good, the Hamiltonian is spent
   }
 }
 

@@ -200,6 +200,7 @@ constexpr int kWyNB = 128;
 cudaError_t init_eigvec_attributes();
 void launch_wy_t(const double* S, const double* tau, int n_refl, double* T, cudaStream_t s);
 // energy = 0.5*sum_{ev>=0} sqrt(ev)/nsl - 0.5*sum_nonint; out[0]=E, out[1]=sum sqrt, out[2]=nimag
+// out[3]=kTraceOk: the energy stands, whatever a trace form left there before
 void launch_energy(const double* ev, int n, int nsl, const double* scalars, double* out,
                    cudaStream_t s);
 // ---- two-stage tridiagonalisation (PDSYEV('N','L') reduction, UTILS.f90:835) ----
@@ -289,7 +290,8 @@ struct TraceArgs {
   double* linv;            // kTraceBatch * ceil(n/64) blocks of 64 x 64
   void* ws;                // trace_ws_bytes(n)
   const double* scalars;   // relay scalars ([1] = sum of 3 omega)
-  double* out;             // energy outputs: [0] E, [1] sum sqrt, [2] 0 negative, [3] kTraceOk or kTraceRefused
+  double* out;             // energy outputs: [0] E, [1] sum sqrt, [2] 0 negative, [3] kTraceOk or kTraceRefused (the
+                           // eigenvalue energy that then takes its place makes it kTraceOk)
   int* err;
 };
 constexpr double kTraceOk = 1.0, kTraceRefused = 2.0;
