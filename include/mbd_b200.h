@@ -236,7 +236,10 @@ void* mbd_rsscs_stream(mbd_ctx* ctx);
  *                            its first sweep wait for a count that no sweep
  *                            reaches, so that its bounded wait runs out and the
  *                            compute reports MBD_ERR_TIMEOUT; the context stays
- *                            usable.  For testing failure detection; 0 (the
+ *                            usable.  2: the Cholesky launches make the tiles
+ *                            of their first block column wait for a diagonal
+ *                            block that never comes (matrices of more than 64
+ *                            rows).  For testing failure detection; 0 (the
  *                            default) turns it off.
  *   MBD_OPT_FP32_TENSOR_BUILD 1: MIXED and MIXED_LEARNED build the short-range
  *                            dipole tensors of the relay matrices in FP32

@@ -259,6 +259,7 @@ int relay_direct(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, double* L, cudaEvent_
   cf.info = gd->info;
   cf.sync = sl.chol_sync.as<int>();
   cf.err = ctx->err_flag;
+  cf.stall = ctx->test_stall_wait == kStallFactor;
   MBD_CUDA(launch_chol_flow(cf, ctx->num_sms, s));
   ctx->launches += 1;
   record_timing(ctx, ev_factor, s);
@@ -439,7 +440,7 @@ void drop_graphs(mbd_ctx* ctx, bool keep_first) {
 }
 
 int band_to_tridiag_single(mbd_ctx* ctx, double* Br, int n, double* d, double* e, DevBuf& scratch, cudaStream_t s) {
-  const int C = (ctx->cluster_chase && !ctx->test_stall_wait && n <= sb2st_cluster_max_n() &&
+  const int C = (ctx->cluster_chase && ctx->test_stall_wait != kStallChase && n <= sb2st_cluster_max_n() &&
                  tuned_chase_c(ctx, n) != kChaseFlag)
                     ? sb2st_cluster_size(n, 1, ctx->num_sms, tuned_chase_c(ctx, n)) : 0;
   if (C > 0) {
@@ -541,7 +542,7 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   // the two-stage tridiagonalisation)
   if (gd->trace) {
     TraceArgs ta{gd->hmat, p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
-                 sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag};
+                 sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag, ctx->test_stall_wait == kStallFactor};
     MBD_CUDA(launch_trace_energy(ta, ctx->num_sms, s));
     ctx->launches += trace_launches(p.nH);
   } else if (two_stage(ctx, p.nH)) {
@@ -643,7 +644,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
   // Energies as traces: not while an eigenvalue kernel is asked for (its
   // environment switches, the stalled chase of the failure tests)
   for (auto& gd : ctx->geoms) gd->trace = false;
-  if (eigen && ctx->trace_form && !ctx->test_stall_wait)
+  if (eigen && ctx->trace_form && ctx->test_stall_wait != kStallChase)
     for (int g : ctx->order) ctx->geoms[g]->trace = ctx->geoms[g]->plan.nH <= kTraceMaxN;
   // A batch whose buffers are all there already (a program's second call of a
   // size) does not ask how much memory is free: that query goes through the
@@ -859,7 +860,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
   int big = 0;
   for (int g : ctx->order)
     if (banded(g)) big = std::max(big, ctx->geoms[g]->plan.nH);
-  const bool cluster_ok = ctx->cluster_chase && !ctx->test_stall_wait && big > 0 &&
+  const bool cluster_ok = ctx->cluster_chase && ctx->test_stall_wait != kStallChase && big > 0 &&
                           big <= sb2st_cluster_max_n() && tuned_chase_c(ctx, big) != kChaseFlag;
   const int cap = cluster_ok ? sb2st_cluster_max_n() : 0;
   ctx->band_max_n = ctx->band_cluster_max_n = 0;
@@ -1019,7 +1020,7 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
   if (ctx->n_band_jobs > ctx->n_band_cluster) {
     MBD_CUDA(launch_sb2st(ctx->band_jobs + ctx->n_band_cluster, ctx->n_band_jobs - ctx->n_band_cluster,
                           ctx->sweep_items, ctx->n_sweep_items, ctx->sweep_progress.as<int>(), ctx->err_flag,
-                          ctx->num_sms, ctx->band_max_n, ctx->sweeps_in_flight, ctx->test_stall_wait ? 0 : -1, s));
+                          ctx->num_sms, ctx->band_max_n, ctx->sweeps_in_flight, ctx->test_stall_wait == kStallChase ? 0 : -1, s));
     ctx->launches += 3;
   }
   record_timing(ctx, bev[2], s);
@@ -1389,7 +1390,9 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
         if (st == MBD_OK && !gd->trace) st = run_tail_single(ctx, gd, ctx->slots[gd->slot]->stream);
         if (st != MBD_OK) return st;
         const cudaStream_t ss = ctx->slots[gd->slot]->stream;
-        MBD_CUDA(fetch_one(gd, ss));   // the re-run's results replace the staged ones
+        // the re-run's results replace the staged ones; its waits may have run out
+        MBD_CUDA(cudaMemcpyAsync(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ss));
+        MBD_CUDA(fetch_one(gd, ss));
         MBD_CUDA(cudaStreamSynchronize(ss));
         r.refine_iters = -1;
       }
@@ -1415,11 +1418,10 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
     const double* scal = reinterpret_cast<const double*>(host(gd->scalars));
     const double* en = reinterpret_cast<const double*>(host(gd->energy));
     const int* info = reinterpret_cast<const int*>(host(gd->info));
-    int status = MBD_OK;
+    int status = err;   // first: what unfinished factors say of the matrix means nothing
     for (int f = 0; f < 21; ++f)
-      if (info[f] != 0) status = MBD_ERR_RELAY_NOT_SPD;
+      if (status == MBD_OK && info[f] != 0) status = MBD_ERR_RELAY_NOT_SPD;
     if (status == MBD_OK && scal[2] > 0.0) status = MBD_ERR_NONPOSITIVE_ALPHA;
-    if (status == MBD_OK && err != 0) status = err;
     r.status = status;
     r.c6_mol = scal[0];
     if (status == MBD_OK) {
@@ -1725,7 +1727,7 @@ int mbd_rsscs_set_option(mbd_ctx* ctx, int option, double value) {
       return MBD_OK;
     }
     case MBD_OPT_TEST_STALL_WAIT: {
-      const int on = value != 0.0;
+      const int on = value == kStallFactor ? kStallFactor : (value != 0.0 ? kStallChase : 0);
       if (on != ctx->test_stall_wait) {
         MBD_CUDA(cudaSetDevice(ctx->device));
         MBD_CUDA(cudaDeviceSynchronize());

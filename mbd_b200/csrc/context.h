@@ -31,6 +31,8 @@ struct NvtxRange {
 // ||B - A X||_F / ||B||_F that accepts its result.
 constexpr int kRefineIters = 4;
 constexpr double kResidualGate = 1e-10;
+// MBD_OPT_TEST_STALL_WAIT: which launches have a wait that nothing ends.
+constexpr int kStallChase = 1, kStallFactor = 2;
 // Relay slots (streams with private relay workspaces) of one context.
 constexpr int kMaxSlots = 8;
 // Share of free device memory the relay slots of one batch may plan for.
@@ -256,7 +258,7 @@ struct mbd_ctx {
   // options (mbd_rsscs_set_option)
   double residual_gate = mbd::kResidualGate;   // accepted ||B - A X||_F / ||B||_F of the fast relay solves
   double wait_limit_s = 2.0;                   // bounded device waits (per device)
-  int test_stall_wait = 0;                     // 1: the bulge-chasing launch's first wait runs out
+  int test_stall_wait = 0;                     // kStallChase or kStallFactor: a wait of that launch runs out
   int f32_tensor_build = 0;                    // 1: mixed modes build the relay tensors in FP32 arithmetic
   bool cg_fp32 = false;                        // learned mode: block-CG matrix passes on the FP32 copy (this batch)
   int cg_fp32_mode = -1;                       // 1 always, 0 never, -1 where the copy fits (reserve_learned)

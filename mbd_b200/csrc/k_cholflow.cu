@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
       run(std::integral_constant<int, 2>());
     }
     if (!early) {
-      if (tid == 0) wait_count(diag + b, k + 1, a.err);
+      if (tid == 0) wait_count(diag + b, a.stall && k == 0 ? 1 << 30 : k + 1, a.err);
       __syncthreads();
       copy_inverse(n_chunks);
       copy_inverse(n_chunks + 1);

@@ -480,6 +480,7 @@ cudaError_t launch_trace_energy(const TraceArgs& a, int num_sms, cudaStream_t s)
   f.info = w.info;
   f.sync = w.sync;
   f.err = a.err;
+  f.stall = a.stall;
   cudaError_t e = launch_chol_flow(f, num_sms, s);
   if (e != cudaSuccess) return e;
   trace_energy_kernel<<<1, 32, 0, s>>>(w, a.n, T, a.nsl, a.scalars, a.out);

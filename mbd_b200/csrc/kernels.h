@@ -93,6 +93,7 @@ struct CholFlowArgs {
   int* info;               // [batch]: first failing column + 1 where a pivot is not positive; zeroed by the caller
   int* sync;               // chol_flow_sync_ints(n, batch) ints
   int* err;                // the context's error flag (a wait that ran out)
+  bool stall;              // tests: the first tiles wait for a diagonal block that never comes
 };
 constexpr int kCholFlowHead = 32;
 size_t chol_flow_sync_ints(int n, int batch);
@@ -293,6 +294,7 @@ struct TraceArgs {
   double* out;             // energy outputs: [0] E, [1] sum sqrt, [2] 0 negative, [3] kTraceOk or kTraceRefused (the
                            // eigenvalue energy that then takes its place makes it kTraceOk)
   int* err;
+  bool stall;              // CholFlowArgs::stall
 };
 constexpr double kTraceOk = 1.0, kTraceRefused = 2.0;
 size_t trace_ws_bytes(int n);
