@@ -425,6 +425,10 @@ int mbd_rsscs_learned_train(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms, int
   }
   MBD_CUDA(cudaDeviceSynchronize());
   {
+    // a wait of the factors that ran out has left targets of unfinished factors
+    int err = 0;
+    MBD_CUDA(cudaMemcpy(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost));
+    if (err) return err;
     int info_bad = 0;
     for (int g : ctx->order) {
       int info[32];

@@ -1,7 +1,8 @@
 """Waits of the Cholesky launches that run out (from the host: the first tiles
 wait for a diagonal block that never comes, 50 ms limit) end with
-MBD_ERR_TIMEOUT wherever these launches run: a plain compute and the FP64 re-run
-of a solve that missed the residual gate.  The context then works again."""
+MBD_ERR_TIMEOUT wherever these launches run: a plain compute, the FP64 re-run of
+a solve that missed the residual gate, the labels of a training.  The context
+then works again."""
 import numpy as np
 import pytest
 
@@ -63,3 +64,14 @@ def test_rerun_after_a_missed_gate(engine, mode):
     code, res = engine.download()
     assert code == 0 and all(r.refine_iters == -1 for r in res)
     _same(res, refs)
+
+
+def test_training_labels(engine):
+    from mbd_b200 import MbdError
+    items = _items()
+    engine.set_option("test_stall_wait", 2)
+    with pytest.raises(MbdError) as e:
+        engine.learned_train(*_split(items), epochs=1)
+    assert e.value.code == MBD_ERR_TIMEOUT
+    engine.set_option("test_stall_wait", 0)
+    assert np.isfinite(engine.learned_train(*_split(items), epochs=1)).all()
