@@ -1364,7 +1364,10 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
       // with the direct FP64 solve (the plain path) before reading results
       const double* rn = reinterpret_cast<const double*>(host(gd->rnorm2));
       double worst = 0.0;
-      for (int f = 0; f < 21; ++f) worst = std::max(worst, std::sqrt(rn[f] / (3.0 * N)));
+      for (int f = 0; f < 21; ++f) {
+        const double v = std::sqrt(rn[f] / (3.0 * N));
+        worst = std::isfinite(v) ? std::max(worst, v) : std::numeric_limits<double>::infinity();
+      }
       r.err_est[0] = r.err_est[1] = r.err_est[2] = worst;
       r.refine_iters = mixed_direct(*gd, *ctx->slots[gd->slot]) ? 1 : kRefineIters;
       if (ctx->last_mode == MBD_MODE_MIXED_LEARNED) {
