@@ -695,6 +695,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
     }
   }
   for (int g : ctx->order) ctx->geoms[g]->slot = slot_of[g];
+  for (auto& sl : ctx->slots) sl->mixed_direct = true;
   while ((int)ctx->slots.size() < S) {
     std::unique_ptr<RelaySlot> sl(new RelaySlot());
     // slot 0 takes the batch's largest geometry (longest first), whose
@@ -958,9 +959,8 @@ int reserve_mixed(mbd_ctx* ctx) {
       if (e == cudaSuccess) e = grow(sl.solve_sync, sync);
       return e;
     };
-    sl.mixed_direct = true;
     cudaError_t e = reserve();
-    if (e == cudaErrorMemoryAllocation) {
+    if (e == cudaErrorMemoryAllocation && sl.mixed_direct) {   // stays so until the slots are planned again
       cudaGetLastError();
       sl.mixed_direct = false;
       e = reserve();
