@@ -629,7 +629,9 @@ size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, siz
 
 // Assigns the geometries to relay slots (longest first onto the least loaded
 // slot, load = (3N)^3), with as many slots as fit in the device memory share.
-int plan_slots(mbd_ctx* ctx, bool eigen) {
+// tight: memory ran out under a plan made without asking how much is free;
+// asks, and gives back the slots that the new plan does without.
+int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
   const int ng = (int)ctx->order.size();
   int S = std::max(1, std::min(kMaxSlots, ng));
   std::vector<int> slot_of(ctx->geoms.size(), 0);
@@ -650,7 +652,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
   // size) does not ask how much memory is free: that query goes through the
   // driver's kernel part, 0.05 to 2 ms depending on what else the host runs.
   deal(S);
-  bool held = (int)ctx->slots.size() >= S;
+  bool held = !tight && (int)ctx->slots.size() >= S;
   for (int g : ctx->order) {
     if (!held) break;
     const GeomDev& gd = *ctx->geoms[g];
@@ -694,7 +696,9 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
       if (total <= budget || S == 1) break;
     }
   }
+  ctx->slots_unasked = held;
   for (int g : ctx->order) ctx->geoms[g]->slot = slot_of[g];
+  while (tight && (int)ctx->slots.size() > S) ctx->slots.pop_back();
   for (auto& sl : ctx->slots) sl->mixed_direct = true;
   while ((int)ctx->slots.size() < S) {
     std::unique_ptr<RelaySlot> sl(new RelaySlot());
@@ -716,7 +720,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen) {
 
 // Plain-path slot buffers, per-geometry Hamiltonians, the tridiagonal plan and
 // the device job tables of the uploaded batch.
-int prepare_batch(mbd_ctx* ctx, bool eigen) {
+int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
   drop_graphs(ctx, true);
   ctx->order.clear();
   for (size_t g = 0; g < ctx->geoms.size(); ++g)
@@ -753,7 +757,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen) {
     ctx->n_trd_groups = ctx->trd_total_ctas = ctx->n_eig_jobs = ctx->n_eig_batch = 0;
     return MBD_OK;
   }
-  int st = plan_slots(ctx, eigen);
+  int st = plan_slots(ctx, eigen, tight);
   if (st != MBD_OK) return st;
   // geometries whose energy comes from eigenvalues, by the two-stage reduction
   auto banded = [&](int g) {
@@ -1263,13 +1267,17 @@ int mbd_rsscs_compute(mbd_ctx* ctx, int mode) {
   if (mode != MBD_MODE_PLAIN_FP64 && mode != MBD_MODE_MIXED && mode != MBD_MODE_MIXED_LEARNED) return MBD_ERR_ARG;
   if (mode == MBD_MODE_MIXED_LEARNED && ctx->use_net && !ctx->have_net) return MBD_ERR_NO_NETWORK;
   MBD_CUDA(cudaSetDevice(ctx->device));
-  if (mode == MBD_MODE_MIXED) {
-    int st = reserve_mixed(ctx);
-    if (st != MBD_OK) return st;
-  } else if (mode == MBD_MODE_MIXED_LEARNED) {
-    int st = reserve_learned(ctx);
-    if (st != MBD_OK) return st;
+  auto reserve = [&] {
+    return mode == MBD_MODE_MIXED ? reserve_mixed(ctx) : (mode == MBD_MODE_MIXED_LEARNED ? reserve_learned(ctx) : MBD_OK);
+  };
+  int st = reserve();
+  if (st == MBD_ERR_OUT_OF_MEMORY && ctx->slots_unasked) {   // fewer slots, for what memory there is
+    cudaGetLastError();
+    MBD_CUDA(cudaDeviceSynchronize());
+    st = prepare_batch(ctx, true, true);
+    if (st == MBD_OK) st = reserve();
   }
+  if (st != MBD_OK) return st;
   ctx->last_mode = mode;
   // From the second compute of a batch in a mode on, capture the batch into a
   // CUDA graph once and replay it; a batch computed once (energy_batch, an

@@ -168,6 +168,7 @@ struct mbd_ctx {
   std::vector<std::unique_ptr<mbd::GeomDev>> geoms;
   std::vector<std::unique_ptr<mbd::RelaySlot>> slots;
   int n_slots = 0;                           // slots in use for the current batch
+  bool slots_unasked = false;                // planned without asking how much memory is free (plan_slots)
   mbd::DevBuf tridiag_ws, tables, misc, fb_ws;
   mbd::DevBuf fb_band, fb_trd;   // a refused trace form's reduction (never part of a graph)
   mbd::DevBuf inputs, results, hmats;   // the batch's geometries: inputs; results (first what goes back); Hamiltonians

@@ -1,6 +1,7 @@
 """Mixed solves when device memory is short (a torch allocation takes the rest
 of it; nothing faults, allocations fail): the FP64 factors that do not fit are
-tried once per upload, not once per compute."""
+tried once per upload, not once per compute, and a batch whose slots were
+planned while there was room is planned again with fewer."""
 import numpy as np
 import pytest
 
@@ -54,3 +55,16 @@ def test_factors_that_do_not_fit_are_tried_once():
         code, res = eng.download()
         assert code == 0 and res[0].refine_iters == 1
         _check(res, [ref])
+
+
+def test_fewer_slots_when_memory_ran_out():
+    from mbd_b200 import Engine
+    from mbd_b200 import synthetic as sy
+    items = [sy.cluster(300, seed=40 + k) for k in range(8)]             # 140 MB of matrices each, as much for the factors
+    geos, sts = [g for g, _ in items], [s for _, s in items]
+    with Engine(0) as eng:
+        eng.energy(*sy.cluster(30, seed=1), "mixed")
+        refs = eng.energy_batch(geos, sts, "plain")
+        with _OnlyLeft(300 * MB):
+            _check(eng.energy_batch(geos, sts, "mixed"), refs)
+        _check(eng.energy_batch(geos, sts, "mixed"), refs)
