@@ -557,39 +557,6 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
 
 namespace {
 
-// Eigen stages of one geometry on stream s with its own launches: the
-// residual-gate fallback of download (run_front has reduced a two-stage
-// geometry's Hamiltonian to its band already), and a refused trace form.
-int run_tail_single(mbd_ctx* ctx, GeomDev* gd, cudaStream_t s) {
-  const GeomPlan& p = gd->plan;
-  if (two_stage(ctx, p.nH)) {
-    double* band = gd->band.as<double>();
-    if (gd->trace) {   // refused: the Hamiltonian is still whole
-      MBD_CUDA(ctx->fb_band.reserve(sizeof(double) * (size_t)p.nH * kBandLd));
-      MBD_CUDA(ctx->fb_trd.reserve(sizeof(double) * sy2sb_workspace_doubles(p.nH)));
-      band = ctx->fb_band.as<double>();
-      MBD_CUDA(launch_sy2sb(gd->hmat, p.ldH, p.nH, ctx->fb_trd.as<double>(), band, ctx->num_sms, s,
-                            tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH),
-                            lookahead_for(ctx, ctx->slots[gd->slot]->la)));
-      ctx->launches += sy2sb_launches(p.nH);
-    }
-    int st = band_to_tridiag_single(ctx, band, p.nH, gd->d, gd->e, ctx->fb_ws, s);
-    if (st != MBD_OK) return st;
-  } else {
-    TridiagJob job{gd->hmat, p.nH, p.ldH, gd->d, gd->e};
-    MBD_CUDA(cudaMemcpyAsync(ctx->job_dev, &job, sizeof(job), cudaMemcpyHostToDevice, s));
-    const int G = tridiag_group_ctas(ctx, p.nH);
-    const size_t wsb = tridiag_workspace_bytes(p.nH, G);
-    MBD_CUDA(ctx->fb_ws.reserve(wsb));
-    MBD_CUDA(launch_tridiag(ctx->job_dev, 1, 1, G, ctx->fb_ws.p, wsb, p.nH, ctx->err_flag, s));
-    ctx->launches += 1;
-  }
-  launch_tridiag_eigenvalues(gd->d, gd->e, p.nH, gd->ev, s);
-  launch_energy(gd->ev, p.nH, p.nsl, gd->scalars, gd->energy, s);
-  ctx->launches += 2;
-  return cuda_status(cudaGetLastError());
-}
-
 // ---- workspaces and the batch plan ----------------------------------------
 
 size_t plain_bytes(const GeomPlan& p, size_t* relay, size_t* linv, size_t* rhs, size_t* sync) {
@@ -718,6 +685,137 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
   return MBD_OK;
 }
 
+// The plan of the eigenvalue stages of the geometries in `list` (descending
+// size): the one-stage grouped launch, the bands' chase and the eigenvalue and
+// energy launches, with their device tables.
+int plan_eigen(mbd_ctx* ctx, const std::vector<int>& list, EigenPlan* ep) {
+  auto banded = [&](int g) { return two_stage(ctx, ctx->geoms[g]->plan.nH); };
+  // one-stage tridiagonal plan for the matrices too large for the two-stage path
+  std::vector<int> sizes, one_stage;
+  for (int g : list)
+    if (!banded(g)) {
+      sizes.push_back(ctx->geoms[g]->plan.nH);
+      one_stage.push_back(g);
+    }
+  const TrdPlan tp = plan_tridiag(sizes, ctx->num_sms * ctx->trd_ctas_per_sm);
+  std::vector<TridiagJob> jobs;
+  std::vector<TridiagGroup> groups;
+  size_t ws_off = 0;
+  int cta = 0;
+  for (size_t b = 0; b < tp.bins.size(); ++b) {
+    TridiagGroup gr{};
+    gr.first_cta = cta;
+    gr.G = tp.G[b];
+    gr.job_begin = (int)jobs.size();
+    gr.nmax = 1;
+    for (int j : tp.bins[b]) {
+      GeomDev* gd = ctx->geoms[one_stage[j]].get();
+      const GeomPlan& p = gd->plan;
+      jobs.push_back(TridiagJob{gd->hmat, p.nH, p.ldH, gd->d, gd->e});
+      gr.nmax = std::max(gr.nmax, p.nH);
+    }
+    gr.job_end = (int)jobs.size();
+    gr.ws_offset = ws_off;
+    ws_off += (tridiag_workspace_bytes(gr.nmax, gr.G) + 255) & ~size_t(255);
+    cta += gr.G;
+    groups.push_back(gr);
+  }
+  ep->n_trd_groups = (int)groups.size();
+  ep->trd_total_ctas = cta;
+  MBD_CUDA(ep->tridiag_ws.reserve(ws_off));
+  // eigenvalue jobs: the batched launch first, then matrices too large for it
+  std::vector<EigJob> eig;
+  ep->eig_single.clear();
+  ep->eig_batch_max_n = 0;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int g : list) {
+      GeomDev* gd = ctx->geoms[g].get();
+      const GeomPlan& p = gd->plan;
+      const bool fits = p.nH <= kEigBatchMaxN;
+      if (fits != (pass == 0)) continue;
+      eig.push_back(EigJob{gd->d, gd->e, gd->ev, gd->scalars, gd->energy, p.nH, p.nsl});
+      if (fits) ep->eig_batch_max_n = std::max(ep->eig_batch_max_n, p.nH);
+      else ep->eig_single.push_back(g);
+    }
+  ep->n_eig_jobs = (int)eig.size();
+  ep->n_eig_batch = ep->n_eig_jobs - (int)ep->eig_single.size();
+  // band -> tridiagonal: one job per two-stage matrix, (job, sweep) items
+  // ordered by sweep then job, each pointing at its job's previous sweep
+  // (the bands that fit a cluster's shared memory first, largest first; the
+  // flag-synchronised chase takes the rest, and all of them while the
+  // failure-detection stall is on: its waits are the ones that can run out)
+  std::vector<BandJob> bjobs, fjobs;
+  // one chase kernel per batch (the two launches would run one after the
+  // other): the one tuned for the batch's largest band, whose chase sets the
+  // launch's length
+  int big = 0;
+  for (int g : list)
+    if (banded(g)) big = std::max(big, ctx->geoms[g]->plan.nH);
+  const bool cluster_ok = ctx->cluster_chase && ctx->test_stall_wait != kStallChase && big > 0 &&
+                          big <= sb2st_cluster_max_n() && tuned_chase_c(ctx, big) != kChaseFlag;
+  const int cap = cluster_ok ? sb2st_cluster_max_n() : 0;
+  ep->band_max_n = ep->band_cluster_max_n = 0;
+  for (int g : list) {
+    GeomDev* gd = ctx->geoms[g].get();
+    if (!banded(g)) continue;
+    const BandJob bj{gd->band.as<double>(), gd->plan.nH, gd->d, gd->e};
+    if (bj.n <= cap) {
+      bjobs.push_back(bj);
+      ep->band_cluster_max_n = std::max(ep->band_cluster_max_n, bj.n);
+    } else {
+      fjobs.push_back(bj);
+      ep->band_max_n = std::max(ep->band_max_n, bj.n);
+    }
+  }
+  std::stable_sort(bjobs.begin(), bjobs.end(), [](const BandJob& a, const BandJob& b) { return a.n > b.n; });
+  ep->n_band_cluster = (int)bjobs.size();
+  ep->band_cluster_C = sb2st_cluster_size(ep->band_cluster_max_n, ep->n_band_cluster, ctx->num_sms,
+                                           tuned_chase_c(ctx, ep->band_cluster_max_n));
+  if (ep->n_band_cluster > 0 && ep->band_cluster_C < 1) {   // no cluster fits after all
+    fjobs.insert(fjobs.begin(), bjobs.begin(), bjobs.end());
+    for (const BandJob& bj : bjobs) ep->band_max_n = std::max(ep->band_max_n, bj.n);
+    bjobs.clear();
+    ep->n_band_cluster = 0;
+  }
+  std::vector<SweepItem> items;
+  {
+    std::vector<int> last(fjobs.size(), -1);
+    for (int i = 0; i + 3 <= ep->band_max_n; ++i)
+      for (size_t j = 0; j < fjobs.size(); ++j) {
+        if (i + 3 > fjobs[j].n) continue;
+        items.push_back(SweepItem{(int)j, i, last[j], 0});
+        last[j] = (int)items.size() - 1;
+      }
+  }
+  bjobs.insert(bjobs.end(), fjobs.begin(), fjobs.end());
+  ep->n_band_jobs = (int)bjobs.size();
+  ep->sweeps_in_flight = 0;
+  for (const BandJob& bj : fjobs) ep->sweeps_in_flight += bj.n / (2 * kBand) + 1;
+  ep->n_sweep_items = (int)items.size();
+  MBD_CUDA(ep->sweep_progress.reserve(2 * sizeof(int) * std::max<size_t>(items.size(), 1)));
+  const size_t b_jobs = bytes_of<TridiagJob>(jobs.size());
+  const size_t b_groups = bytes_of<TridiagGroup>(groups.size());
+  const size_t b_eig = bytes_of<EigJob>(eig.size());
+  const size_t b_bj = bytes_of<BandJob>(bjobs.size());
+  const size_t b_it = bytes_of<SweepItem>(items.size());
+  MBD_CUDA(ep->tables.reserve(b_jobs + b_groups + b_eig + b_bj + b_it));
+  char* base = ep->tables.as<char>();
+  ep->trd_jobs = reinterpret_cast<TridiagJob*>(base);
+  ep->trd_groups = reinterpret_cast<TridiagGroup*>(base + b_jobs);
+  ep->eig_jobs = reinterpret_cast<EigJob*>(base + b_jobs + b_groups);
+  ep->band_jobs = reinterpret_cast<BandJob*>(base + b_jobs + b_groups + b_eig);
+  ep->sweep_items = reinterpret_cast<SweepItem*>(base + b_jobs + b_groups + b_eig + b_bj);
+  std::vector<char> host(b_jobs + b_groups + b_eig + b_bj + b_it, 0);
+  std::memcpy(host.data(), jobs.data(), sizeof(TridiagJob) * jobs.size());
+  std::memcpy(host.data() + b_jobs, groups.data(), sizeof(TridiagGroup) * groups.size());
+  std::memcpy(host.data() + b_jobs + b_groups, eig.data(), sizeof(EigJob) * eig.size());
+  std::memcpy(host.data() + b_jobs + b_groups + b_eig, bjobs.data(), sizeof(BandJob) * bjobs.size());
+  std::memcpy(host.data() + b_jobs + b_groups + b_eig + b_bj, items.data(), sizeof(SweepItem) * items.size());
+  if (!host.empty()) MBD_CUDA(h2d_ordered(ctx, base, host.data(), host.size()));
+  ctx->h2d_bytes += (double)host.size();
+  return MBD_OK;
+}
+
 // Plain-path slot buffers, per-geometry Hamiltonians, the tridiagonal plan and
 // the device job tables of the uploaded batch.
 int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
@@ -754,8 +852,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
     }
   if (ctx->order.empty()) {
     ctx->n_slots = 0;
-    ctx->n_trd_groups = ctx->trd_total_ctas = ctx->n_eig_jobs = ctx->n_eig_batch = 0;
-    return MBD_OK;
+    return plan_eigen(ctx, {}, &ctx->eigen);
   }
   int st = plan_slots(ctx, eigen, tight);
   if (st != MBD_OK) return st;
@@ -800,134 +897,12 @@ int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
     }
   }
   if (!eigen) {
-    ctx->n_trd_groups = ctx->trd_total_ctas = ctx->n_eig_jobs = ctx->n_eig_batch = 0;
-    return MBD_OK;
+    return plan_eigen(ctx, {}, &ctx->eigen);
   }
-  // one-stage tridiagonal plan for the matrices too large for the two-stage path
-  std::vector<int> sizes, one_stage;
+  std::vector<int> list;
   for (int g : ctx->order)
-    if (!ctx->geoms[g]->trace && !two_stage(ctx, ctx->geoms[g]->plan.nH)) {
-      sizes.push_back(ctx->geoms[g]->plan.nH);
-      one_stage.push_back(g);
-    }
-  const TrdPlan tp = plan_tridiag(sizes, ctx->num_sms * ctx->trd_ctas_per_sm);
-  std::vector<TridiagJob> jobs;
-  std::vector<TridiagGroup> groups;
-  size_t ws_off = 0;
-  int cta = 0;
-  for (size_t b = 0; b < tp.bins.size(); ++b) {
-    TridiagGroup gr{};
-    gr.first_cta = cta;
-    gr.G = tp.G[b];
-    gr.job_begin = (int)jobs.size();
-    gr.nmax = 1;
-    for (int j : tp.bins[b]) {
-      GeomDev* gd = ctx->geoms[one_stage[j]].get();
-      const GeomPlan& p = gd->plan;
-      jobs.push_back(TridiagJob{gd->hmat, p.nH, p.ldH, gd->d, gd->e});
-      gr.nmax = std::max(gr.nmax, p.nH);
-    }
-    gr.job_end = (int)jobs.size();
-    gr.ws_offset = ws_off;
-    ws_off += (tridiag_workspace_bytes(gr.nmax, gr.G) + 255) & ~size_t(255);
-    cta += gr.G;
-    groups.push_back(gr);
-  }
-  ctx->n_trd_groups = (int)groups.size();
-  ctx->trd_total_ctas = cta;
-  ctx->trd_est_ms = tp.makespan_us / 1000.0;
-  MBD_CUDA(ctx->tridiag_ws.reserve(ws_off));
-  // eigenvalue jobs: the batched launch first, then matrices too large for it
-  std::vector<EigJob> eig;
-  ctx->eig_single.clear();
-  ctx->eig_batch_max_n = 0;
-  for (int pass = 0; pass < 2; ++pass)
-    for (int g : ctx->order) {
-      GeomDev* gd = ctx->geoms[g].get();
-      const GeomPlan& p = gd->plan;
-      const bool fits = p.nH <= kEigBatchMaxN;
-      if (gd->trace || fits != (pass == 0)) continue;
-      eig.push_back(EigJob{gd->d, gd->e, gd->ev, gd->scalars, gd->energy, p.nH, p.nsl});
-      if (fits) ctx->eig_batch_max_n = std::max(ctx->eig_batch_max_n, p.nH);
-      else ctx->eig_single.push_back(g);
-    }
-  ctx->n_eig_jobs = (int)eig.size();
-  ctx->n_eig_batch = ctx->n_eig_jobs - (int)ctx->eig_single.size();
-  // band -> tridiagonal: one job per two-stage matrix, (job, sweep) items
-  // ordered by sweep then job, each pointing at its job's previous sweep
-  // (the bands that fit a cluster's shared memory first, largest first; the
-  // flag-synchronised chase takes the rest, and all of them while the
-  // failure-detection stall is on: its waits are the ones that can run out)
-  std::vector<BandJob> bjobs, fjobs;
-  // one chase kernel per batch (the two launches would run one after the
-  // other): the one tuned for the batch's largest band, whose chase sets the
-  // launch's length
-  int big = 0;
-  for (int g : ctx->order)
-    if (banded(g)) big = std::max(big, ctx->geoms[g]->plan.nH);
-  const bool cluster_ok = ctx->cluster_chase && ctx->test_stall_wait != kStallChase && big > 0 &&
-                          big <= sb2st_cluster_max_n() && tuned_chase_c(ctx, big) != kChaseFlag;
-  const int cap = cluster_ok ? sb2st_cluster_max_n() : 0;
-  ctx->band_max_n = ctx->band_cluster_max_n = 0;
-  for (int g : ctx->order) {
-    GeomDev* gd = ctx->geoms[g].get();
-    if (!banded(g)) continue;
-    const BandJob bj{gd->band.as<double>(), gd->plan.nH, gd->d, gd->e};
-    if (bj.n <= cap) {
-      bjobs.push_back(bj);
-      ctx->band_cluster_max_n = std::max(ctx->band_cluster_max_n, bj.n);
-    } else {
-      fjobs.push_back(bj);
-      ctx->band_max_n = std::max(ctx->band_max_n, bj.n);
-    }
-  }
-  std::stable_sort(bjobs.begin(), bjobs.end(), [](const BandJob& a, const BandJob& b) { return a.n > b.n; });
-  ctx->n_band_cluster = (int)bjobs.size();
-  ctx->band_cluster_C = sb2st_cluster_size(ctx->band_cluster_max_n, ctx->n_band_cluster, ctx->num_sms,
-                                           tuned_chase_c(ctx, ctx->band_cluster_max_n));
-  if (ctx->n_band_cluster > 0 && ctx->band_cluster_C < 1) {   // no cluster fits after all
-    fjobs.insert(fjobs.begin(), bjobs.begin(), bjobs.end());
-    for (const BandJob& bj : bjobs) ctx->band_max_n = std::max(ctx->band_max_n, bj.n);
-    bjobs.clear();
-    ctx->n_band_cluster = 0;
-  }
-  std::vector<SweepItem> items;
-  {
-    std::vector<int> last(fjobs.size(), -1);
-    for (int i = 0; i + 3 <= ctx->band_max_n; ++i)
-      for (size_t j = 0; j < fjobs.size(); ++j) {
-        if (i + 3 > fjobs[j].n) continue;
-        items.push_back(SweepItem{(int)j, i, last[j], 0});
-        last[j] = (int)items.size() - 1;
-      }
-  }
-  bjobs.insert(bjobs.end(), fjobs.begin(), fjobs.end());
-  ctx->n_band_jobs = (int)bjobs.size();
-  ctx->sweeps_in_flight = 0;
-  for (const BandJob& bj : fjobs) ctx->sweeps_in_flight += bj.n / (2 * kBand) + 1;
-  ctx->n_sweep_items = (int)items.size();
-  MBD_CUDA(ctx->sweep_progress.reserve(2 * sizeof(int) * std::max<size_t>(items.size(), 1)));
-  const size_t b_jobs = bytes_of<TridiagJob>(jobs.size());
-  const size_t b_groups = bytes_of<TridiagGroup>(groups.size());
-  const size_t b_eig = bytes_of<EigJob>(eig.size());
-  const size_t b_bj = bytes_of<BandJob>(bjobs.size());
-  const size_t b_it = bytes_of<SweepItem>(items.size());
-  MBD_CUDA(ctx->tables.reserve(b_jobs + b_groups + b_eig + b_bj + b_it));
-  char* base = ctx->tables.as<char>();
-  ctx->trd_jobs = reinterpret_cast<TridiagJob*>(base);
-  ctx->trd_groups = reinterpret_cast<TridiagGroup*>(base + b_jobs);
-  ctx->eig_jobs = reinterpret_cast<EigJob*>(base + b_jobs + b_groups);
-  ctx->band_jobs = reinterpret_cast<BandJob*>(base + b_jobs + b_groups + b_eig);
-  ctx->sweep_items = reinterpret_cast<SweepItem*>(base + b_jobs + b_groups + b_eig + b_bj);
-  std::vector<char> host(b_jobs + b_groups + b_eig + b_bj + b_it, 0);
-  std::memcpy(host.data(), jobs.data(), sizeof(TridiagJob) * jobs.size());
-  std::memcpy(host.data() + b_jobs, groups.data(), sizeof(TridiagGroup) * groups.size());
-  std::memcpy(host.data() + b_jobs + b_groups, eig.data(), sizeof(EigJob) * eig.size());
-  std::memcpy(host.data() + b_jobs + b_groups + b_eig, bjobs.data(), sizeof(BandJob) * bjobs.size());
-  std::memcpy(host.data() + b_jobs + b_groups + b_eig + b_bj, items.data(), sizeof(SweepItem) * items.size());
-  if (!host.empty()) MBD_CUDA(h2d_ordered(ctx, base, host.data(), host.size()));
-  ctx->h2d_bytes += (double)host.size();
-  return MBD_OK;
+    if (!ctx->geoms[g]->trace) list.push_back(g);
+  return plan_eigen(ctx, list, &ctx->eigen);
 }
 
 // Buffers only the mixed mode uses (allocated on first use).  Where the FP64
@@ -975,6 +950,80 @@ int reserve_mixed(mbd_ctx* ctx) {
   return MBD_OK;
 }
 
+// Enqueues a plan's stages behind the bands and Hamiltonians of its geometries;
+// bev (or null): the batch's timing events.
+int enqueue_eigen(mbd_ctx* ctx, const EigenPlan& ep, cudaStream_t s, const cudaEvent_t* bev) {
+  // bands -> tridiagonal in one persistent launch; matrices too large for the
+  // two-stage path in one grouped one-stage launch
+  if (ep.n_trd_groups > 0) {
+    MBD_CUDA(launch_tridiag_groups(ep.trd_jobs, ep.trd_groups, ep.n_trd_groups, ep.trd_total_ctas,
+                                   ep.tridiag_ws.p, ctx->err_flag, s));
+    ctx->launches += 2;
+  }
+  if (bev) record_timing(ctx, bev[4], s);
+  if (ep.n_band_cluster > 0) {
+    MBD_CUDA(launch_sb2st_cluster(ep.band_jobs, ep.n_band_cluster, ep.band_cluster_max_n,
+                                  ep.band_cluster_C, s));
+    ctx->launches += 1;
+  }
+  if (ep.n_band_jobs > ep.n_band_cluster) {
+    MBD_CUDA(launch_sb2st(ep.band_jobs + ep.n_band_cluster, ep.n_band_jobs - ep.n_band_cluster,
+                          ep.sweep_items, ep.n_sweep_items, ep.sweep_progress.as<int>(), ctx->err_flag,
+                          ctx->num_sms, ep.band_max_n, ep.sweeps_in_flight, ctx->test_stall_wait == kStallChase ? 0 : -1, s));
+    ctx->launches += 3;
+  }
+  if (bev) record_timing(ctx, bev[2], s);
+  // eigenvalues and energies
+  launch_eigen_batch(ep.eig_jobs, ep.n_eig_batch, ep.eig_batch_max_n, s);
+  ctx->launches += ep.n_eig_batch > 0 ? 1 : 0;
+  for (int g : ep.eig_single) {
+    GeomDev* gd = ctx->geoms[g].get();
+    launch_tridiag_eigenvalues(gd->d, gd->e, gd->plan.nH, gd->ev, s);
+    ctx->launches += 2;
+  }
+  launch_energy_batch(ep.eig_jobs, ep.n_eig_jobs, s);
+  ctx->launches += ep.n_eig_jobs > 0 ? 1 : 0;
+  return cuda_status(cudaGetLastError());
+}
+
+// Lets stream s wait for everything enqueued on the slots' streams.
+int join_slots(mbd_ctx* ctx, cudaStream_t s) {
+  for (int k = 0; k < ctx->n_slots; ++k) {
+    MBD_CUDA(cudaEventRecord(ctx->slots[k]->done, ctx->slots[k]->stream));
+    MBD_CUDA(cudaStreamWaitEvent(s, ctx->slots[k]->done, 0));
+  }
+  return MBD_OK;
+}
+
+// The energies of `list` (descending size) from eigenvalues, after a compute:
+// geometries whose trace form was refused (their Hamiltonians are whole), and
+// re-runs of the residual gate (reduced to their bands by run_front already,
+// unless they too were traced).  The reductions run side by side on the slots'
+// streams, then one launch a stage serves all, as in the batch: 40 chains of 10
+// to 88 Na atoms 65 ms one after the other, 10.5 so.
+int run_tail(mbd_ctx* ctx, const std::vector<int>& list) {
+  for (int g : list) {
+    GeomDev* gd = ctx->geoms[g].get();
+    if (!gd->trace || !two_stage(ctx, gd->plan.nH)) continue;
+    MBD_CUDA(gd->band.reserve(sizeof(double) * (size_t)gd->plan.nH * kBandLd));
+    MBD_CUDA(ctx->slots[gd->slot]->tail_trd_ws.reserve(sizeof(double) * sy2sb_workspace_doubles(gd->plan.nH)));
+  }
+  int st = plan_eigen(ctx, list, &ctx->tail);
+  if (st != MBD_OK) return st;
+  for (int g : list) {
+    GeomDev* gd = ctx->geoms[g].get();
+    const GeomPlan& p = gd->plan;
+    if (!gd->trace || !two_stage(ctx, p.nH)) continue;
+    RelaySlot& sl = *ctx->slots[gd->slot];
+    MBD_CUDA(launch_sy2sb(gd->hmat, p.ldH, p.nH, sl.tail_trd_ws.as<double>(), gd->band.as<double>(), ctx->num_sms,
+                          sl.stream, tuned_rows(ctx, p.nH), tuned_panel_qr(ctx, p.nH), lookahead_for(ctx, sl.la)));
+    ctx->launches += sy2sb_launches(p.nH);
+  }
+  st = join_slots(ctx, ctx->stream);
+  if (st != MBD_OK) return st;
+  return enqueue_eigen(ctx, ctx->tail, ctx->stream, nullptr);
+}
+
 // Enqueues the whole batch (relay stages on the slots' streams, then the
 // batch-wide eigen stages on the context stream).  Stream-capture safe: no
 // allocation, no host-side copies, and the mixed solve's progress flags are
@@ -1003,41 +1052,11 @@ int enqueue_batch(mbd_ctx* ctx, int mode) {
     int st = run_front(ctx, ctx->geoms[g].get(), g, mode);
     if (st != MBD_OK) return st;
   }
-  for (int k = 0; k < ctx->n_slots; ++k) {
-    MBD_CUDA(cudaEventRecord(ctx->slots[k]->done, ctx->slots[k]->stream));
-    MBD_CUDA(cudaStreamWaitEvent(s, ctx->slots[k]->done, 0));
-  }
+  int st = join_slots(ctx, s);
+  if (st != MBD_OK) return st;
   record_timing(ctx, bev[1], s);
-  // bands -> tridiagonal in one persistent launch; matrices too large for the
-  // two-stage path in one grouped one-stage launch
-  if (ctx->n_trd_groups > 0) {
-    MBD_CUDA(launch_tridiag_groups(ctx->trd_jobs, ctx->trd_groups, ctx->n_trd_groups, ctx->trd_total_ctas,
-                                   ctx->tridiag_ws.p, ctx->err_flag, s));
-    ctx->launches += 2;
-  }
-  record_timing(ctx, bev[4], s);
-  if (ctx->n_band_cluster > 0) {
-    MBD_CUDA(launch_sb2st_cluster(ctx->band_jobs, ctx->n_band_cluster, ctx->band_cluster_max_n,
-                                  ctx->band_cluster_C, s));
-    ctx->launches += 1;
-  }
-  if (ctx->n_band_jobs > ctx->n_band_cluster) {
-    MBD_CUDA(launch_sb2st(ctx->band_jobs + ctx->n_band_cluster, ctx->n_band_jobs - ctx->n_band_cluster,
-                          ctx->sweep_items, ctx->n_sweep_items, ctx->sweep_progress.as<int>(), ctx->err_flag,
-                          ctx->num_sms, ctx->band_max_n, ctx->sweeps_in_flight, ctx->test_stall_wait == kStallChase ? 0 : -1, s));
-    ctx->launches += 3;
-  }
-  record_timing(ctx, bev[2], s);
-  // eigenvalues and energies
-  launch_eigen_batch(ctx->eig_jobs, ctx->n_eig_batch, ctx->eig_batch_max_n, s);
-  ctx->launches += ctx->n_eig_batch > 0 ? 1 : 0;
-  for (int g : ctx->eig_single) {
-    GeomDev* gd = ctx->geoms[g].get();
-    launch_tridiag_eigenvalues(gd->d, gd->e, gd->plan.nH, gd->ev, s);
-    ctx->launches += 2;
-  }
-  launch_energy_batch(ctx->eig_jobs, ctx->n_eig_jobs, s);
-  ctx->launches += ctx->n_eig_jobs > 0 ? 1 : 0;
+  st = enqueue_eigen(ctx, ctx->eigen, s, bev);
+  if (st != MBD_OK) return st;
   record_timing(ctx, bev[3], s);
   return cuda_status(cudaGetLastError());
 }
@@ -1335,45 +1354,47 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
   const char* dev_out = ctx->results.as<char>();
   MBD_CUDA(cudaMemcpyAsync(hs, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   ctx->d2h_bytes = sizeof(int);
-  auto fetch = [&](size_t at, size_t bytes, cudaStream_t s) -> cudaError_t {
+  auto fetch = [&](size_t at, size_t bytes) -> cudaError_t {
     ctx->d2h_bytes += (double)bytes;
-    return cudaMemcpyAsync(hs + kHead + at, dev_out + at, bytes, cudaMemcpyDeviceToHost, s);
+    return cudaMemcpyAsync(hs + kHead + at, dev_out + at, bytes, cudaMemcpyDeviceToHost, ctx->stream);
   };
-  auto fetch_one = [&](const GeomDev* gd, cudaStream_t s) { return fetch(gd->out_at, gd->out_bytes, s); };
-  if (!ctx->order.empty()) MBD_CUDA(fetch(0, ctx->out_bytes, ctx->stream));
+  if (!ctx->order.empty()) MBD_CUDA(fetch(0, ctx->out_bytes));
   MBD_CUDA(cudaStreamSynchronize(ctx->stream));
   int err = 0;
   std::memcpy(&err, hs, sizeof(int));
+  // what a re-run of some geometries left in the place of their staged
+  // results; its device waits may have run out
+  auto fetch_again = [&](const std::vector<int>& list) -> int {
+    MBD_CUDA(cudaMemcpyAsync(hs, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    for (int g : list) MBD_CUDA(fetch(ctx->geoms[g]->out_at, ctx->geoms[g]->out_bytes));
+    MBD_CUDA(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(&err, hs, sizeof(int));
+    return MBD_OK;
+  };
   auto host = [&](const void* dev) -> const char* { return hs + kHead + (static_cast<const char*>(dev) - dev_out); };
   // the stage timings are read from their events when someone asks for them
   ctx->timed.pending = true;
   ctx->timed.set = ctx->event_set;
   ctx->timed.geoms.clear();
   for (int g : ctx->order) ctx->timed.geoms.emplace_back(g, ctx->geoms[g]->trace);
-  int first = MBD_OK;
   for (size_t g = 0; g < ctx->geoms.size(); ++g) {
-    GeomDev* gd = ctx->geoms[g].get();
-    const GeomPlan& p = gd->plan;
     mbd_result& r = out[g];
-    r.status = gd->status_host;
-    for (int k = 0; k < 3; ++k) r.supercell[k] = p.sl[k];
+    r.status = ctx->geoms[g]->status_host;
+    for (int k = 0; k < 3; ++k) r.supercell[k] = ctx->geoms[g]->plan.sl[k];
     r.refine_iters = 0;
     for (int k = 0; k < 3; ++k) r.err_est[k] = 0.0;
-    if (gd->status_host != MBD_OK) {
-      r.energy_Ha = std::nan("");
-      r.c6_mol = std::nan("");
-      r.nimag = 0;
-      if (first == MBD_OK) first = r.status;
-      continue;
-    }
-    const int N = p.N;
-    if (ctx->last_mode != MBD_MODE_PLAIN_FP64) {
-      // residual gate of the mixed relay solve; a miss re-runs this geometry
-      // with the direct FP64 solve (the plain path) before reading results
+  }
+  // residual gate of the mixed relay solves; a miss re-runs the geometry with
+  // the direct FP64 solve (the plain path) before its results are read
+  std::vector<int> rerun, tail;
+  if (ctx->last_mode != MBD_MODE_PLAIN_FP64)
+    for (int g : ctx->order) {
+      GeomDev* gd = ctx->geoms[g].get();
+      mbd_result& r = out[g];
       const double* rn = reinterpret_cast<const double*>(host(gd->rnorm2));
       double worst = 0.0;
       for (int f = 0; f < 21; ++f) {
-        const double v = std::sqrt(rn[f] / (3.0 * N));
+        const double v = std::sqrt(rn[f] / (3.0 * gd->plan.N));
         worst = std::isfinite(v) ? std::max(worst, v) : std::numeric_limits<double>::infinity();
       }
       r.err_est[0] = r.err_est[1] = r.err_est[2] = worst;
@@ -1396,34 +1417,48 @@ int mbd_rsscs_download(mbd_ctx* ctx, mbd_result* out) {
         gd->cg_iters_seen = ok ? (int)most : 0;
         gd->cg_iters_seen1 = ok ? (int)most1 : 0;
       }
-      if (!(worst <= ctx->residual_gate)) {
-        int st = run_front(ctx, gd, (int)g, MBD_MODE_PLAIN_FP64);
-        if (st == MBD_OK && !gd->trace) st = run_tail_single(ctx, gd, ctx->slots[gd->slot]->stream);
-        if (st != MBD_OK) return st;
-        const cudaStream_t ss = ctx->slots[gd->slot]->stream;
-        // the re-run's results replace the staged ones; its waits may have run out
-        MBD_CUDA(cudaMemcpyAsync(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ss));
-        MBD_CUDA(fetch_one(gd, ss));
-        MBD_CUDA(cudaStreamSynchronize(ss));
-        r.refine_iters = -1;
-      }
+      if (worst <= ctx->residual_gate) continue;
+      rerun.push_back(g);
+      r.refine_iters = -1;
     }
-    if (gd->trace && err == 0) {
-      // a refused trace form (an imaginary mode, or a Hamiltonian too near
-      // one): the eigenvalues, if the relay gave a Hamiltonian at all
-      const double* sc = reinterpret_cast<const double*>(host(gd->scalars));
-      const int* fi = reinterpret_cast<const int*>(host(gd->info));
-      bool relay_ok = sc[2] == 0.0;
-      for (int f = 0; f < 21; ++f) relay_ok = relay_ok && fi[f] == 0;
-      if (relay_ok && reinterpret_cast<const double*>(host(gd->energy))[3] != kTraceOk) {
-        const cudaStream_t ss = ctx->slots[gd->slot]->stream;
-        int st = run_tail_single(ctx, gd, ss);
-        if (st != MBD_OK) return st;
-        MBD_CUDA(cudaMemcpyAsync(&err, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ss));
-        MBD_CUDA(fetch_one(gd, ss));
-        MBD_CUDA(cudaStreamSynchronize(ss));
-      }
+  if (!rerun.empty()) {
+    for (int g : rerun) {
+      int st = run_front(ctx, ctx->geoms[g].get(), g, MBD_MODE_PLAIN_FP64);
+      if (st != MBD_OK) return st;
+      if (!ctx->geoms[g]->trace) tail.push_back(g);
     }
+    int st = join_slots(ctx, ctx->stream);
+    if (st == MBD_OK) st = fetch_again(rerun);
+    if (st != MBD_OK) return st;
+  }
+  // refused trace forms (an imaginary mode, or a Hamiltonian too near one): the
+  // eigenvalues, where the relay gave a Hamiltonian at all
+  for (int g : ctx->order) {
+    const GeomDev* gd = ctx->geoms[g].get();
+    if (!gd->trace || reinterpret_cast<const double*>(host(gd->energy))[3] == kTraceOk) continue;
+    const int* info = reinterpret_cast<const int*>(host(gd->info));
+    const bool relay_ok = std::all_of(info, info + 21, [](int i) { return i == 0; });
+    if (relay_ok && reinterpret_cast<const double*>(host(gd->scalars))[2] == 0.0) tail.push_back(g);
+  }
+  if (!tail.empty() && err == 0) {
+    std::stable_sort(tail.begin(), tail.end(),
+                     [&](int a, int b) { return ctx->geoms[a]->plan.n > ctx->geoms[b]->plan.n; });
+    int st = run_tail(ctx, tail);
+    if (st == MBD_OK) st = fetch_again(tail);
+    if (st != MBD_OK) return st;
+  }
+  int first = MBD_OK;
+  for (size_t g = 0; g < ctx->geoms.size(); ++g) {
+    GeomDev* gd = ctx->geoms[g].get();
+    mbd_result& r = out[g];
+    if (gd->status_host != MBD_OK) {
+      r.energy_Ha = std::nan("");
+      r.c6_mol = std::nan("");
+      r.nimag = 0;
+      if (first == MBD_OK) first = r.status;
+      continue;
+    }
+    const int N = gd->plan.N;
     const double* aiw = reinterpret_cast<const double*>(host(gd->alpha_iw));
     const double* molpol = reinterpret_cast<const double*>(host(gd->molpol));
     const double* scal = reinterpret_cast<const double*>(host(gd->scalars));

@@ -109,6 +109,25 @@ struct GeomDev {
   DevBuf train;      // x [21N][8] and S_true [21N][9] of a training batch
 };
 
+// The eigenvalue stages of some geometries of the batch: tables and workspaces
+// of their batch-wide launches.
+struct EigenPlan {
+  DevBuf tables, tridiag_ws, sweep_progress;
+  TridiagJob* trd_jobs = nullptr;
+  TridiagGroup* trd_groups = nullptr;
+  EigJob* eig_jobs = nullptr;
+  BandJob* band_jobs = nullptr;
+  SweepItem* sweep_items = nullptr;
+  int n_band_jobs = 0, n_sweep_items = 0, band_max_n = 0;
+  // band jobs [0, n_band_cluster) run in the cluster-resident chase (cluster
+  // size band_cluster_C, largest n band_cluster_max_n), the rest in the
+  // flag-synchronised one
+  int n_band_cluster = 0, band_cluster_C = 0, band_cluster_max_n = 0;
+  long long sweeps_in_flight = 0;
+  int n_trd_groups = 0, trd_total_ctas = 0, n_eig_jobs = 0, n_eig_batch = 0, eig_batch_max_n = 0;
+  std::vector<int> eig_single;               // geometries whose eigenvalues need their own launch
+};
+
 // One relay slot: a stream and the relay workspaces of the geometries it runs
 // (sized for the largest of them).
 struct RelaySlot {
@@ -118,7 +137,7 @@ struct RelaySlot {
   DevBuf relay64, linv, rhs, chol_sync;                       // plain FP64 path
   DevBuf relay32, p_hi, p_lo, l_hi, l_lo, mixv, res_ws, solve_sync;   // mixed path
   DevBuf cg, gnn;                                             // learned path: CG vectors, network work
-  DevBuf trd_ws;                                              // dense -> band workspace
+  DevBuf trd_ws, tail_trd_ws;                                 // dense -> band workspace; of refused trace forms
   DevBuf trace_ws;                                            // trace form: bounds, nodes, counters
   int solve_epoch = 0;
   bool mixed_direct = true;   // room for the FP64 factors of the mixed mode's small geometries
@@ -131,7 +150,7 @@ struct RelaySlot {
   }
   size_t held() const {
     return relay64.bytes + linv.bytes + rhs.bytes + chol_sync.bytes + relay32.bytes + p_hi.bytes + p_lo.bytes + l_hi.bytes +
-           l_lo.bytes + mixv.bytes + res_ws.bytes + solve_sync.bytes + cg.bytes + gnn.bytes + trd_ws.bytes + trace_ws.bytes;
+           l_lo.bytes + mixv.bytes + res_ws.bytes + solve_sync.bytes + cg.bytes + gnn.bytes + trd_ws.bytes + tail_trd_ws.bytes + trace_ws.bytes;
   }
 };
 
@@ -169,8 +188,7 @@ struct mbd_ctx {
   std::vector<std::unique_ptr<mbd::RelaySlot>> slots;
   int n_slots = 0;                           // slots in use for the current batch
   bool slots_unasked = false;                // planned without asking how much memory is free (plan_slots)
-  mbd::DevBuf tridiag_ws, tables, misc, fb_ws;
-  mbd::DevBuf fb_band, fb_trd;   // a refused trace form's reduction (never part of a graph)
+  mbd::DevBuf misc, fb_ws;
   mbd::DevBuf inputs, results, hmats;   // the batch's geometries: inputs; results (first what goes back); Hamiltonians
   size_t out_bytes = 0;                 // of results, what goes back to the host
   mbd::HostBuf in_staging, staging;     // upload and download: one copy for the batch
@@ -180,24 +198,10 @@ struct mbd_ctx {
   // standalone eigenvalue call: matrix, (d, e, eigenvalues, scratch), workspace
   mbd::DevBuf eig_a, eig_vec, eig_ws;
   mbd::DevBuf eigh_buf;   // mbd_rsscs_eigh: matrix, reflectors, vectors, Gram, scratch
-  // batch plan (device tables in `tables`)
-  mbd::TridiagJob* trd_jobs = nullptr;
-  mbd::TridiagGroup* trd_groups = nullptr;
-  mbd::EigJob* eig_jobs = nullptr;
-  mbd::BandJob* band_jobs = nullptr;
-  mbd::SweepItem* sweep_items = nullptr;
-  mbd::DevBuf sweep_progress;
-  int n_band_jobs = 0, n_sweep_items = 0, band_max_n = 0;
-  // band jobs [0, n_band_cluster) run in the cluster-resident chase (cluster
-  // size band_cluster_C, largest n band_cluster_max_n), the rest in the
-  // flag-synchronised one
-  int n_band_cluster = 0, band_cluster_C = 0, band_cluster_max_n = 0;
+  mbd::EigenPlan eigen;      // the batch's geometries whose energies come from eigenvalues
+  mbd::EigenPlan tail;       // those a download finds to need them (never part of a graph)
   bool cluster_chase = true;                 // MBD_B200_CLUSTER_CHASE=0 turns the cluster-resident chase off
-  long long sweeps_in_flight = 0;
-  int n_trd_groups = 0, trd_total_ctas = 0, n_eig_jobs = 0, n_eig_batch = 0, eig_batch_max_n = 0;
-  double trd_est_ms = 0.0;
   std::vector<int> order;                    // geometries that run, descending relay size
-  std::vector<int> eig_single;               // geometries whose eigenvalues need their own launch
   double* weights_dev = nullptr;
   double* omega_dev = nullptr;               // the 21 imaginary frequencies
   // learned warm start: network parameters, Adam state, training work

@@ -189,9 +189,10 @@ int autotune(mbd_ctx* ctx, int max_n) {
   if (status != MBD_OK) return status;
   // the captured graphs and the batch's chase plan used the old choices
   drop_graphs(ctx);
-  if (ctx->n_band_cluster > 0)
-    ctx->band_cluster_C = sb2st_cluster_size(ctx->band_cluster_max_n, ctx->n_band_cluster, ctx->num_sms,
-                                             ctx->tune[tune_class(ctx->band_cluster_max_n)].chase_c);
+  EigenPlan& ep = ctx->eigen;
+  if (ep.n_band_cluster > 0)
+    ep.band_cluster_C = sb2st_cluster_size(ep.band_cluster_max_n, ep.n_band_cluster, ctx->num_sms,
+                                           ctx->tune[tune_class(ep.band_cluster_max_n)].chase_c);
   return MBD_OK;
 }
 
