@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "chol64.cuh"
@@ -72,14 +73,15 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 }
 
 // Waits until *p >= want; past the limit (or once any wait has run out) it
-// records the time-out and returns `want`, so every task still ends.
-__device__ int wait_count(const int* p, int want, int* err) {
+// records the time-out and returns `want`, so every task still ends; so it does
+// once the launch is called off (*stop).
+__device__ int wait_count(const int* p, int want, int* err, const int* stop) {
   int v = ld_acquire(p);
   if (v >= want) return v;
   const long long limit = wait_limit_cycles();
   const long long t0 = clock64();
   while ((v = ld_acquire(p)) < want) {
-    if (*(volatile int*)err != 0) return want;
+    if (*(volatile int*)err != 0 || (stop && *(const volatile int*)stop != 0)) return want;
     if (clock64() - t0 > limit) {
       atomicCAS(err, 0, kErrTimeout);
       return want;
@@ -104,7 +106,11 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
   if (nb <= 0) return;
   int k = 0;
   long long base = 0;                          // first ticket of block column k
-  if (tid == 0) s_ticket = atomicAdd(ticket, 1);
+  auto draw = [&] {                            // none once the launch is called off
+    const int t = atomicAdd(ticket, 1);
+    return a.stop && *(const volatile int*)a.stop != 0 ? INT_MAX : t;
+  };
+  if (tid == 0) s_ticket = draw();
   for (;;) {
     __syncthreads();
     const int t = s_ticket;
@@ -126,9 +132,9 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
     int avail = 0;                                   // block columns known to be finished for all operands
     auto await = [&](int want) {                     // block-uniform
       if (tid == 0) {
-        int v = wait_count(done_b + k, want, a.err);
-        if (!is_diag) v = min(v, wait_count(done_b + rb0, want, a.err));
-        if (two) v = min(v, wait_count(done_b + rb0 + 1, want, a.err));
+        int v = wait_count(done_b + k, want, a.err, a.stop);
+        if (!is_diag) v = min(v, wait_count(done_b + rb0, want, a.err, a.stop));
+        if (two) v = min(v, wait_count(done_b + rb0 + 1, want, a.err, a.stop));
         s_avail = v;
       }
       __syncthreads();
@@ -249,7 +255,7 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
         for (int o = 16; o > 0; o >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
         if (lane == 0) a.logdet[(size_t)b * T + k] = lg;
       }
-      if (tid == 0) s_ticket = atomicAdd(ticket, 1);
+      if (tid == 0) s_ticket = draw();
       continue;
     }
     // tile: T = A - sum, then L = T Linv^T with the diagonal block's inverse.
@@ -354,7 +360,7 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
       run(std::integral_constant<int, 2>());
     }
     if (!early) {
-      if (tid == 0) wait_count(diag + b, a.stall && k == 0 ? 1 << 30 : k + 1, a.err);
+      if (tid == 0) wait_count(diag + b, a.stall && k == 0 ? 1 << 30 : k + 1, a.err, a.stop);
       __syncthreads();
       copy_inverse(n_chunks);
       copy_inverse(n_chunks + 1);
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(kFlowThreads, 2) chol_flow_kernel(CholFlowArgs
     cp_wait<0>();
     __syncthreads();
     int next = 0;
-    if (tid == 0) next = atomicAdd(ticket, 1);   // this task waits for nothing any more
+    if (tid == 0) next = draw();   // this task waits for nothing any more
     const double* X0 = dsm + (n_chunks % kStages) * kStageElems + g * XS + 2 * q4;
     const double* X1 = dsm + ((n_chunks + 1) % kStages) * kStageElems + g * XS + 2 * q4;
     // 64 rows at a time, so that the block row the next diagonal block waits

@@ -93,6 +93,7 @@ struct CholFlowArgs {
   int* info;               // [batch]: first failing column + 1 where a pivot is not positive; zeroed by the caller
   int* sync;               // chol_flow_sync_ints(n, batch) ints
   int* err;                // the context's error flag (a wait that ran out)
+  const int* stop;         // the launch is called off once this is not 0 (results are then unfinished); or null
   bool stall;              // tests: the first tiles wait for a diagonal block that never comes
 };
 constexpr int kCholFlowHead = 32;
