@@ -541,7 +541,8 @@ int run_front(mbd_ctx* ctx, GeomDev* gd, int gi, int mode, bool relay_only) {
   // 6. the energy from shifted Cholesky factors, or dense -> band (stage 1 of
   // the two-stage tridiagonalisation)
   if (gd->trace) {
-    TraceArgs ta{gd->hmat, p.nH, p.ldH, p.nsl, sl.relay64.as<double>(), sl.linv.as<double>(),
+    TraceArgs ta{gd->hmat, p.nH, p.ldH, p.nsl, learned ? kTraceDigitsIterative : kTraceDigits,
+                 sl.relay64.as<double>(), sl.linv.as<double>(),
                  sl.trace_ws.p, gd->scalars, gd->energy, ctx->err_flag, ctx->test_stall_wait == kStallFactor};
     MBD_CUDA(launch_trace_energy(ta, ctx->num_sms, s));
     ctx->launches += trace_launches(p.nH);

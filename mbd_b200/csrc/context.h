@@ -348,7 +348,7 @@ int reserve_learned(mbd_ctx* ctx);
 int band_to_tridiag_single(mbd_ctx* ctx, double* Br, int n, double* d, double* e, DevBuf& scratch, cudaStream_t s);
 int relay_learned(mbd_ctx* ctx, GeomDev* gd, RelaySlot& sl, size_t mstride, cudaEvent_t ev_net, double** X_out);
 
-// Largest Hamiltonian the trace form takes: its 21 factors need 14 GB there,
+// Largest Hamiltonian the trace form takes: its 23 factors need 16 GB there,
 // and the work grows as 5 to 7 n^3 against (4/3) n^3 of the reduction to a
 // band.  Energy of one cluster (ms, trace form / reduction): n = 1500 0.9 / 17,
 // 3000 4.7 / 37, 6000 37 / 87, 7500 55 / 123, 9000 96 / 165.

@@ -43,11 +43,6 @@ constexpr double kLowerShare = 0.2;      // m over the smallest diagonal entry
 constexpr int kLanczosSteps = 16;
 constexpr int kLanczosMinN = 2500;
 constexpr double kRitzShare = 0.7;       // m over the smallest Ritz value
-// Digits the rule is run to: exp(-33) of the strip estimate, measured
-// <= 2e-16 of sum sqrt(lambda) on clusters, molecules, sheets and boxes
-// (spectra from LAPACK, M/m from 6 to 160: 8 to 14 nodes).
-constexpr double kDigits = 33.0;
-
 struct TraceWs {
   double* part;      // [T][T * 64] absolute row sums per block column
   double* rowred;    // [T][3] per block row: largest Gershgorin bound, smallest diagonal, sum of the diagonal
@@ -322,7 +317,7 @@ __device__ double smallest_ritz(const TraceWs& w, int T) {
 }
 
 // Bounds, node count and nodes; one warp.
-__global__ void __launch_bounds__(32) nodes_kernel(TraceWs w, int n, int T) {
+__global__ void __launch_bounds__(32) nodes_kernel(TraceWs w, int n, int T, double digits) {
   const int lane = threadIdx.x;
   double hi = -1e300, lo = 1e300, tr = 0.0;
   for (int b = lane; b < T; b += 32) {
@@ -341,7 +336,7 @@ __global__ void __launch_bounds__(32) nodes_kernel(TraceWs w, int n, int T) {
   if (n >= kLanczosMinN && lo > 0.0) m = kRitzShare * smallest_ritz(w, T);
   int nodes = 0;
   if (lo > 0.0 && m > 0.0 && M >= lo && M < 1e300) {
-    const double want = ceil(kDigits * (log(M / m) + 2.772588722239781) / (2.0 * 9.869604401089358));
+    const double want = ceil(digits * (log(M / m) + 2.772588722239781) / (2.0 * 9.869604401089358));
     nodes = want <= kTraceNodes ? (int)want : 0;
   }
   if (lane < kTraceBatch) w.info[lane] = 0;
@@ -462,7 +457,7 @@ cudaError_t launch_trace_energy(const TraceArgs& a, int num_sms, cudaStream_t s)
       lanczos_next_kernel<<<T, NB, 0, s>>>(w, T, k);
     }
   }
-  nodes_kernel<<<1, 32, 0, s>>>(w, a.n, T);
+  nodes_kernel<<<1, 32, 0, s>>>(w, a.n, T, a.digits);
   CholFlowArgs f{};
   f.src = a.H;
   f.src_stride = 0;
