@@ -821,6 +821,7 @@ int plan_eigen(mbd_ctx* ctx, const std::vector<int>& list, EigenPlan* ep) {
 // the device job tables of the uploaded batch.
 int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
   drop_graphs(ctx, true);
+  ctx->replan = false;
   ctx->order.clear();
   for (size_t g = 0; g < ctx->geoms.size(); ++g)
     if (ctx->geoms[g]->status_host == MBD_OK) ctx->order.push_back((int)g);
@@ -1287,6 +1288,11 @@ int mbd_rsscs_compute(mbd_ctx* ctx, int mode) {
   if (mode != MBD_MODE_PLAIN_FP64 && mode != MBD_MODE_MIXED && mode != MBD_MODE_MIXED_LEARNED) return MBD_ERR_ARG;
   if (mode == MBD_MODE_MIXED_LEARNED && ctx->use_net && !ctx->have_net) return MBD_ERR_NO_NETWORK;
   MBD_CUDA(cudaSetDevice(ctx->device));
+  if (ctx->replan) {   // an option that the plan depends on has changed since the upload
+    MBD_CUDA(cudaDeviceSynchronize());
+    int st = prepare_batch(ctx, true);
+    if (st != MBD_OK) return st;
+  }
   auto reserve = [&] {
     return mode == MBD_MODE_MIXED ? reserve_mixed(ctx) : (mode == MBD_MODE_MIXED_LEARNED ? reserve_learned(ctx) : MBD_OK);
   };
@@ -1779,6 +1785,8 @@ int mbd_rsscs_set_option(mbd_ctx* ctx, int option, double value) {
         MBD_CUDA(cudaSetDevice(ctx->device));
         MBD_CUDA(cudaDeviceSynchronize());
         drop_graphs(ctx);   // the captured launches carry the old setting
+        // the chase's stall needs the eigenvalue path (plan_slots)
+        if (on == kStallChase || ctx->test_stall_wait == kStallChase) ctx->replan = true;
       }
       ctx->test_stall_wait = on;
       return MBD_OK;

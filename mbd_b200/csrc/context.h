@@ -187,6 +187,7 @@ struct mbd_ctx {
   std::vector<std::unique_ptr<mbd::GeomDev>> geoms;
   std::vector<std::unique_ptr<mbd::RelaySlot>> slots;
   int n_slots = 0;                           // slots in use for the current batch
+  bool replan = false;                       // the next compute plans the batch again (prepare_batch)
   bool slots_unasked = false;                // planned without asking how much memory is free (plan_slots)
   mbd::DevBuf misc, fb_ws;
   mbd::DevBuf inputs, results, hmats;   // the batch's geometries: inputs; results (first what goes back); Hamiltonians
