@@ -650,7 +650,8 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
       for (int g : ctx->order) {
         const GeomPlan& p = ctx->geoms[g]->plan;
         size_t a, b, c, d, e, f, h;
-        size_t bytes = plain_bytes(p, &a, &b, &c, &h) + mixed_bytes(p, &d, &e, &f, &h, &a, p.n <= kMixedDirectMaxN);
+        size_t bytes = plain_bytes(p, &a, &b, &c, &h) +
+                       mixed_bytes(p, &d, &e, &f, &h, &a, ctx->mixed_direct && p.n <= kMixedDirectMaxN);
         // the trace form's factors past what the relay's matrices leave
         if (ctx->geoms[g]->trace) {
           plain_bytes(p, &a, &b, &c, &h);
@@ -667,7 +668,6 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
   ctx->slots_unasked = held;
   for (int g : ctx->order) ctx->geoms[g]->slot = slot_of[g];
   while (tight && (int)ctx->slots.size() > S) ctx->slots.pop_back();
-  for (auto& sl : ctx->slots) sl->mixed_direct = true;
   while ((int)ctx->slots.size() < S) {
     std::unique_ptr<RelaySlot> sl(new RelaySlot());
     // slot 0 takes the batch's largest geometry (longest first), whose
@@ -682,6 +682,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
     MBD_CUDA(create_lookahead(&sl->la));
     ctx->slots.push_back(std::move(sl));
   }
+  for (auto& sl : ctx->slots) sl->mixed_direct = ctx->mixed_direct;
   ctx->n_slots = S;
   return MBD_OK;
 }
@@ -1183,6 +1184,10 @@ int mbd_rsscs_create(mbd_ctx** out, int device) {
     // previous panel's trailing update (MBD_B200_LOOKAHEAD=0: one stream)
     const char* la = std::getenv("MBD_B200_LOOKAHEAD");
     ctx->lookahead = !(la && la[0] == '0');
+    // the mixed mode's FP64 factors of small relay matrices
+    // (MBD_B200_MIXED_DIRECT=0: 3xTF32 factors and refinement at every size)
+    const char* md = std::getenv("MBD_B200_MIXED_DIRECT");
+    ctx->mixed_direct = !(md && md[0] == '0');
     // stream priorities (the largest geometry's slot, the look-ahead QR),
     // kept by captured graphs (MBD_B200_PRIORITY=0: default priority everywhere)
     const char* pr = std::getenv("MBD_B200_PRIORITY");

@@ -195,6 +195,7 @@ struct mbd_ctx {
   mbd::HostBuf in_staging, staging;     // upload and download: one copy for the batch
   mbd::Sy2sbLookAhead la_ctx{};   // look-ahead stream and events of the context-stream reductions
   bool lookahead = true;     // dense -> band look-ahead (MBD_B200_LOOKAHEAD=0: off)
+  bool mixed_direct = true;  // FP64 factors for small relay matrices in the mixed mode (MBD_B200_MIXED_DIRECT=0: off)
   bool priorities = true;    // stream and graph-node priorities (MBD_B200_PRIORITY=0: off)
   // standalone eigenvalue call: matrix, (d, e, eigenvalues, scratch), workspace
   mbd::DevBuf eig_a, eig_vec, eig_ws;
