@@ -61,10 +61,6 @@ __device__ __forceinline__ int chunk_row(int t) {
   return t < (m + 1) * (m + 1) ? 2 * m : 2 * m + 1;
 }
 
-__device__ __forceinline__ void ring_copy(unsigned dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-
 template <typename T>
 __global__ void __launch_bounds__(ST, 1) strip_kernel(StripArgs<T> a) {
   using D = Dims<T>;
@@ -307,13 +303,12 @@ __global__ void __launch_bounds__(ST, 1) strip_kernel(StripArgs<T> a) {
 
 template <typename T>
 int launch(const StripArgs<T>& a, cudaStream_t s) {
-  static int sms = 0;
-  if (sms == 0) {
+  static const int sms = [] {
     int dev = 0, v = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    sms = v > 0 ? v : 148;
-  }
+    return v > 0 ? v : 148;
+  }();
   const int ctas = std::min(sms, chunks_before<T>(a.nt) * a.batch);
   strip_kernel<T><<<ctas, ST, Dims<T>::kSmem, s>>>(a);
   return ctas;

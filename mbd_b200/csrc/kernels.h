@@ -342,11 +342,14 @@ void launch_cg_setup(const CgArgs& a, cudaStream_t s);
 // sums either way).
 void launch_cg_iteration(const CgArgs& a, int it, cudaStream_t s, bool fp32 = false);
 // Iterations [it0, it1) of an FP32-pass phase in one launch, for n <= kCgClusterMaxN
-// (state as launch_cg_iteration leaves it, but for the Z^T R slots).  Relay
-// solve of one cluster, four launches an iteration against this (ms): N = 61
-// 0.44 / 0.30, 200 0.77 / 0.56, 500 1.63 / 1.66, 680 2.05 / 1.97; beyond, a
-// cluster per frequency leaves too much of the device idle once most
-// frequencies have converged.
+// (state as launch_cg_iteration leaves it, but for the Z^T R slots).  Four
+// launches an iteration against this (ms).  A call on one cluster: N = 61 1.68 /
+// 0.66, 200 2.20 / 1.20, 500 3.51 / 2.64, 680 5.24 / 4.20; a cluster's share of a
+// batch's call: 24 of N = 61 0.96 / 0.24, 24 of 200 1.03 / 0.46, 16 of 500 2.21 /
+// 1.81, 16 of 680 3.58 / 3.29.  With the gaps between launches gone (the relay
+// solve alone in a replayed graph) the two meet there: 500 1.63 / 1.66, 680 2.05 /
+// 1.97; beyond, a cluster per frequency leaves too much of the device idle once
+// most frequencies have converged.
 constexpr int kCgClusterMaxN = 2048;
 cudaError_t init_cg_attributes();
 // share: geometries whose solves run side by side.

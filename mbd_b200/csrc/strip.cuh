@@ -112,10 +112,10 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   return r;
 }
 
-__device__ __forceinline__ void ring_copy(unsigned dst, const float* src) {
+__device__ __forceinline__ void ring_copy(unsigned dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void ring_copy(float4* dst, const float* src) {
+__device__ __forceinline__ void ring_copy(float4* dst, const void* src) {
   ring_copy((unsigned)__cvta_generic_to_shared(dst), src);
 }
 
