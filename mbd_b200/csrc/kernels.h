@@ -283,18 +283,18 @@ cudaError_t launch_sb2st_cluster(const BandJob* jobs, int n_jobs, int max_n, int
 // ---- the energy as a trace (k_trace.cu) ----
 // sum_i sqrt(lambda_i) of the Hamiltonian from shifted Cholesky factors,
 // without its eigenvalues.  Node 0 certifies H - m I positive definite.
-constexpr int kTraceNodes = 22;                    // quadrature nodes at most: spectra of M/m <= 10 800 in 36 digits
+constexpr int kTraceNodes = 22;                    // quadrature nodes at most: spectra of M/m <= 15 300 in 35 digits
 constexpr int kTraceBatch = kTraceNodes + 1;
-// Digits the rule is run to, as the exponent of its strip estimate.  exp(-36):
-// measured <= 3e-17 of sum sqrt(lambda) on spectra of clusters, molecules,
+// Digits the rule is run to, as the exponent of its strip estimate.  exp(-35):
+// measured <= 9e-17 of sum sqrt(lambda) on spectra of clusters, molecules,
 // sheets and boxes (LAPACK's, summed in extended precision; M/m from 7 to 825: 9
-// to 18 nodes), a tenth of what rounding leaves.  Energies of 39 systems of 12 to
-// 533 atoms against extended precision, rms of the relative error: 5.5e-14;
-// exp(-33) 1.5e-13, from eigenvalues 8.9e-14.  exp(-33), mostly a node fewer
-// (256-atom box of 6144 rows 31.3 against 33.7 ms a call), leaves up to 7e-16 of
-// the sum, 5e-13 of the energy: for Hamiltonians from an iterative relay solve,
-// whose own residual of 1e-11 to 1e-10 is in the energy too.
-constexpr double kTraceDigits = 36.0, kTraceDigitsIterative = 33.0;
+// to 17 nodes), under what rounding leaves.  Energies of 39 systems of 12 to 533
+// atoms against extended precision, rms of the relative error: exp(-35) 5.7e-14,
+// exp(-36) 5.5e-14, exp(-33) 1.5e-13, from eigenvalues 8.9e-14.  exp(-33), mostly a
+// node fewer (1000 atoms 11.45 against 11.72 ms a call), leaves up to 7e-16 of the
+// sum, 5e-13 of the energy: for Hamiltonians from an iterative relay solve, whose
+// own residual of 1e-11 to 1e-10 is in the energy too.
+constexpr double kTraceDigits = 35.0, kTraceDigitsIterative = 33.0;
 struct TraceArgs {
   const double* H;         // n x n, row-major lower, ld
   int n, ld, nsl;
