@@ -19,8 +19,9 @@ value : energies/s of the headline mode (mixed_learned: block-CG relay solve
         inputs resident in HBM (mbd_rsscs_compute only), device-timed with
         CUDA events on the library's stream, max over ranks.
 plain_fp64 : the same workload in the plain FP64 mode, timed the same way;
-mixed_direct / learned_no_network : the 3xTF32 direct relay solve and the
-        block-CG without the network, timed the same way.
+mixed_direct / learned_no_network : the mixed mode (FP64 relay factors up to
+        5700 rows, 3xTF32 factors and refinement beyond) and the block-CG
+        without the network, timed the same way.
 e2e   : the headline mode through mbd_rsscs_energy_batch with host buffers
         (upload + compute + download every step), wall clock.  Each step
         uploads the batch anew, so its compute launches kernel by kernel.
@@ -420,7 +421,7 @@ def roofline(stage_ms, sizes, mode):
                 "kernel_ms": trace_ms,
                 "peak_source": "nominal FP64 (148 SM x 64 DFMA/clk x 1965 MHz); no FP64 entry in MEASURED_PEAKS.json",
                 "algorithmic": "(4/3)(3N)^3 flop per energy, the reduction that the trace form replaces; it does "
-                               "15 to 21 factors of (3N)^3/3 at 25 to 34 TFLOP/s instead (the stage time is summed "
+                               "13 to 15 factors of (3N)^3/3 at 25 to 34 TFLOP/s instead (the stage time is summed "
                                "over the slots' overlapping streams)",
                 "stage_ms": stages}
     if dom == "relay_factor":
