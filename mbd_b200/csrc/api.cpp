@@ -597,9 +597,7 @@ size_t mixed_bytes(const GeomPlan& p, size_t* r32, size_t* pan, size_t* vec, siz
 
 // Assigns the geometries to relay slots (longest first onto the least loaded
 // slot, load = (3N)^3), with as many slots as fit in the device memory share.
-// tight: memory ran out under a plan made without asking how much is free;
-// asks, and gives back the slots that the new plan does without.
-int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
+int plan_slots(mbd_ctx* ctx, bool eigen) {
   const int ng = (int)ctx->order.size();
   int S = std::max(1, std::min(kMaxSlots, ng));
   std::vector<int> slot_of(ctx->geoms.size(), 0);
@@ -620,7 +618,7 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
   // size) does not ask how much memory is free: that query goes through the
   // driver's kernel part, 0.05 to 2 ms depending on what else the host runs.
   deal(S);
-  bool held = !tight && (int)ctx->slots.size() >= S;
+  bool held = (int)ctx->slots.size() >= S;
   for (int g : ctx->order) {
     if (!held) break;
     const GeomDev& gd = *ctx->geoms[g];
@@ -667,7 +665,6 @@ int plan_slots(mbd_ctx* ctx, bool eigen, bool tight) {
   }
   ctx->slots_unasked = held;
   for (int g : ctx->order) ctx->geoms[g]->slot = slot_of[g];
-  while (tight && (int)ctx->slots.size() > S) ctx->slots.pop_back();
   while ((int)ctx->slots.size() < S) {
     std::unique_ptr<RelaySlot> sl(new RelaySlot());
     // slot 0 takes the batch's largest geometry (longest first), whose
@@ -820,8 +817,15 @@ int plan_eigen(mbd_ctx* ctx, const std::vector<int>& list, EigenPlan* ep) {
 
 // Plain-path slot buffers, per-geometry Hamiltonians, the tridiagonal plan and
 // the device job tables of the uploaded batch.
+// tight: memory ran out; the slots of earlier batches give theirs back and are
+// planned anew (the device is idle).
 int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
   drop_graphs(ctx, true);
+  if (tight) {
+    cudaGetLastError();
+    ctx->n_slots = 0;
+    ctx->slots.clear();
+  }
   ctx->replan = false;
   ctx->order.clear();
   for (size_t g = 0; g < ctx->geoms.size(); ++g)
@@ -857,7 +861,7 @@ int prepare_batch(mbd_ctx* ctx, bool eigen, bool tight = false) {
     ctx->n_slots = 0;
     return plan_eigen(ctx, {}, &ctx->eigen);
   }
-  int st = plan_slots(ctx, eigen, tight);
+  int st = plan_slots(ctx, eigen);
   if (st != MBD_OK) return st;
   // geometries whose energy comes from eigenvalues, by the two-stage reduction
   auto banded = [&](int g) {
@@ -1275,7 +1279,9 @@ int upload_batch(mbd_ctx* ctx, int n_geom, const mbd_geom* geoms, bool eigen) {
   if (st != MBD_OK) return st;
   int first = MBD_OK;
   for (int g = 0; g < n_geom && first == MBD_OK; ++g) first = ctx->geoms[g]->status_host;
+  const bool had_slots = !ctx->slots.empty();
   st = prepare_batch(ctx, eigen);
+  if (st == MBD_ERR_OUT_OF_MEMORY && had_slots) st = prepare_batch(ctx, eigen, true);
   if (st != MBD_OK) return st;
   ctx->have_batch = eigen;
   return first;
@@ -1303,7 +1309,6 @@ int mbd_rsscs_compute(mbd_ctx* ctx, int mode) {
   };
   int st = reserve();
   if (st == MBD_ERR_OUT_OF_MEMORY && ctx->slots_unasked) {   // fewer slots, for what memory there is
-    cudaGetLastError();
     MBD_CUDA(cudaDeviceSynchronize());
     st = prepare_batch(ctx, true, true);
     if (st == MBD_OK) st = reserve();
